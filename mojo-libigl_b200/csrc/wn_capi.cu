@@ -21,6 +21,7 @@
 #include "../../include/wn_b200.h"
 #include "wn_aabb.h"
 #include "wn_adjoint.h"
+#include "wn_exact.h"
 #include "wn_fwn.h"
 #include "wn_normals.h"
 #include "wn_batch.h"
@@ -200,6 +201,12 @@ int forward_fp64_host(const double* tri, const double* q, double* w, int64_t nf,
                       int mode) {
   if (nf < 0 || nq < 0) return fail(WN_EINVAL, "negative size (nf=%lld, nq=%lld)",
                                     (long long)nf, (long long)nq);
+  const bool automatic = mode == kFp64Auto;
+  if (automatic)
+    mode = nf >= 4096 && nf <= 0x7fffffffLL &&
+                   static_cast<double>(nf) * static_cast<double>(nq) >= 1e9
+               ? kFp64Tiled
+               : kFp64ArgProd;
   if (mode != kFp64ArgProd && mode != kFp64Direct && mode != kFp64Tiled)
     return fail(WN_EINVAL, "bad mode %d", mode);
   if (mode == kFp64Tiled && nf > 0x7fffffffLL) return fail(WN_EINVAL, "more than 2^31-1 faces");
@@ -210,6 +217,41 @@ int forward_fp64_host(const double* tri, const double* q, double* w, int64_t nf,
   DeviceCtx* c = context(&code);
   if (!c) return code;
   const int64_t ld = even_ld(nf);
+  if (automatic && exact_pays(nf, nq)) {
+    // Its scratch is larger than the all-pairs path's: where it cannot be had, that
+    // path serves the call.
+    const ExactPlan xp = plan_exact(nf, nq);
+    cudaError_t e;
+    if ((e = c->tri.ensure(sizeof(double) * 9 * ld)) != cudaSuccess ||
+        (e = c->q.ensure(sizeof(double) * 3 * nq)) != cudaSuccess ||
+        (e = c->w.ensure(sizeof(double) * nq)) != cudaSuccess)
+      return cuda_fail(e, "device allocation");
+    if (c->scratch.ensure(xp.bytes) == cudaSuccess) {
+      double* w_d = static_cast<double*>(c->w.ptr);
+      const double* q_d = static_cast<const double*>(c->q.ptr);
+      const double* tri_d = static_cast<const double*>(c->tri.ptr);
+      if ((e = cudaMemcpy2DAsync(c->tri.ptr, sizeof(double) * ld, tri, sizeof(double) * nf,
+                                 sizeof(double) * nf, 9, cudaMemcpyHostToDevice, c->stream)) !=
+              cudaSuccess ||
+          (e = cudaMemcpyAsync(c->q.ptr, q, sizeof(double) * 3 * nq, cudaMemcpyHostToDevice,
+                               c->stream)) != cudaSuccess)
+        return cuda_fail(e, "copy of the inputs");
+      int64_t nitem = -1;
+      if ((e = exact_build(xp, tri_d, ld, q_d, c->scratch.ptr, kExactMostFp64, &nitem,
+                           c->stream)) != cudaSuccess)
+        return cuda_fail(e, "mesh preparation");
+      if (nitem >= 0) {
+        if ((e = exact_eval(xp, nitem, q_d, w_d, c->scratch.ptr, c->sms, c->stream)) != cudaSuccess)
+          return cuda_fail(e, "exact winding-number launch");
+        if ((e = cudaMemcpyAsync(w, w_d, sizeof(double) * nq, cudaMemcpyDeviceToHost,
+                                 c->stream)) != cudaSuccess)
+          return cuda_fail(e, "copy of the result");
+        return collect_device_error(c, c->stream);
+      }
+    } else {
+      cudaGetLastError();
+    }
+  }
   const Fp64Plan plan = plan_fp64(nf, nq, c->sms);
   const Fp64TiledPlan tplan = plan_fp64_tiled(mixed_tiles(nf), nq, c->sms);
   size_t scratch = sizeof(double) * (plan.scratch_doubles + 1);
@@ -445,6 +487,45 @@ int wn_forward_fp64_device(const double* tri, int64_t ld, const double* q, doubl
   e = launch_fp64(plan, mode, tri, ld, nf, q, nq, w, scratch, c->err, st);
   if (scratch) cudaFreeAsync(scratch, st);
   return e == cudaSuccess ? WN_OK : cuda_fail(e, "FP64 winding-number launch");
+}
+
+int wn_forward_exact_device(const double* tri, int64_t ld, const double* q, double* w, int64_t nf,
+                            int64_t nq, int mixed, int* taken, void* stream) {
+  WN_NVTX_RANGE();
+  if (!taken) return fail(WN_EINVAL, "null taken");
+  *taken = 0;
+  if (nf < 0 || nq < 0 || ld < nf)
+    return fail(WN_EINVAL, "bad sizes (nf=%lld, nq=%lld, ld=%lld)", (long long)nf, (long long)nq,
+                (long long)ld);
+  if (!exact_pays(nf, nq)) return WN_OK;
+  if (!tri || !q || !w) return fail(WN_EINVAL, "null pointer");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // It waits for the stream once, which a capture does not allow.
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(st, &capture);
+  if (e != cudaSuccess) return cuda_fail(e, "stream state");
+  if (capture != cudaStreamCaptureStatusNone) return WN_OK;
+  int sms = 0;
+  {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    int code = WN_OK;
+    DeviceCtx* c = context(&code);
+    if (!c) return code;
+    sms = c->sms;
+  }
+  const ExactPlan p = plan_exact(nf, nq);
+  void* scratch = nullptr;
+  if (dev_malloc_async(&scratch, p.bytes, st) != cudaSuccess) {
+    cudaGetLastError();
+    return WN_OK;  // the caller's all-pairs path needs less memory
+  }
+  int64_t nitem = -1;
+  e = exact_build(p, tri, ld, q, scratch, mixed ? kExactMostMixed : kExactMostFp64, &nitem, st);
+  if (e == cudaSuccess && nitem >= 0) e = exact_eval(p, nitem, q, w, scratch, sms, st);
+  cudaFreeAsync(scratch, st);
+  if (e != cudaSuccess) return cuda_fail(e, "exact winding-number launch");
+  *taken = nitem >= 0 ? 1 : 0;
+  return WN_OK;
 }
 
 int wn_forward_mixed_host(const double* tri, const double* q, double* w, int64_t nf, int64_t nq,
@@ -1497,11 +1578,9 @@ int wn_signed_distance_fast_device(void* tree, void* fast, double beta, const do
 // give pair terms bit-identical to the reference.
 int64_t mli_winding_gpu(int64_t tri, int64_t q, int64_t dst, int64_t nf, int64_t nq) {
   WN_NVTX_RANGE();
-  const bool large = nf >= 4096 && static_cast<double>(nf) * static_cast<double>(nq) >= 1e9 &&
-                     nf <= 0x7fffffffLL;
   return forward_fp64_host(reinterpret_cast<const double*>(tri),
                            reinterpret_cast<const double*>(q), reinterpret_cast<double*>(dst), nf,
-                           nq, large ? kFp64Tiled : kFp64ArgProd) == WN_OK
+                           nq, kFp64Auto) == WN_OK
              ? 1
              : 0;
 }

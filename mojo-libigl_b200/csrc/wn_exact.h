@@ -1,0 +1,52 @@
+// Exact generalized winding number from near faces, boundary edges and an
+// integer (see wn_exact.cu for the method).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstddef>
+#include <cstdint>
+
+namespace wn {
+
+constexpr int kExactLeafFaces = 8;
+constexpr int kExactArity = 4;
+constexpr int kExactMaxLevels = 16;
+
+// Where the device arrays of one evaluation lie in its scratch block.
+struct ExactPlan {
+  int64_t nf = 0, nq = 0;
+  int64_t nleaf = 0, nnode = 0;
+  int nlevel = 0;
+  int64_t level_off[kExactMaxLevels] = {}, level_n[kExactMaxLevels] = {};
+  int64_t max_roots = 0;   // root edges kept; more than this and the method is not taken
+  uint32_t hash_slots = 0;  // a power of two
+  size_t info, faces64, faces32, partner, nb, lead, moments, test, eval, counts, first, groups,
+      roots, root_leaf;
+  size_t keys_in, keys_out, vals_in, vals_out, heads, next, pick, succ, perm, list, cub;
+  size_t cub_bytes = 0, bytes = 0;
+};
+
+// Whether a call of this size should take the method (the mesh's edges still decide).
+bool exact_pays(int64_t nf, int64_t nq);
+
+ExactPlan plan_exact(int64_t nf, int64_t nq);
+
+// The boundary's triangles and single edges that the method may take per face. Each costs
+// every query about 7e-12 s, a pair 5.5e-12 s in the FP64 all-pairs kernels and 1.2e-12 s
+// in the mixed one (327,680-face mesh with 8 % of its faces deleted, 0.087 per face, x
+// 262,144 queries: 47 ms against 440 and 94).
+constexpr double kExactMostFp64 = 0.55, kExactMostMixed = 0.13;
+
+// Pairs the mesh's edges, waits for the stream and reports in *nitem the triangles and
+// single edges of the boundary; -1 if they are more than `most` per face or the mesh is
+// not fit for the method (nothing further is done then). Else builds the tree and the
+// query order in `scratch` (plan.bytes).
+cudaError_t exact_build(const ExactPlan& p, const double* tri, int64_t ld, const double* q,
+                        void* scratch, double most, int64_t* nitem, cudaStream_t stream);
+
+// W of the queries (in the order given) after exact_build on the same stream.
+cudaError_t exact_eval(const ExactPlan& p, int64_t nitem, const double* q, double* w,
+                       void* scratch, int sms, cudaStream_t stream);
+
+}  // namespace wn

@@ -100,6 +100,22 @@ def forward_fp64_prepared(tri: torch.Tensor, ld: int, nf: int, O: torch.Tensor) 
     return w
 
 
+def forward_exact(tri: torch.Tensor, ld: int, nf: int, O: torch.Tensor,
+                  mixed: bool = False) -> torch.Tensor | None:
+    """Plain FP64 W from the near faces and the far faces' boundary (wn_exact.cu),
+    within rounding of forward_fp64; None where an all-pairs kernel (mixed: the
+    mixed-precision one) should run: small calls, faces that share no edges, a
+    stream under capture."""
+    q = O.to(torch.float64).contiguous()
+    w = torch.empty(q.shape[0], dtype=torch.float64, device=q.device)
+    taken = ctypes.c_int(0)
+    if q.shape[0] and nf:
+        _check(_lib.lib().wn_forward_exact_device(tri.data_ptr(), ld, q.data_ptr(), w.data_ptr(),
+                                                  nf, q.shape[0], int(mixed),
+                                                  ctypes.byref(taken), _stream()))
+    return w if taken.value else None
+
+
 class PreparedMesh:
     """A mesh prepared for the mixed-precision kernels (Morton-ordered tiles)."""
 
@@ -336,7 +352,14 @@ class WindingNumberFunction(torch.autograd.Function):
     def forward(ctx, V, F, O, precision="fp64", adjoint="edges"):
         tri, ld, nf = triangle_soa(V, F)
         ctx.mesh = None
-        if precision == "mixed":
+        # A mixed forward whose result is rounded to less than 64 bits takes the
+        # FP64 one where that is the faster; a 64-bit result keeps the mixed kernel.
+        w = None
+        if precision == "fp64" or O.dtype != torch.float64:
+            w = forward_exact(tri, ld, nf, O, mixed=precision == "mixed")
+        if w is not None:
+            pass
+        elif precision == "mixed":
             mesh = PreparedMesh(tri, ld, nf)
             w = mesh.forward(O)
             if adjoint in ("faces", "auto", "welded"):
@@ -361,7 +384,7 @@ class WindingNumberFunction(torch.autograd.Function):
         if adjoint == "auto":
             edges = boundary_edges(V, F)
             adjoint = "edges"
-            if ctx.mesh is not None and edges[1] > FACE_COST * ctx.nf:
+            if ctx.precision == "mixed" and edges[1] > FACE_COST * ctx.nf:
                 welded = welded_edges(V, F)
                 adjoint = "welded" if welded[1] < FACE_COST * ctx.nf else "faces"
             if adjoint != "faces" and ctx.mesh is not None:
@@ -374,10 +397,12 @@ class WindingNumberFunction(torch.autograd.Function):
             if ctx.mesh is not None:
                 ctx.mesh.close()
                 ctx.mesh = None
-        elif ctx.mesh is not None:
-            dq, dtri = ctx.mesh.backward(O, gW)
+        elif ctx.precision == "mixed":
+            mesh = ctx.mesh if ctx.mesh is not None else PreparedMesh(ctx.tri, ctx.ld, ctx.nf)
+            ctx.mesh = None
+            dq, dtri = mesh.backward(O, gW)
             dV = gather_vertices(dtri, ctx.ld, ctx.nf, F, V.shape[0])
-            ctx.mesh.close()
+            mesh.close()
         else:
             dV, dq = backward_fp64(ctx.tri, ctx.ld, ctx.nf, O, gW, F, V.shape[0])
         return dV.to(V.dtype), None, dq.to(O.dtype), None, None
