@@ -1,21 +1,39 @@
-// Closest-point traversal of the median-split hierarchy on sm_100a: one thread
-// per query, the reference's ordered depth-first walk (src/capi.mojo:522-586)
-// with its exact FP64 arithmetic (wn_aabb.cuh), so distances, face indices and
-// closest points are bit-identical to the reference's CPU path, ties included.
+// Closest points on sm_100a, bit-identical to the reference's CPU query
+// (src/capi.mojo:522-586: an ordered depth-first walk of the median-split hierarchy
+// with strict and non-strict tests in given places), ties included. One thread per
+// point; above kAabbSortMin points the threads take them in Morton order (perm).
 //
-// The walk is a chain of dependent reads (node record -> child boxes -> next
-// node) over a tree that sits in L2 (a 327,680-face mesh: 21.0 MB of node
-// records + 26 MB of face records), so the kernel is bound by load latency and
-// FP64 issue, not by HBM bandwidth. What helps is keeping a warp's 32 walks
-// alike: above kAabbSortMin queries the threads take their queries in Morton
-// order (perm), and every record is read with 16-byte non-coherent loads.
+// The reference's walk is a chain in a fixed order, and its order is a poor one: the
+// best distance comes down slowly, and FP64 boxes are read at every step. So the
+// minimum is found first, in an order and with bounds of its own, and then the face
+// that the reference's order would have kept:
 //
-// Each stack entry keeps the box distance computed when it was pushed. The
-// reference recomputes that distance from the same box when it pops the node;
-// the value is the same double, so the pop-time test `d > best` is unchanged.
-// The stored key is max(box distance, slab bound) (wn_aabb.h): a child is
-// pushed, and later expanded, only when both are <= best. The push order is
-// decided by the box distances alone, as in the reference.
+// 1. aabb_any_order_kernel walks the tree nearer disc centre first, skipping children
+//    by FP32 boxes and discs (wn_aabb.h), faces by discs of their own, and evaluates
+//    the others with the reference's FP64 arithmetic (wn_aabb.cuh). What it skips is
+//    farther than the best, so afterwards `best` is the smallest squared distance B
+//    that any face of the mesh evaluates to, and the faces that evaluate to B exactly
+//    have all been seen.
+// 2. The reference's result is the first of these in its order, if it looks at all of
+//    them: a leaf is looked at when its box distance is <= the best at that time, and
+//    that is never below B. So if every one of their leaves has a box distance <= B,
+//    the winner is the first by the walk's order, which two faces' common ancestor
+//    decides: the child with the smaller box distance comes first (the right one when
+//    they are equal), within a leaf the order of the records.
+// 3. Where rounding puts a leaf's box distance above B, or more than kTies faces tie,
+//    the thread does the reference's own walk.
+//
+// Trees that the library did not build may have boxes that do not hold their faces,
+// and closest points on very thin faces lose their digits: no bound of step 1 holds
+// then, and aabb_query_kernel does the reference's walk for every point.
+//
+// Bound by the walks' divergence and load latency, not by HBM or FP64 throughput (the
+// tree sits in L2; ncu, 524,288 points inside and around the 327,680-face sphere: 8.2 of
+// 32 lanes active, issue 42 %, FP64 pipe 15 %). Measured against the reference's walk
+// with box and slab (a range of n.x) alone: 327,680 faces x 2^20 points 10.1 -> 2.4 ms,
+// 243,602 (terrain) x 2^20 1.54 -> 1.34 ms, x 10,000 0.18 -> 0.12 ms. The reference's
+// order with the discs: 5.1 ms. Keeping the warp's lanes in step, leaves held until 1, 4,
+// 8 or more lanes have one: slower in either order (3.2 ms at best here).
 #include <cuda_runtime.h>
 
 #include "wn_aabb.cuh"
@@ -27,10 +45,20 @@ namespace wn {
 namespace {
 
 constexpr int kAabbThreads = 128;
+constexpr int kTies = 8;
+// Consecutive points of the (Morton) order that share a warp; its other lanes take
+// points from elsewhere, so that 32 of the longest walks do not meet in one warp, which
+// the rest of the GPU then waits for (327,680 faces x 2^20 points, stack in local memory:
+// 32 3.17 ms, 16 2.64, 8 2.87, 4 2.95).
+constexpr int kGroup = 16;
+// A face is thin below |n|^2 = kThin * (longest side)^4: thinner than about 1 : 1000.
+constexpr double kThin = 1e-6;
 
 struct AabbArgs {
   const AabbNodeRec* __restrict__ nodes;
+  const AabbWalkRec* __restrict__ walk;
   const AabbTriRec* __restrict__ tris;
+  const AabbDisc* __restrict__ face_discs;
   const double* __restrict__ P;
   const uint32_t* __restrict__ perm;
   double* __restrict__ sqrd;
@@ -40,33 +68,52 @@ struct AabbArgs {
   int64_t np, nnodes;
   double root[6];
   double scale;
+  int levels;  // depth of the tree
+};
+
+struct Best {
+  double d2, x, y, z;
+  int64_t face;
 };
 
 __device__ __forceinline__ double2 ldg2(const double* p) {
   return __ldg(reinterpret_cast<const double2*>(p));
 }
 
-// Squared lower bound on the distance from p to the faces inside a slab, less
-// the rounding margin `e` (0 when the slab cannot separate them).
-__device__ __forceinline__ double slab_bound2(double px, double py, double pz, float nx, float ny,
-                                              float nz, float lo, float hi, double e) {
-  const double t = fma(static_cast<double>(nz), pz,
-                       fma(static_cast<double>(ny), py, static_cast<double>(nx) * px));
-  const double g = fmax(static_cast<double>(lo) - t, t - static_cast<double>(hi)) - e;
-  return g > 0.0 ? g * g * (1.0 - kSlabMargin) : 0.0;
+__device__ __forceinline__ ClosestHit closest_on_record(const AabbTriRec* tr, double px, double py,
+                                                        double pz, int64_t& face) {
+  const double2 w0 = ldg2(tr->a), w1 = ldg2(tr->a + 2), w2 = ldg2(tr->b + 1);
+  const double2 w3 = ldg2(tr->c), w4 = ldg2(tr->c + 2);
+  face = __double_as_longlong(w4.y);
+  return closest_on_triangle(px, py, pz, w0.x, w0.y, w1.x, w1.y, w2.x, w2.y, w3.x, w3.y, w4.x);
 }
 
-__global__ void __launch_bounds__(kAabbThreads) aabb_query_kernel(const AabbArgs a) {
-  const int64_t t = static_cast<int64_t>(blockIdx.x) * kAabbThreads + threadIdx.x;
-  if (t >= a.np) return;
-  const int64_t qi = a.perm ? static_cast<int64_t>(a.perm[t]) : t;
-  const double px = a.P[3 * qi], py = a.P[3 * qi + 1], pz = a.P[3 * qi + 2];
-  double best = 1.0e300;
-  int64_t best_face = -1;
-  double bx = 0.0, by = 0.0, bz = 0.0;
-  // Slab margin for this point; no slab skips at all for huge or non-finite input.
-  double margin = kSlabMargin * (a.scale + fabs(px) + fabs(py) + fabs(pz));
-  if (!(margin < 1e100)) margin = INFINITY;
+__device__ __forceinline__ double box_of(const double* box, double px, double py, double pz) {
+  const double2 b0 = ldg2(box), b1 = ldg2(box + 2), b2 = ldg2(box + 4);
+  return box_distance2(px, py, pz, b0.x, b0.y, b1.x, b1.y, b2.x, b2.y);
+}
+
+// Squared lower bound on the distance from p to the faces inside a disc, less the
+// rounding margin `e`; v2 receives the squared distance from its centre.
+__device__ __forceinline__ float disc_bound2(float px, float py, float pz, const float4& nt,
+                                             const float4& cr, float e, float& v2) {
+  const float x = px - cr.x, y = py - cr.y, z = pz - cr.z;
+  const float h = nt.x * x + nt.y * y + nt.z * z;
+  v2 = x * x + y * y + z * z;
+  const float g = fmaxf(fabsf(h) - nt.w - e, 0.0f);
+  const float l = fmaxf(sqrtf(fmaxf(v2 * (1.0f - 2e-6f) - h * h, 0.0f)) - cr.w - e, 0.0f);
+  return (g * g + l * l) * (1.0f - kWalkRel);
+}
+// The reference's walk. Each stack entry keeps the box distance computed when it was
+// pushed (the reference recomputes the same double from the same box at the pop), or
+// the disc bound where that is larger: such a child holds no face that the reference
+// would take. The order is decided by the box distances alone.
+__device__ __noinline__ Best ordered_walk(const AabbArgs& a, double px, double py, double pz) {
+  const double size = a.scale + fabs(px) + fabs(py) + fabs(pz);
+  const float margin = size < 1e15 ? kWalkMargin * __double2float_ru(size) : INFINITY;
+  const float fx = static_cast<float>(px), fy = static_cast<float>(py),
+              fz = static_cast<float>(pz);
+  Best r{1.0e300, 0.0, 0.0, 0.0, -1};
   int stack_node[kAabbStack];
   double stack_d2[kAabbStack];
   int sp = 0;
@@ -78,60 +125,353 @@ __global__ void __launch_bounds__(kAabbThreads) aabb_query_kernel(const AabbArgs
   }
   while (sp > 0) {
     --sp;
-    if (stack_d2[sp] > best) continue;
+    if (stack_d2[sp] > r.d2) continue;
     const AabbNodeRec* nd = a.nodes + stack_node[sp];
     const int4 meta = __ldg(reinterpret_cast<const int4*>(nd));
     if (meta.w > 0) {
-      const AabbTriRec* tr = a.tris + meta.z;
-      for (int k = 0; k < meta.w; ++k, ++tr) {
-        const double2 w0 = ldg2(tr->a), w1 = ldg2(tr->a + 2), w2 = ldg2(tr->b + 1);
-        const double2 w3 = ldg2(tr->c), w4 = ldg2(tr->c + 2);
-        const ClosestHit h = closest_on_triangle(px, py, pz, w0.x, w0.y, w1.x, w1.y, w2.x, w2.y,
-                                                 w3.x, w3.y, w4.x);
-        if (h.d2 < best) {
-          best = h.d2;
-          best_face = __double_as_longlong(w4.y);
-          bx = h.x;
-          by = h.y;
-          bz = h.z;
-        }
+      for (int k = 0; k < meta.w; ++k) {
+        int64_t face;
+        const ClosestHit h = closest_on_record(a.tris + meta.z + k, px, py, pz, face);
+        if (h.d2 < r.d2) r = Best{h.d2, h.x, h.y, h.z, face};
       }
     } else {
-      const double2 l0 = ldg2(nd->lbox), l1 = ldg2(nd->lbox + 2), l2 = ldg2(nd->lbox + 4);
-      const double2 r0 = ldg2(nd->rbox), r1 = ldg2(nd->rbox + 2), r2 = ldg2(nd->rbox + 4);
-      const float4 s0 = __ldg(reinterpret_cast<const float4*>(&nd->lslab));
-      const float4 s1 = __ldg(reinterpret_cast<const float4*>(&nd->lslab) + 1);
-      const float2 s2 = __ldg(reinterpret_cast<const float2*>(&nd->rslab.lo));
-      const double dl = box_distance2(px, py, pz, l0.x, l0.y, l1.x, l1.y, l2.x, l2.y);
-      const double dr = box_distance2(px, py, pz, r0.x, r0.y, r1.x, r1.y, r2.x, r2.y);
-      const double kl = fmax(dl, slab_bound2(px, py, pz, s0.x, s0.y, s0.z, s0.w, s1.x, margin));
-      const double kr = fmax(dr, slab_bound2(px, py, pz, s1.y, s1.z, s1.w, s2.x, s2.y, margin));
+      const double dl = box_of(nd->lbox, px, py, pz), dr = box_of(nd->rbox, px, py, pz);
+      double kl = dl, kr = dr;
+      if (a.walk) {
+        const float4* disc = reinterpret_cast<const float4*>(a.walk + (nd - a.nodes)) + 1;
+        float v2;
+        kl = fmax(kl, static_cast<double>(disc_bound2(fx, fy, fz, __ldg(disc), __ldg(disc + 1),
+                                                      margin, v2)));
+        kr = fmax(kr, static_cast<double>(disc_bound2(fx, fy, fz, __ldg(disc + 2),
+                                                      __ldg(disc + 3), margin, v2)));
+      }
       // Farther child first, so the nearer one is popped next (capi.mojo:571-586).
       const bool left_near = dl < dr;
       const int first = left_near ? meta.y : meta.x, second = left_near ? meta.x : meta.y;
       const double dfirst = left_near ? kr : kl, dsecond = left_near ? kl : kr;
       if (sp + 2 > kAabbStack) {  // cannot happen for a validated tree
         atomicOr(a.err, kErrBadLaunch);
-        best_face = -2;
+        r.face = -2;
         break;
       }
-      if (dfirst <= best) {
+      if (dfirst <= r.d2) {
         stack_node[sp] = first;
         stack_d2[sp] = dfirst;
         ++sp;
       }
-      if (dsecond <= best) {
+      if (dsecond <= r.d2) {
         stack_node[sp] = second;
         stack_d2[sp] = dsecond;
         ++sp;
       }
     }
   }
-  a.sqrd[qi] = best;
-  a.index[qi] = best_face;
-  a.closest[3 * qi] = bx;
-  a.closest[3 * qi + 1] = by;
-  a.closest[3 * qi + 2] = bz;
+  return r;
+}
+
+__device__ __forceinline__ void store_result(const AabbArgs& a, int64_t qi, const Best& r) {
+  a.sqrd[qi] = r.d2;
+  a.index[qi] = r.face;
+  a.closest[3 * qi] = r.x;
+  a.closest[3 * qi + 1] = r.y;
+  a.closest[3 * qi + 2] = r.z;
+}
+
+__global__ void __launch_bounds__(kAabbThreads) aabb_query_kernel(const AabbArgs a) {
+  const int64_t t = static_cast<int64_t>(blockIdx.x) * kAabbThreads + threadIdx.x;
+  if (t >= a.np) return;
+  const int64_t qi = a.perm ? static_cast<int64_t>(a.perm[t]) : t;
+  store_result(a, qi, ordered_walk(a, a.P[3 * qi], a.P[3 * qi + 1], a.P[3 * qi + 2]));
+}
+
+__device__ __forceinline__ float box_bound2(float px, float py, float pz, float lx, float ly,
+                                            float lz, float hx, float hy, float hz, float e) {
+  const float x = fmaxf(fmaxf(lx - px, px - hx) - e, 0.0f);
+  const float y = fmaxf(fmaxf(ly - py, py - hy) - e, 0.0f);
+  const float z = fmaxf(fmaxf(lz - pz, pz - hz) - e, 0.0f);
+  return (x * x + y * y + z * z) * (1.0f - kWalkRel);
+}
+
+// Whether the reference's walk reaches face record i before face record j.
+__device__ __forceinline__ bool comes_first(const AabbArgs& a, int i, int j, double px, double py,
+                                            double pz) {
+  int node = 0;
+  for (;;) {
+    const int4 m = __ldg(reinterpret_cast<const int4*>(a.walk + node));
+    if (m.w > 0) return i < j;
+    const bool il = i < m.z, jl = j < m.z;
+    if (il == jl) {
+      node = il ? m.x : m.y;
+      continue;
+    }
+    const AabbNodeRec* nd = a.nodes + node;
+    const bool left_near = box_of(nd->lbox, px, py, pz) < box_of(nd->rbox, px, py, pz);
+    return il == left_near;
+  }
+}
+
+__global__ void __launch_bounds__(kAabbThreads) aabb_any_order_kernel(const AabbArgs a) {
+  // (node, bound) per level and thread; in local memory it competed with the tree for L1
+  // (2.64 -> 2.44 ms).
+  extern __shared__ uint2 s_stack[];
+  const int64_t slot = static_cast<int64_t>(blockIdx.x) * kAabbThreads + threadIdx.x;
+  const int64_t nwarp = (a.np + 31) / 32, warp = slot / 32, lane = slot % 32;
+  if (warp >= nwarp) return;
+  const int64_t t = (lane / kGroup) * (nwarp * kGroup) + warp * kGroup + lane % kGroup;
+  if (t >= a.np) return;
+  const int64_t qi = a.perm ? static_cast<int64_t>(a.perm[t]) : t;
+  const double px = a.P[3 * qi], py = a.P[3 * qi + 1], pz = a.P[3 * qi + 2];
+  // No bound skips anything for huge or non-finite input.
+  const double size = a.scale + fabs(px) + fabs(py) + fabs(pz);
+  const float margin = size < 1e15 ? kWalkMargin * __double2float_ru(size) : INFINITY;
+  const float fx = static_cast<float>(px), fy = static_cast<float>(py),
+              fz = static_cast<float>(pz);
+  Best r{1.0e300, 0.0, 0.0, 0.0, -1};
+  float bestf = INFINITY;  // r.d2, rounded up
+  int tie[kTies], tie_slot[kTies], nties = 0;  // face records that evaluate to r.d2
+  uint2* stack = s_stack + threadIdx.x;
+  int sp = 0, node = 0;
+  while (node >= 0) {
+    const float4* rec = reinterpret_cast<const float4*>(a.walk + node);
+    const int4 meta = __ldg(reinterpret_cast<const int4*>(rec));
+    int go = -1;
+    if (meta.w > 0) {
+      // The faces whose own discs do not rule them out, up to 32 at a time, then those
+      // exactly.
+      for (int k0 = 0; k0 < meta.w; k0 += 32) {
+        const int n = min(meta.w - k0, 32);
+        const float4* disc = reinterpret_cast<const float4*>(a.face_discs + meta.z + k0);
+        unsigned todo = 0;
+        for (int k = 0; k < n; ++k) {
+          float v2;
+          const float lb = disc_bound2(fx, fy, fz, __ldg(disc + 2 * k), __ldg(disc + 2 * k + 1),
+                                       margin, v2);
+          if (!(lb > bestf)) todo |= 1u << k;
+        }
+        while (todo) {
+          const int k = meta.z + k0 + __ffs(todo) - 1;
+          todo &= todo - 1;
+          int64_t face;
+          const ClosestHit h = closest_on_record(a.tris + k, px, py, pz, face);
+          if (h.d2 < r.d2) {
+            r = Best{h.d2, h.x, h.y, h.z, face};
+            bestf = __double2float_ru(h.d2);
+            nties = 0;
+          }
+          if (h.d2 == r.d2) {
+            if (nties < kTies) {
+              tie[nties] = k;
+              tie_slot[nties] = meta.x;
+            }
+            ++nties;
+          }
+        }
+      }
+    } else {
+      const float4 ln = __ldg(rec + 1), lc = __ldg(rec + 2), rn = __ldg(rec + 3),
+                   rc = __ldg(rec + 4), b0 = __ldg(rec + 5), b1 = __ldg(rec + 6),
+                   b2 = __ldg(rec + 7);
+      float vl, vr;
+      const float kl = fmaxf(disc_bound2(fx, fy, fz, ln, lc, margin, vl),
+                             box_bound2(fx, fy, fz, b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, margin));
+      const float kr = fmaxf(disc_bound2(fx, fy, fz, rn, rc, margin, vr),
+                             box_bound2(fx, fy, fz, b1.z, b1.w, b2.x, b2.y, b2.z, b2.w, margin));
+      const bool left = !(kl > bestf), right = !(kr > bestf);
+      if (left && right) {
+        const bool left_first = vl < vr;
+        go = left_first ? meta.x : meta.y;
+        if (sp < a.levels) {  // always, in a validated tree
+          stack[sp * kAabbThreads] = make_uint2(static_cast<unsigned>(left_first ? meta.y : meta.x),
+                                                __float_as_uint(left_first ? kr : kl));
+          ++sp;
+        } else {
+          nties = kTies + 1;  // not all seen: the reference's walk decides
+          atomicOr(a.err, kErrBadLaunch);
+        }
+      } else if (left || right) {
+        go = left ? meta.x : meta.y;
+      }
+    }
+    while (go < 0 && sp > 0) {
+      --sp;
+      const uint2 e = stack[sp * kAabbThreads];
+      if (!(__uint_as_float(e.y) > bestf)) go = static_cast<int>(e.x);
+    }
+    node = go;
+  }
+  bool sure = nties >= 1 && nties <= kTies;
+  for (int k = 0; sure && k < nties; ++k) {
+    const int slot = tie_slot[k];
+    const double d = slot < 0 ? box_distance2(px, py, pz, a.root[0], a.root[1], a.root[2],
+                                              a.root[3], a.root[4], a.root[5])
+                              : box_of(slot & 1 ? a.nodes[slot >> 1].rbox : a.nodes[slot >> 1].lbox,
+                                       px, py, pz);
+    sure = d <= r.d2;
+  }
+  if (sure && nties > 1) {
+    int win = tie[0];
+    for (int k = 1; k < nties; ++k)
+      if (comes_first(a, tie[k], win, px, py, pz)) win = tie[k];
+    const ClosestHit h = closest_on_record(a.tris + win, px, py, pz, r.face);
+    r.x = h.x;
+    r.y = h.y;
+    r.z = h.z;
+  }
+  if (!sure) r = ordered_walk(a, px, py, pz);
+  store_result(a, qi, r);
+}
+
+// ---- discs ---------------------------------------------------------------------
+
+template <class T, class F>
+__device__ __forceinline__ T block_reduce(T v, T* part, F f) {
+  for (int o = 16; o; o >>= 1) v = f(v, __shfl_xor_sync(~0u, v, o));
+  const int nw = blockDim.x >> 5;
+  if (nw == 1) return v;
+  __syncthreads();  // the array's last readers are done
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = part[0];
+  for (int k = 1; k < nw; ++k) v = f(v, part[k]);
+  return v;
+}
+
+// The disc of one node per CTA: of node list[blockIdx.x], or of node blockIdx.x unless
+// it has more than kDiscBig faces. Three passes over its vertices: normal and shape of
+// the faces; ranges along the normal and two axes across it (the centre); thickness and
+// radius about the centre as rounded to FP32.
+__global__ void aabb_disc_kernel(const AabbTriRec* __restrict__ tris,
+                                 const AabbSpan* __restrict__ spans, const int32_t* list,
+                                 double scale, AabbWalkRec* nodes) {
+  __shared__ double part[32];
+  const int64_t node = list ? list[blockIdx.x] : static_cast<int64_t>(blockIdx.x);
+  const AabbSpan s = spans[node];
+  if (s.slot < 0 || s.last <= s.first || !(scale < 1e100)) return;
+  if (!list && s.last - s.first > kDiscBig) return;
+  const int step = static_cast<int>(blockDim.x);
+  const auto add = [](double a, double b) { return a + b; };
+  const auto low = [](double a, double b) { return fmin(a, b); };
+  const auto high = [](double a, double b) { return fmax(a, b); };
+  double nx = 0.0, ny = 0.0, nz = 0.0, thin = 0.0;
+  for (int k = s.first + threadIdx.x; k < s.last; k += step) {
+    const AabbTriRec& t = tris[k];
+    const double ux = t.b[0] - t.a[0], uy = t.b[1] - t.a[1], uz = t.b[2] - t.a[2];
+    const double wx = t.c[0] - t.a[0], wy = t.c[1] - t.a[1], wz = t.c[2] - t.a[2];
+    const double ex = wx - ux, ey = wy - uy, ez = wz - uz;
+    const double cx = uy * wz - uz * wy, cy = uz * wx - ux * wz, cz = ux * wy - uy * wx;
+    const double l2 = fmax(fmax(ux * ux + uy * uy + uz * uz, wx * wx + wy * wy + wz * wz),
+                           ex * ex + ey * ey + ez * ez);
+    if (!(cx * cx + cy * cy + cz * cz >= kThin * l2 * l2)) thin = 1.0;
+    nx += cx;
+    ny += cy;
+    nz += cz;
+  }
+  nx = block_reduce(nx, part, add);
+  ny = block_reduce(ny, part, add);
+  nz = block_reduce(nz, part, add);
+  thin = block_reduce(thin, part, high);
+  const double len = sqrt(nx * nx + ny * ny + nz * nz);
+  const bool has = len > 0.0 && len < INFINITY;
+  nx = has ? nx / len : 1.0;
+  ny = has ? ny / len : 0.0;
+  nz = has ? nz / len : 0.0;
+  // As floats, shortened until |n| <= 1 (then |n.(p - x)| <= |p - x|).
+  const double keep = 1.0 - 1.5e-7;
+  const float fx = static_cast<float>(nx * keep), fy = static_cast<float>(ny * keep),
+              fz = static_cast<float>(nz * keep);
+  // Two axes across n.
+  const bool zmost = fabs(nz) < 0.7;
+  const double vx0 = zmost ? ny : -nz, vy0 = zmost ? -nx : 0.0, vz0 = zmost ? 0.0 : nx;
+  const double vl = 1.0 / sqrt(vx0 * vx0 + vy0 * vy0 + vz0 * vz0);
+  const double ux = vx0 * vl, uy = vy0 * vl, uz = vz0 * vl;
+  const double wx = ny * uz - nz * uy, wy = nz * ux - nx * uz, wz = nx * uy - ny * ux;
+  double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+  for (int k = s.first + threadIdx.x; k < s.last; k += step)
+    for (int j = 0; j < 3; ++j) {
+      const double* x = j == 0 ? tris[k].a : (j == 1 ? tris[k].b : tris[k].c);
+      const double d[3] = {nx * x[0] + ny * x[1] + nz * x[2], ux * x[0] + uy * x[1] + uz * x[2],
+                           wx * x[0] + wy * x[1] + wz * x[2]};
+      for (int i = 0; i < 3; ++i) {
+        lo[i] = fmin(lo[i], d[i]);
+        hi[i] = fmax(hi[i], d[i]);
+      }
+    }
+  double mid[3];
+  for (int i = 0; i < 3; ++i)
+    mid[i] = 0.5 * (block_reduce(lo[i], part, low) + block_reduce(hi[i], part, high));
+  const float cx = static_cast<float>(nx * mid[0] + ux * mid[1] + wx * mid[2]);
+  const float cy = static_cast<float>(ny * mid[0] + uy * mid[1] + wy * mid[2]);
+  const float cz = static_cast<float>(nz * mid[0] + uz * mid[1] + wz * mid[2]);
+  double t = 0.0, r2 = 0.0, w2 = 0.0;
+  for (int k = s.first + threadIdx.x; k < s.last; k += step)
+    for (int j = 0; j < 3; ++j) {
+      const double* x = j == 0 ? tris[k].a : (j == 1 ? tris[k].b : tris[k].c);
+      const double dx = x[0] - cx, dy = x[1] - cy, dz = x[2] - cz;
+      const double h = static_cast<double>(fx) * dx + static_cast<double>(fy) * dy +
+                       static_cast<double>(fz) * dz;
+      const double q = dx * dx + dy * dy + dz * dz;
+      t = fmax(t, fabs(h));
+      r2 = fmax(r2, q - h * h);
+      w2 = fmax(w2, q);
+    }
+  t = block_reduce(t, part, high);
+  r2 = block_reduce(r2, part, high);
+  w2 = block_reduce(w2, part, high);
+  if (threadIdx.x != 0) return;
+  AabbWalkRec& parent = nodes[s.slot >> 1];
+  AabbDisc& out = s.slot & 1 ? parent.rdisc : parent.ldisc;
+  const double pad = 1e-12 * scale;  // >> the rounding of the sums above
+  out.n[0] = fx;
+  out.n[1] = fy;
+  out.n[2] = fz;
+  out.c[0] = cx;
+  out.c[1] = cy;
+  out.c[2] = cz;
+  out.t = __double2float_ru(t + pad);
+  out.r = thin > 0.0 ? INFINITY : __double2float_ru(sqrt(r2 + 1e-14 * w2) * (1.0 + 1e-9) + pad);
+}
+
+// The disc of every face: about its centroid, along its own normal.
+__global__ void aabb_face_disc_kernel(const AabbTriRec* __restrict__ tris, int64_t n,
+                                      double scale, AabbDisc* __restrict__ out,
+                                      int32_t* __restrict__ thin) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const AabbTriRec& t = tris[i];
+  const double ux = t.b[0] - t.a[0], uy = t.b[1] - t.a[1], uz = t.b[2] - t.a[2];
+  const double wx = t.c[0] - t.a[0], wy = t.c[1] - t.a[1], wz = t.c[2] - t.a[2];
+  const double ex = wx - ux, ey = wy - uy, ez = wz - uz;
+  double nx = uy * wz - uz * wy, ny = uz * wx - ux * wz, nz = ux * wy - uy * wx;
+  const double l2 = fmax(fmax(ux * ux + uy * uy + uz * uz, wx * wx + wy * wy + wz * wz),
+                         ex * ex + ey * ey + ez * ez);
+  const double nn = nx * nx + ny * ny + nz * nz;
+  const bool is_thin = !(nn >= kThin * l2 * l2);
+  if (is_thin) *thin = 1;
+  const double inv = nn > 0.0 && nn < INFINITY ? (1.0 - 1.5e-7) / sqrt(nn) : 0.0;
+  AabbDisc d;
+  d.n[0] = static_cast<float>(nx * inv);
+  d.n[1] = static_cast<float>(ny * inv);
+  d.n[2] = static_cast<float>(nz * inv);
+  d.t = d.r = INFINITY;
+  for (int j = 0; j < 3; ++j) d.c[j] = static_cast<float>((t.a[j] + t.b[j] + t.c[j]) / 3.0);
+  if (scale < 1e100) {
+    double h = 0.0, r2 = 0.0, w2 = 0.0;
+    for (int j = 0; j < 3; ++j) {
+      const double* x = j == 0 ? t.a : (j == 1 ? t.b : t.c);
+      const double dx = x[0] - d.c[0], dy = x[1] - d.c[1], dz = x[2] - d.c[2];
+      const double p = d.n[0] * dx + d.n[1] * dy + d.n[2] * dz;
+      const double q = dx * dx + dy * dy + dz * dz;
+      h = fmax(h, fabs(p));
+      r2 = fmax(r2, q - p * p);
+      w2 = fmax(w2, q);
+    }
+    const double pad = 1e-12 * scale;
+    d.t = __double2float_ru(h + pad);
+    if (!is_thin) d.r = __double2float_ru(sqrt(r2 + 1e-14 * w2) * (1.0 + 1e-9) + pad);
+  }
+  float4* dst = reinterpret_cast<float4*>(out + i);
+  dst[0] = make_float4(d.n[0], d.n[1], d.n[2], d.t);
+  dst[1] = make_float4(d.c[0], d.c[1], d.c[2], d.r);
 }
 
 __global__ void signed_from_winding_kernel(const double* __restrict__ w, double* __restrict__ s,
@@ -149,12 +489,31 @@ cudaError_t aabb_query(const AabbDeviceTree& t, const double* P, int64_t np, con
                        cudaStream_t stream) {
   if (np <= 0) return cudaSuccess;
   if (t.depth + 1 > kAabbStack) return cudaErrorInvalidValue;
-  AabbArgs a{t.nodes, t.tris, P, perm, sqrd, index, closest, err, np, t.nnodes, {}, t.scale};
+  AabbArgs a{t.nodes, t.walk, t.tris, t.face_discs, P, perm, sqrd, index, closest, err, np,
+             t.nnodes, {}, t.scale, t.depth};
   for (int k = 0; k < 6; ++k) a.root[k] = t.root[k];
   const int64_t blocks = (np + kAabbThreads - 1) / kAabbThreads;
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  aabb_query_kernel<<<static_cast<unsigned>(blocks), kAabbThreads, 0, stream>>>(a);
+  if (t.any_order && t.nnodes > 0)
+    aabb_any_order_kernel<<<static_cast<unsigned>(blocks), kAabbThreads,
+                            sizeof(uint2) * kAabbThreads * t.depth, stream>>>(a);
+  else
+    aabb_query_kernel<<<static_cast<unsigned>(blocks), kAabbThreads, 0, stream>>>(a);
   g_launches.fetch_add(1, std::memory_order_relaxed);
+  return cudaGetLastError();
+}
+
+cudaError_t aabb_discs(const AabbDeviceTree& t, const AabbSpan* spans, const int32_t* big,
+                       int64_t nbig, int32_t* thin, cudaStream_t stream) {
+  if (t.nnodes <= 0) return cudaSuccess;
+  aabb_disc_kernel<<<static_cast<unsigned>(t.nnodes), 32, 0, stream>>>(t.tris, spans, nullptr,
+                                                                       t.scale, t.walk);
+  if (nbig > 0)
+    aabb_disc_kernel<<<static_cast<unsigned>(nbig), 512, 0, stream>>>(t.tris, spans, big, t.scale,
+                                                                      t.walk);
+  aabb_face_disc_kernel<<<static_cast<unsigned>((t.nleaf_faces + 255) / 256), 256, 0, stream>>>(
+      t.tris, t.nleaf_faces, t.scale, t.face_discs, thin);
+  g_launches.fetch_add(nbig > 0 ? 3 : 2, std::memory_order_relaxed);
   return cudaGetLastError();
 }
 

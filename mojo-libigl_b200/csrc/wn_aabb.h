@@ -4,22 +4,22 @@
 //
 // The tree is the one the reference builds in python/igl/__init__.py:286-319
 // (boxes lo/hi, nodes left/right/start/count, faces in leaf order, nodes in
-// preorder); the traversal is src/capi.mojo:522-586. On the device each node
-// becomes one 160-byte record holding the boxes of BOTH children next to the
-// child indices, so an internal node costs one record read for its two box
-// tests; the faces of every leaf sit contiguously in leaf order, 80 bytes each
-// (corners A, B, C and the face index).
+// preorder); the reference's traversal is src/capi.mojo:522-586. On the device a
+// node has two records. AabbNodeRec holds the FP64 boxes of BOTH children next to the
+// child indices, for the reference's own walk. AabbWalkRec holds bounds of both
+// children in FP32, for the walk in any order that wn_aabb.cu starts with: the box,
+// and a disc.
 //
-// Each child also carries a slab: a unit normal n (the normalised area-weighted
-// sum of its faces' normals) and the range [lo, hi] of n.x over every vertex of
-// its faces, rounded outward. Every point of those faces lies in the slab, so
-// max(lo - n.p, n.p - hi) bounds the distance from p to any of them from below.
-// The traversal skips a child when that bound, less a rounding margin, already
-// exceeds the best squared distance: none of its faces could be taken (a face
-// is taken only when strictly closer than the best so far, and the best only
-// decreases), so skipping changes no later decision and the result stays the
-// reference's. For curved surfaces it removes most of the leaves whose boxes
-// reach toward a point that is far from the surface.
+// A disc is a unit normal n (the normalised area-weighted sum of the faces' normals), a
+// centre c, and the thickness t and radius r such that every vertex x of the faces has
+// |n.(x - c)| <= t and lies within r of the axis c + s n. The faces lie in that
+// cylinder, so with h = n.(p - c) and l the distance of p from the axis,
+// max(|h| - t, 0)^2 + max(l - r, 0)^2 bounds the squared distance from p to any of
+// them from below. A child is skipped when that bound, less a rounding margin, exceeds
+// the best squared distance. Points away from a curved surface reach many boxes but
+// few discs: inside a 327,680-face sphere the reference's walk tests 595 faces a point
+// with the boxes alone, 367 with the range of n.x (a slab) beside them, 46 with the
+// discs, 29 when the order is by the discs' centres.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -28,19 +28,32 @@
 
 namespace wn {
 
-struct AabbSlab {
-  float n[3];   // unit normal
-  float lo, hi;  // range of n.x over the child's vertices, rounded outward (+-inf: no slab)
+struct __align__(16) AabbDisc {
+  float n[3], t;  // unit normal (|n| <= 1), half thickness; +inf: no bound along n
+  float c[3], r;  // centre, radius; +inf: no bound across n
 };
 
-struct __align__(32) AabbNodeRec {
+struct __align__(16) AabbNodeRec {
   int32_t left, right, start, count;  // count > 0: a leaf of faces [start, start+count)
   double lbox[6];  // left child's box (lo xyz, hi xyz); unused for a leaf
   double rbox[6];  // right child's box
-  AabbSlab lslab, rslab;
-  int32_t pad[2];
 };
-static_assert(sizeof(AabbNodeRec) == 160, "node record is five 32-byte sectors");
+static_assert(sizeof(AabbNodeRec) == 112, "node record is seven 16-byte words");
+
+struct __align__(16) AabbWalkRec {
+  int32_t left, right;  // a leaf: its place beside its parent (AabbSpan::slot), unused
+  int32_t start, count;  // as AabbNodeRec's; an internal node: its right child's first face
+  AabbDisc ldisc, rdisc;
+  float lbox[6], rbox[6];  // rounded outward
+};
+static_assert(sizeof(AabbWalkRec) == 128, "walk record is one cache line");
+
+// A node's faces (a run [first, last) of the face records; empty if they are not one
+// run, possible only in a caller-made tree) and where its disc goes: 2 * parent + side,
+// -1 for the root.
+struct AabbSpan {
+  int32_t first, last, slot;
+};
 
 struct __align__(16) AabbTriRec {
   double a[3], b[3], c[3];
@@ -51,11 +64,14 @@ static_assert(sizeof(AabbTriRec) == 80, "face record is five 16-byte words");
 // A device-resident tree (immutable once built).
 struct AabbDeviceTree {
   AabbNodeRec* nodes = nullptr;
+  AabbWalkRec* walk = nullptr;
   AabbTriRec* tris = nullptr;
+  AabbDisc* face_discs = nullptr;  // one per face record
   int64_t nnodes = 0, nleaf_faces = 0;
   int depth = 0;       // levels, root = 1
   double root[6] = {};  // root box (the traversal tests it when the root is popped)
-  double scale = 0.0;   // largest |coordinate| of the mesh (sets the slab margin)
+  double scale = 0.0;   // largest |coordinate| of the mesh (sets the rounding margin)
+  bool any_order = false;  // aabb_pack's *regular, and no thin face (aabb_discs)
 };
 
 // Deepest tree the kernels accept (traversal stack of kAabbStack entries,
@@ -74,6 +90,16 @@ cudaError_t aabb_query(const AabbDeviceTree& t, const double* P, int64_t np, con
                        double* sqrd, int64_t* index, double* closest, int* err,
                        cudaStream_t stream);
 
+// Fills in the discs of a tree, its nodes' and its faces', whose records are on the
+// device (spans: nnodes, device; big: the nbig nodes of more than kDiscBig faces,
+// device). *thin (device, set to 0 before) becomes 1 if some face is thinner than
+// 1 : 1000: the reference's closest point on such a face may lie off it (the barycentric
+// quotients lose their digits), so no bound holds for it and only the reference's own
+// order says whether it is looked at.
+constexpr int kDiscBig = 256;
+cudaError_t aabb_discs(const AabbDeviceTree& t, const AabbSpan* spans, const int32_t* big,
+                       int64_t nbig, int32_t* thin, cudaStream_t stream);
+
 // s[i] <- sqrt(s[i]), negated where |w[i]| > 1/2 (inside a closed, consistently
 // oriented surface).
 cudaError_t signed_from_winding(const double* w, double* s, int64_t n, cudaStream_t stream);
@@ -89,18 +115,21 @@ int64_t aabb_build(const double* V, int64_t nv, const int64_t* F, int64_t nf, in
                    double* boxes, int64_t* nodes, int64_t* order, int threads, const char** why);
 
 // Validates caller-supplied tree arrays and converts them to the device
-// records (host memory, caller-sized: nnodes node records, nf face records),
-// slabs included; *scale receives the largest |coordinate| of the mesh.
-// Returns the depth (root = 1), or a negative value with the reason in *why.
+// records (host memory, caller-sized: nnodes node and walk records and spans, nf face
+// records); the discs are left without bounds, for aabb_discs to fill in on the device.
+// *scale receives the largest |coordinate| of the mesh; *regular whether every box holds
+// its children's boxes or its faces and every face lies in one leaf, as in the trees
+// that aabb_build makes. Returns the depth (root = 1), or a negative value with the
+// reason in *why.
 int64_t aabb_pack(const double* V, int64_t nv, const int64_t* F, int64_t nf, const double* boxes,
                   const int64_t* nodes, const int64_t* order, int64_t nnodes,
-                  AabbNodeRec* node_out, AabbTriRec* tri_out, double* scale, const char** why);
+                  AabbNodeRec* node_out, AabbWalkRec* walk_out, AabbSpan* span_out,
+                  AabbTriRec* tri_out, double* scale, bool* regular, const char** why);
 
-// Relative size of the slab margin: a child is skipped only when
-// (bound - kSlabMargin * (scale + |px| + |py| + |pz|))^2 * (1 - kSlabMargin)
-// exceeds the best squared distance. The margin covers the rounding of n.p,
-// of the slab ends and of the reference's own closest-point arithmetic (each
-// a few units of 2^-53 of the coordinates), with a factor above 1000 to spare.
-constexpr double kSlabMargin = 4e-12;
+// The walk's bounds are computed in FP32 from p - c: kWalkMargin * (scale + |px| + |py| +
+// |pz|) covers the rounding of p, of the differences and of their products (under 20
+// units of 2^-24 of the coordinates), kWalkRel the relative rest; both are far above
+// the rounding of the reference's own FP64 closest-point arithmetic.
+constexpr float kWalkMargin = 2e-6f, kWalkRel = 1e-5f;
 
 }  // namespace wn

@@ -208,88 +208,45 @@ float round_up(double x) {
   return f;
 }
 
-// Slab of every node: the normalised area-weighted normal sum of its faces,
-// stored as floats scaled so that |n| <= 1 (then |n.(p - x)| <= |p - x|), and
-// the range of n.x over the vertices of its faces, widened by a margin for the
-// FP64 rounding of n.x and rounded outward to float. A node whose faces are not
-// one contiguous run of `order` (possible only in a caller-made tree) gets the
-// empty slab [-inf, +inf], which never skips anything.
-void build_slabs(const AabbTriRec* tris, const int64_t* nodes, int64_t nnodes, double scale,
-                 std::vector<AabbSlab>& slabs, int threads) {
-  std::vector<double> nsum(3 * static_cast<size_t>(nnodes), 0.0);
-  std::vector<int64_t> first(nnodes), last(nnodes);
-  std::vector<char> whole(nnodes, 1);
+// Every node's run of face records and its place beside its parent; false unless every
+// internal node's run is its left child's followed by its right child's and every node
+// but the root has one parent (else, possible only in a caller-made tree, the runs mean
+// nothing).
+bool node_spans(const int64_t* nodes, int64_t nnodes, AabbSpan* span) {
+  bool whole = true;
+  for (int64_t i = 0; i < nnodes; ++i) span[i].slot = -1;
   for (int64_t i = nnodes - 1; i >= 0; --i) {  // children come after their parent
     const int64_t* nd = nodes + 4 * i;
-    double* n = &nsum[3 * i];
     if (nd[3] > 0) {
-      first[i] = nd[2];
-      last[i] = nd[2] + nd[3];
-      for (int64_t k = first[i]; k < last[i]; ++k) {
-        const AabbTriRec& t = tris[k];
-        const double u[3] = {t.b[0] - t.a[0], t.b[1] - t.a[1], t.b[2] - t.a[2]};
-        const double w[3] = {t.c[0] - t.a[0], t.c[1] - t.a[1], t.c[2] - t.a[2]};
-        n[0] += u[1] * w[2] - u[2] * w[1];
-        n[1] += u[2] * w[0] - u[0] * w[2];
-        n[2] += u[0] * w[1] - u[1] * w[0];
-      }
-    } else {
-      const int64_t l = nd[0], r = nd[1];
-      for (int k = 0; k < 3; ++k) n[k] = nsum[3 * l + k] + nsum[3 * r + k];
-      first[i] = std::min(first[l], first[r]);
-      last[i] = std::max(last[l], last[r]);
-      whole[i] = whole[l] && whole[r] && (last[l] == first[r] || last[r] == first[l]);
+      span[i].first = static_cast<int32_t>(nd[2]);
+      span[i].last = static_cast<int32_t>(nd[2] + nd[3]);
+      continue;
     }
+    AabbSpan &l = span[nd[0]], &r = span[nd[1]];
+    whole = whole && nd[0] != nd[1] && l.slot < 0 && r.slot < 0 && l.last == r.first;
+    l.slot = static_cast<int32_t>(2 * i);
+    r.slot = static_cast<int32_t>(2 * i + 1);
+    span[i].first = l.first;
+    span[i].last = r.last;
   }
-  slabs.assign(static_cast<size_t>(nnodes), AabbSlab{{0.f, 0.f, 0.f}, -INFINITY, INFINITY});
-  const double pad = 1e-13 * 3.0 * scale;  // >> the rounding of a 3-term dot product
-  auto work = [&](int64_t begin, int64_t step) {
-    for (int64_t i = begin; i < nnodes; i += step) {
-      if (!whole[i]) continue;
-      const double* s = &nsum[3 * i];
-      const double len = std::sqrt(s[0] * s[0] + s[1] * s[1] + s[2] * s[2]);
-      double n[3] = {1.0, 0.0, 0.0};
-      if (len > 0.0 && std::isfinite(len))
-        for (int k = 0; k < 3; ++k) n[k] = s[k] / len;
-      float nf[3];
-      for (int k = 0; k < 3; ++k) nf[k] = static_cast<float>(n[k]);
-      for (int guard = 0; guard < 8; ++guard) {  // shrink until |nf| <= 1
-        const double m = std::sqrt(static_cast<double>(nf[0]) * nf[0] +
-                                   static_cast<double>(nf[1]) * nf[1] +
-                                   static_cast<double>(nf[2]) * nf[2]);
-        if (m <= 1.0) break;
-        for (int k = 0; k < 3; ++k) nf[k] *= 1.0f - 1.0f / 8388608.0f;
-      }
-      double lo = INFINITY, hi = -INFINITY;
-      for (int64_t k = first[i]; k < last[i]; ++k) {
-        const AabbTriRec& t = tris[k];
-        for (const double* v : {t.a, t.b, t.c}) {
-          const double d = static_cast<double>(nf[0]) * v[0] + static_cast<double>(nf[1]) * v[1] +
-                           static_cast<double>(nf[2]) * v[2];
-          lo = std::min(lo, d);
-          hi = std::max(hi, d);
-        }
-      }
-      AabbSlab& out = slabs[i];
-      for (int k = 0; k < 3; ++k) out.n[k] = nf[k];
-      out.lo = round_down(lo - pad);
-      out.hi = round_up(hi + pad);
-    }
-  };
-  if (threads <= 1 || nnodes < 4096) {
-    work(0, 1);
-  } else {
-    std::vector<std::thread> pool;
-    for (int t = 0; t < threads; ++t) pool.emplace_back(work, t, threads);
-    for (auto& th : pool) th.join();
-  }
+  return whole;
+}
+
+// Whether `box` holds the n points.
+bool holds(const double* box, const double* points, int64_t n) {
+  for (int64_t k = 0; k < n; ++k, points += 3)
+    for (int x = 0; x < 3; ++x)
+      if (!(points[x] >= box[x] && points[x] <= box[3 + x])) return false;
+  return true;
 }
 
 }  // namespace
 
 int64_t aabb_pack(const double* V, int64_t nv, const int64_t* F, int64_t nf, const double* boxes,
                   const int64_t* nodes, const int64_t* order, int64_t nnodes,
-                  AabbNodeRec* node_out, AabbTriRec* tri_out, double* scale, const char** why) {
+                  AabbNodeRec* node_out, AabbWalkRec* walk_out, AabbSpan* span_out,
+                  AabbTriRec* tri_out, double* scale, bool* regular, const char** why) {
+  *regular = false;
   *scale = 0.0;
   if (nnodes == 0) return 0;
   if (nnodes < 0 || nnodes > 0x7fffffffLL || nf <= 0 || nf > 0x7fffffffLL) {
@@ -330,7 +287,6 @@ int64_t aabb_pack(const double* V, int64_t nv, const int64_t* F, int64_t nf, con
     const int64_t* nd = nodes + 4 * i;
     AabbNodeRec& r = node_out[i];
     for (int k = 0; k < 6; ++k) r.lbox[k] = r.rbox[k] = 0.0;
-    for (int k = 0; k < 2; ++k) r.pad[k] = 0;
     if (level[i] == 0) {
       *why = "node unreachable from the root";
       return -1;
@@ -366,18 +322,35 @@ int64_t aabb_pack(const double* V, int64_t nv, const int64_t* F, int64_t nf, con
     *why = "tree deeper than the traversal stack";
     return -1;
   }
-  std::vector<AabbSlab> slabs;
-  build_slabs(tri_out, nodes, nnodes, *scale, slabs,
-              static_cast<int>(std::max(1u, std::thread::hardware_concurrency())));
+  bool sound = node_spans(nodes, nnodes, span_out);
+  const AabbDisc none{{0.f, 0.f, 0.f}, INFINITY, {0.f, 0.f, 0.f}, INFINITY};
   for (int64_t i = 0; i < nnodes; ++i) {
-    AabbNodeRec& r = node_out[i];
+    const AabbNodeRec& r = node_out[i];
+    AabbWalkRec& w = walk_out[i];
+    const double* box = boxes + 6 * i;
+    w.ldisc = w.rdisc = none;
+    w.start = r.start;
+    w.count = r.count;
     if (r.count > 0) {
-      r.lslab = r.rslab = AabbSlab{{0.f, 0.f, 0.f}, -INFINITY, INFINITY};
-    } else {
-      r.lslab = slabs[r.left];
-      r.rslab = slabs[r.right];
+      w.left = span_out[i].slot;
+      w.right = -1;
+      for (int k = 0; k < 6; ++k) w.lbox[k] = w.rbox[k] = 0.f;
+      for (int64_t k = r.start; sound && k < static_cast<int64_t>(r.start) + r.count; ++k)
+        sound = holds(box, tri_out[k].a, 3);  // the three corners lie behind each other
+      continue;
+    }
+    w.left = r.left;
+    w.right = r.right;
+    w.start = span_out[r.right].first;
+    sound = sound && holds(box, r.lbox, 2) && holds(box, r.rbox, 2);
+    for (int k = 0; k < 3; ++k) {
+      w.lbox[k] = round_down(r.lbox[k]);
+      w.rbox[k] = round_down(r.rbox[k]);
+      w.lbox[3 + k] = round_up(r.lbox[3 + k]);
+      w.rbox[3 + k] = round_up(r.rbox[3 + k]);
     }
   }
+  *regular = sound;
   return depth;
 }
 

@@ -1023,14 +1023,18 @@ int wn_aabb_create(const double* V, int64_t nv, const int64_t* F, int64_t nf,
     return fail(WN_EINVAL, "null pointer");
   std::vector<AabbNodeRec> nrec(static_cast<size_t>(nnodes));
   std::vector<AabbTriRec> trec(static_cast<size_t>(nnodes > 0 ? nf : 0));
+  std::vector<AabbWalkRec> wrec(static_cast<size_t>(nnodes));
+  std::vector<AabbSpan> spans(static_cast<size_t>(nnodes));
   const char* why = "";
   double scale = 0.0;
+  bool regular = false;
   const int64_t depth = aabb_pack(V, nv, F, nf, boxes, nodes, order, nnodes, nrec.data(),
-                                  trec.data(), &scale, &why);
+                                  wrec.data(), spans.data(), trec.data(), &scale, &regular, &why);
   if (depth < 0) return fail(WN_EINVAL, "invalid tree: %s", why);
   std::lock_guard<std::mutex> lock(g_mutex);
   int code = WN_OK;
-  if (!context(&code)) return code;
+  DeviceCtx* c = context(&code);
+  if (!c) return code;
   AabbHandle* h = new AabbHandle();
   cudaGetDevice(&h->device);
   h->t.nnodes = nnodes;
@@ -1039,18 +1043,49 @@ int wn_aabb_create(const double* V, int64_t nv, const int64_t* F, int64_t nf,
   h->t.scale = scale;
   if (nnodes > 0) {
     for (int k = 0; k < 6; ++k) h->t.root[k] = boxes[k];
+    std::vector<int32_t> big;  // nodes whose discs take a CTA each
+    if (regular)
+      for (int64_t i = 0; i < nnodes; ++i)
+        if (spans[i].last - spans[i].first > kDiscBig) big.push_back(static_cast<int32_t>(i));
+    const int64_t nbig = static_cast<int64_t>(big.size());
+    big.push_back(0);  // the flag for thin faces
+    AabbSpan* spans_d = nullptr;
+    int32_t* big_d = nullptr;
+    int32_t thin = 0;
     cudaError_t e;
     if ((e = dev_malloc(&h->t.nodes, sizeof(AabbNodeRec) * nrec.size())) != cudaSuccess ||
         (e = dev_malloc(&h->t.tris, sizeof(AabbTriRec) * trec.size())) != cudaSuccess ||
         (e = cudaMemcpy(h->t.nodes, nrec.data(), sizeof(AabbNodeRec) * nrec.size(),
                         cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemcpy(h->t.tris, trec.data(), sizeof(AabbTriRec) * trec.size(),
-                        cudaMemcpyHostToDevice)) != cudaSuccess) {
+                        cudaMemcpyHostToDevice)) != cudaSuccess ||
+        (regular &&
+         ((e = dev_malloc(&h->t.walk, sizeof(AabbWalkRec) * wrec.size())) != cudaSuccess ||
+          (e = cudaMemcpy(h->t.walk, wrec.data(), sizeof(AabbWalkRec) * wrec.size(),
+                          cudaMemcpyHostToDevice)) != cudaSuccess ||
+          (e = dev_malloc(&h->t.face_discs, sizeof(AabbDisc) * trec.size())) != cudaSuccess ||
+          (e = dev_malloc(&spans_d, sizeof(AabbSpan) * spans.size())) != cudaSuccess ||
+          (e = cudaMemcpy(spans_d, spans.data(), sizeof(AabbSpan) * spans.size(),
+                          cudaMemcpyHostToDevice)) != cudaSuccess ||
+          (e = dev_malloc(&big_d, sizeof(int32_t) * big.size())) != cudaSuccess ||
+          (e = cudaMemcpy(big_d, big.data(), sizeof(int32_t) * big.size(),
+                          cudaMemcpyHostToDevice)) != cudaSuccess ||
+          (e = aabb_discs(h->t, spans_d, big_d, nbig, big_d + nbig, c->stream)) != cudaSuccess ||
+          (e = cudaMemcpyAsync(&thin, big_d + nbig, sizeof(int32_t), cudaMemcpyDeviceToHost,
+                               c->stream)) != cudaSuccess ||
+          (e = cudaStreamSynchronize(c->stream)) != cudaSuccess))) {
+      cudaFree(spans_d);
+      cudaFree(big_d);
       cudaFree(h->t.nodes);
       cudaFree(h->t.tris);
+      cudaFree(h->t.walk);
+      cudaFree(h->t.face_discs);
       delete h;
       return cuda_fail(e, "device tree upload");
     }
+    cudaFree(spans_d);
+    cudaFree(big_d);
+    h->t.any_order = regular && thin == 0;
   }
   *tree = h;
   return WN_OK;
@@ -1065,6 +1100,8 @@ int wn_aabb_destroy(void* tree) {
   cudaDeviceSynchronize();
   cudaFree(h->t.nodes);
   cudaFree(h->t.tris);
+  cudaFree(h->t.walk);
+  cudaFree(h->t.face_discs);
   cudaSetDevice(prev);
   delete h;
   return WN_OK;
