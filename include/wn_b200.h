@@ -137,6 +137,7 @@ int wn_forward_fp64_device(const double* tri, int64_t ld, const double* q, doubl
  * beyond 1e75, or its scratch (about 450 bytes per face, 24 per query) could not be
  * allocated: then use one of the all-pairs entry points; mixed = 1 says that this
  * would be a mixed-precision one, which is harder to beat. Waits for the stream once. Device pointers; tri: 9 rows with row stride ld doubles. */
+int wn_exact_pays(int64_t nf, int64_t nq); /* 1: the sizes are worth the call */
 int wn_forward_exact_device(const double* tri, int64_t ld, const double* q, double* w, int64_t nf,
                             int64_t nq, int mixed, int* taken, void* stream);
 

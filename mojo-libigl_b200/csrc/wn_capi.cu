@@ -489,6 +489,8 @@ int wn_forward_fp64_device(const double* tri, int64_t ld, const double* q, doubl
   return e == cudaSuccess ? WN_OK : cuda_fail(e, "FP64 winding-number launch");
 }
 
+int wn_exact_pays(int64_t nf, int64_t nq) { return exact_pays(nf, nq) ? 1 : 0; }
+
 int wn_forward_exact_device(const double* tri, int64_t ld, const double* q, double* w, int64_t nf,
                             int64_t nq, int mixed, int* taken, void* stream) {
   WN_NVTX_RANGE();

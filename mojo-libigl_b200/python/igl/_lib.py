@@ -60,6 +60,7 @@ _WN_SIGNATURES = {
     "wn_probe_fma_tflops": ([C_INT, ctypes.POINTER(ctypes.c_double)], C_INT),
     "wn_forward_fp64_host": ([P, P, P, I, I, C_INT], C_INT),
     "wn_forward_fp64_device": ([P, I, P, P, I, I, C_INT, P], C_INT),
+    "wn_exact_pays": ([I, I], C_INT),
     "wn_forward_exact_device": ([P, I, P, P, I, I, C_INT, ctypes.POINTER(C_INT), P], C_INT),
     "wn_forward_mixed_host": ([P, P, P, I, I, ctypes.c_double], C_INT),
     "wn_mixed_mesh_create": ([P, I, I, ctypes.c_double, P, ctypes.POINTER(P)], C_INT),

@@ -106,13 +106,15 @@ def forward_exact(tri: torch.Tensor, ld: int, nf: int, O: torch.Tensor,
     within rounding of forward_fp64; None where an all-pairs kernel (mixed: the
     mixed-precision one) should run: small calls, faces that share no edges, a
     stream under capture."""
+    handle = _lib.lib()
+    if not handle.wn_exact_pays(nf, O.shape[0]):
+        return None
     q = O.to(torch.float64).contiguous()
     w = torch.empty(q.shape[0], dtype=torch.float64, device=q.device)
     taken = ctypes.c_int(0)
-    if q.shape[0] and nf:
-        _check(_lib.lib().wn_forward_exact_device(tri.data_ptr(), ld, q.data_ptr(), w.data_ptr(),
-                                                  nf, q.shape[0], int(mixed),
-                                                  ctypes.byref(taken), _stream()))
+    _check(handle.wn_forward_exact_device(tri.data_ptr(), ld, q.data_ptr(), w.data_ptr(), nf,
+                                          q.shape[0], int(mixed), ctypes.byref(taken),
+                                          _stream()))
     return w if taken.value else None
 
 
