@@ -657,12 +657,22 @@ __global__ void __launch_bounds__(THREADS, 2) adjoint_edges_kernel(const EdgeAdj
           const double qx = ev[k][3] - ox, qy = ev[k][4] - oy, qz = ev[k][5] - oz;
           const double pp = px * px + py * py + pz * pz;
           const double qq = qx * qx + qy * qy + qz * qz;
-          const double rp = rsqrt(pp), rq = rsqrt(qq);
-          const double rpq = rp * rq;
-          const double d = 1.0 + (px * qx + py * qy + pz * qz) * rpq;
+          const double pq = px * qx + py * qy + pz * qz;
+          double rp = rsqrt64(pp), rq = rsqrt64(qq);
+          double rpq = rp * rq;
+          double d = 1.0 + pq * rpq, rd = rcp64(d);
+          // Where d loses its digits (the query all but on the edge) its last ones
+          // matter: the library functions there, as in refine_edge_grad.
+          if (!(d > 1e-2)) {
+            rp = rsqrt(pp);
+            rq = rsqrt(qq);
+            rpq = rp * rq;
+            d = 1.0 + pq * rpq;
+            rd = 1.0 / d;
+          }
           // Zero for padding (m = 0) and where the derivative does not exist.
           const bool ok = ev[k][6] != 0.0 && pp > 0.0 && qq > 0.0 && d > 0.0;
-          const double w = ok ? g * ev[k][6] * rpq / d : 0.0;
+          const double w = ok ? g * ev[k][6] * rpq * rd : 0.0;
           const double cp = ok ? rp * w : 0.0, cq = ok ? rq * w : 0.0;
           const double x0 = py * qz - pz * qy, x1 = pz * qx - px * qz, x2 = px * qy - py * qx;
           acc[k][0] -= cp * x0;
@@ -758,6 +768,12 @@ __global__ void gather_vertex_kernel(const double* __restrict__ dtri, int64_t ld
 }
 
 constexpr int kAdjThreads = 128, kAdjFpt = 2, kAdjQc = 64;
+// Edges per thread of the FP64 edge adjoint: four share a query's dL/do reduction (15
+// shuffled additions), two CTAs per SM (4,572 edges x 100,003 queries, whole call: 3.35
+// ms with two edges and the library's rsqrt and division, 3.55 with four; with rsqrt64
+// and rcp64, the library's near d = 0 only, 2.57; without that branch 2.29, FP64 pipe
+// 74 %).
+constexpr int kAdjEpt = 4;
 
 int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
@@ -786,11 +802,11 @@ AdjointPlan plan_waves(int64_t nblocks, int64_t nq, int64_t slots, int64_t qc) {
 // against ngroups * elem_doubles of per-element partials (elem_doubles = 9 * ld for
 // faces), for about two waves of `slots` resident CTAs.
 AdjointPlan plan_balanced(int64_t nblocks, int64_t nq, int64_t slots, int64_t qc,
-                          int64_t elem_doubles) {
+                          int64_t elem_doubles, int waves = 2) {
   AdjointPlan p;
   nblocks = std::max<int64_t>(1, nblocks);
   nq = std::max<int64_t>(1, nq);
-  const int64_t target = 2 * std::max<int64_t>(1, slots);
+  const int64_t target = waves * std::max<int64_t>(1, slots);
   const double r = std::sqrt(static_cast<double>(target) * static_cast<double>(elem_doubles) /
                              (3.0 * static_cast<double>(nq)));
   const int64_t nranges =
@@ -856,9 +872,9 @@ cudaError_t adjoint_fp64(const AdjointPlan& p, const double* tri, int64_t ld, in
 
 AdjointPlan plan_adjoint_edges(int64_t ne, int64_t nq, int sms) {
   const int slots = resident_ctas(
-      reinterpret_cast<const void*>(adjoint_edges_kernel<kAdjThreads, kAdjFpt, kAdjQc>),
+      reinterpret_cast<const void*>(adjoint_edges_kernel<kAdjThreads, kAdjEpt, kAdjQc>),
       kAdjThreads, 0, sms);
-  return plan_waves(cdiv(ne, kAdjThreads * kAdjFpt), nq, slots, kAdjQc);
+  return plan_waves(cdiv(ne, kAdjThreads * kAdjEpt), nq, slots, kAdjQc);
 }
 
 size_t adjoint_edges_scratch_bytes(const AdjointPlan& p, int64_t le, int64_t nq) {
@@ -882,7 +898,7 @@ cudaError_t adjoint_edges(const AdjointPlan& p, const double* edges, int64_t le,
   if (e != cudaSuccess) return e;
   EdgeAdjointArgs a{edges, le, ne, q, gw, nq, p.blocks_per_range, p.queries_per_group,
                     dO_part, dE_part};
-  adjoint_edges_kernel<kAdjThreads, kAdjFpt, kAdjQc>
+  adjoint_edges_kernel<kAdjThreads, kAdjEpt, kAdjQc>
       <<<dim3(static_cast<unsigned>(p.nranges), static_cast<unsigned>(p.ngroups)), kAdjThreads, 0,
          stream>>>(a);
   finish_dq_kernel<<<static_cast<unsigned>(cdiv(nq * 3, 256)), 256, 0, stream>>>(dO_part, p.nranges,
@@ -1519,20 +1535,30 @@ __global__ void __launch_bounds__(kFaThreads, 5)
 }
 
 // dedge[row][edge_of[slot]] = (1/4pi) sum_g dE_part[g][row][slot] (sorted slots to input edges).
-__global__ void finish_dedge_sorted_kernel(const double* __restrict__ part, int64_t ngroups,
-                                           int64_t ld64, const uint32_t* __restrict__ edge_of,
-                                           int64_t le, double* __restrict__ dedge) {
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= 6 * ld64) return;
-  const int64_t r = i / ld64, sl = i % ld64;
-  const uint32_t e = edge_of[sl];
-  if (e == 0xffffffffu) return;
+// 32 slots x 8 slices of the groups: one thread for all of a slot's groups was a chain of
+// their loads (178 edges in 740 groups: 1.2 ms for the whole adjoint, 0.76 so).
+__global__ void __launch_bounds__(256) finish_dedge_sorted_kernel(
+    const double* __restrict__ part, int64_t ngroups, int64_t ld64,
+    const uint32_t* __restrict__ edge_of, int64_t le, double* __restrict__ dedge) {
+  __shared__ double slice[8][32];
+  const int64_t r = blockIdx.y, sl = static_cast<int64_t>(blockIdx.x) * 32 + threadIdx.x;
   double s = 0.0;
-  for (int64_t g = 0; g < ngroups; ++g) s += part[(g * 6 + r) * ld64 + sl];
-  dedge[r * le + e] = s * kInv4Pi;
+  for (int64_t g = threadIdx.y; g < ngroups; g += 8) s += part[(g * 6 + r) * ld64 + sl];
+  slice[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.y != 0) return;
+  for (int k = 1; k < 8; ++k) s += slice[k][threadIdx.x];
+  const uint32_t e = edge_of[sl];
+  if (e != 0xffffffffu) dedge[r * le + e] = s * kInv4Pi;
 }
 
 constexpr int kEaQc = kFaQc;
+// CTAs of the single-mesh kernel in resident waves. Those whose queries lie near their
+// edges take several times as long as the others, and with two waves the GPU waited for
+// them (30,720 welded edges x 131,072 near-surface queries: 12.2 ms; 4 waves 10.3, 8 9.0,
+// 16 8.0; 4,572 boundary edges x 262,144: 6.4, 5.8, 5.0, 4.7). Their partial sums grow
+// with the root of this.
+constexpr int kEdgeWaves = 16;
 constexpr int kEaQcNoDq = 32;  // without dL/do shares a 32-query chunk is cheap in shared memory
 
 // Scratch layout of adjoint_edges_mixed (each piece 256-byte aligned).
@@ -1577,7 +1603,7 @@ AdjointPlan plan_adjoint_edges_mixed(int64_t ne, int64_t nq, int sms, bool no_dq
   const int slots = resident_ctas(reinterpret_cast<const void*>(kernel), kFaThreads, smem, sms);
   const int64_t ntiles = std::max<int64_t>(1, cdiv(ne, kTileFaces));
   return plan_balanced(cdiv(ntiles, kFaTiles), nq, slots, no_dq ? kEaQcNoDq : kEaQc,
-                       6 * ntiles * kTileFaces);
+                       6 * ntiles * kTileFaces, kEdgeWaves);
 }
 
 size_t adjoint_edges_mixed_scratch_bytes(const AdjointPlan& p, int64_t ne, int64_t nq) {
@@ -1638,8 +1664,8 @@ cudaError_t adjoint_edges_mixed(const AdjointPlan& p, const double* edges, int64
   if (!no_dq)
     finish_dq_sorted_kernel<<<static_cast<unsigned>(cdiv(nq * 3, 256)), 256, 0, stream>>>(
         dO_part, p.nranges, nq, qperm, dq);
-  finish_dedge_sorted_kernel<<<static_cast<unsigned>(cdiv(6 * ld64, 256)), 256, 0, stream>>>(
-      dE_part, p.ngroups, ld64, edge_of, le, dedge);
+  finish_dedge_sorted_kernel<<<dim3(static_cast<unsigned>(cdiv(ld64, 32)), 6), dim3(32, 8), 0,
+                               stream>>>(dE_part, p.ngroups, ld64, edge_of, le, dedge);
   g_launches.fetch_add(no_dq ? 6 : 7, std::memory_order_relaxed);
   return cudaGetLastError();
 }

@@ -45,6 +45,7 @@
 
 #include <algorithm>
 
+#include "wn_common.cuh"
 #include "wn_exact.h"
 #include "wn_internal.h"
 #include "wn_pair.cuh"
@@ -973,18 +974,6 @@ __device__ __forceinline__ float mid_value(const float4* s, int sub, const float
     zi = ni;
   }
   return atan2f(zi, zr) * static_cast<float>(1.0 / kTwoPi) + static_cast<float>(turns);
-}
-
-// 1 / sqrt(x) in FP64 from the hardware's approximation by one step of Halley's
-// (third-order) iteration: with e = 1 - x y^2, y (1 + e/2 + 3 e^2/8) leaves a relative
-// error of 5 e^3 / 16, below rounding for e < 2^-18. 5 FP64 operations and no branch;
-// x = 0, a subnormal, infinity or NaN give NaN or infinity, which the callers' test of
-// the factor's size catches.
-__device__ __forceinline__ double rsqrt64(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x * y, y, 1.0);
-  return fma(y * e, fma(e, 0.375, 0.5), y);
 }
 
 // Running product of the boundary's z; `cond` keeps the smallest exponent seen.
