@@ -203,7 +203,7 @@ int wn_mixed_stats(int64_t* refined_pairs, int64_t* careful_visits, int reset);
  * a sequence of forwards can be captured in a CUDA graph.
  *   nv/nf/nq: host arrays of nmesh sizes; faces: host, total_nf x 3 int64,
  *   vertex indices local to each mesh (meshes concatenated in order).
- *   qpt: queries per thread (1, 2 or 4); target_pairs: pairs per work item;
+ *   qpt: queries per thread (1, 2 or 4); target_pairs: pairs per work item at most;
  *   ctas_per_sm: persistent CTAs per SM (0 = as many as fit); tile_faces: faces
  *   per far test and angle product, 64 or 32 (each half of a 64-face tile on its
  *   own).

@@ -1910,6 +1910,9 @@ __global__ void batch_finish_dedge_kernel(const double* __restrict__ dE_part,
   dedge[r * le + e] = s * kInv4Pi;
 }
 
+// Items per SM at least, so that the last ones end together (16 uneven meshes, 1.0e10
+// pairs: 6.06 ms at 8, 5.57 at 16, 5.40 at 64).
+constexpr int64_t kBatchItemsPerSm = 64;
 constexpr int64_t kBatchMixedBlocks = 16;     // largest item: 4-tile blocks per range
 constexpr int64_t kBatchMixedQueries = 4096;  // (4,096 edges) and sorted queries per group
 static_assert(kBatchMixedQueries % kFaFlushQueries == 0, "groups hold whole FP32 flushes");
@@ -2105,7 +2108,7 @@ cudaError_t batch_edges_create(BatchState* b, const int64_t* F) {
   std::vector<int32_t> tile_count, tile_mesh;
   std::vector<BatchMixedItem> mitems;
   {
-    // Item size: the largest that still gives at least 8 items per SM (halving the
+    // Item size: the largest that still gives kBatchItemsPerSm items (halving the
     // longer side, edges or queries, down to one block or one FP32 flush of queries).
     int64_t br = kBatchMixedBlocks, qg = kBatchMixedQueries;
     auto items_for = [&](int64_t r, int64_t g) {
@@ -2115,7 +2118,7 @@ cudaError_t batch_edges_create(BatchState* b, const int64_t* F) {
           n += cdiv(cdiv(cdiv(meshes[m].ne, kTileFaces), kFaTiles), r) * cdiv(meshes[m].nq, g);
       return n;
     };
-    const int64_t want = 8 * std::max(1, b->sms);
+    const int64_t want = kBatchItemsPerSm * std::max(1, b->sms);
     while (items_for(br, qg) < want && (br > 1 || qg > kFaFlushQueries)) {
       if (qg > kFaFlushQueries && (qg >= br * kFaTiles * kTileFaces || br == 1))
         qg /= 2;

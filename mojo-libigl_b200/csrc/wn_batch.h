@@ -29,7 +29,7 @@ struct BatchMeshInfo {
 
 struct BatchPlan {
   int qpt = 2;
-  int64_t target_pairs = int64_t(1) << 23;  // pairs per work item
+  int64_t target_pairs = int64_t(1) << 23;  // pairs per work item at most
   int ctas_per_sm = 0;                      // 0 = as many as fit
   double kappa = 4.0;
   int tile_faces = 64;                      // 64, or 32: far test and angle per half tile
