@@ -657,22 +657,12 @@ __global__ void __launch_bounds__(THREADS, 2) adjoint_edges_kernel(const EdgeAdj
           const double qx = ev[k][3] - ox, qy = ev[k][4] - oy, qz = ev[k][5] - oz;
           const double pp = px * px + py * py + pz * pz;
           const double qq = qx * qx + qy * qy + qz * qz;
-          const double pq = px * qx + py * qy + pz * qz;
-          double rp = rsqrt64(pp), rq = rsqrt64(qq);
-          double rpq = rp * rq;
-          double d = 1.0 + pq * rpq, rd = rcp64(d);
-          // Where d loses its digits (the query all but on the edge) its last ones
-          // matter: the library functions there, as in refine_edge_grad.
-          if (!(d > 1e-2)) {
-            rp = rsqrt(pp);
-            rq = rsqrt(qq);
-            rpq = rp * rq;
-            d = 1.0 + pq * rpq;
-            rd = 1.0 / d;
-          }
+          const double rp = rsqrt(pp), rq = rsqrt(qq);
+          const double rpq = rp * rq;
+          const double d = 1.0 + (px * qx + py * qy + pz * qz) * rpq;
           // Zero for padding (m = 0) and where the derivative does not exist.
           const bool ok = ev[k][6] != 0.0 && pp > 0.0 && qq > 0.0 && d > 0.0;
-          const double w = ok ? g * ev[k][6] * rpq * rd : 0.0;
+          const double w = ok ? g * ev[k][6] * rpq / d : 0.0;
           const double cp = ok ? rp * w : 0.0, cq = ok ? rq * w : 0.0;
           const double x0 = py * qz - pz * qy, x1 = pz * qx - px * qz, x2 = px * qy - py * qx;
           acc[k][0] -= cp * x0;
@@ -768,12 +758,6 @@ __global__ void gather_vertex_kernel(const double* __restrict__ dtri, int64_t ld
 }
 
 constexpr int kAdjThreads = 128, kAdjFpt = 2, kAdjQc = 64;
-// Edges per thread of the FP64 edge adjoint: four share a query's dL/do reduction (15
-// shuffled additions), two CTAs per SM (4,572 edges x 100,003 queries, whole call: 3.35
-// ms with two edges and the library's rsqrt and division, 3.55 with four; with rsqrt64
-// and rcp64, the library's near d = 0 only, 2.57; without that branch 2.29, FP64 pipe
-// 74 %).
-constexpr int kAdjEpt = 4;
 
 int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
@@ -800,7 +784,7 @@ AdjointPlan plan_waves(int64_t nblocks, int64_t nq, int64_t slots, int64_t qc) {
 // Like plan_waves, but the split between face ranges and query groups balances the
 // two partial arrays the split creates: nranges * nq * 3 doubles of dL/do partials
 // against ngroups * elem_doubles of per-element partials (elem_doubles = 9 * ld for
-// faces), for about two waves of `slots` resident CTAs.
+// faces), for about `waves` waves of `slots` resident CTAs.
 AdjointPlan plan_balanced(int64_t nblocks, int64_t nq, int64_t slots, int64_t qc,
                           int64_t elem_doubles, int waves = 2) {
   AdjointPlan p;
@@ -872,9 +856,9 @@ cudaError_t adjoint_fp64(const AdjointPlan& p, const double* tri, int64_t ld, in
 
 AdjointPlan plan_adjoint_edges(int64_t ne, int64_t nq, int sms) {
   const int slots = resident_ctas(
-      reinterpret_cast<const void*>(adjoint_edges_kernel<kAdjThreads, kAdjEpt, kAdjQc>),
+      reinterpret_cast<const void*>(adjoint_edges_kernel<kAdjThreads, kAdjFpt, kAdjQc>),
       kAdjThreads, 0, sms);
-  return plan_waves(cdiv(ne, kAdjThreads * kAdjEpt), nq, slots, kAdjQc);
+  return plan_waves(cdiv(ne, kAdjThreads * kAdjFpt), nq, slots, kAdjQc);
 }
 
 size_t adjoint_edges_scratch_bytes(const AdjointPlan& p, int64_t le, int64_t nq) {
@@ -898,7 +882,7 @@ cudaError_t adjoint_edges(const AdjointPlan& p, const double* edges, int64_t le,
   if (e != cudaSuccess) return e;
   EdgeAdjointArgs a{edges, le, ne, q, gw, nq, p.blocks_per_range, p.queries_per_group,
                     dO_part, dE_part};
-  adjoint_edges_kernel<kAdjThreads, kAdjEpt, kAdjQc>
+  adjoint_edges_kernel<kAdjThreads, kAdjFpt, kAdjQc>
       <<<dim3(static_cast<unsigned>(p.nranges), static_cast<unsigned>(p.ngroups)), kAdjThreads, 0,
          stream>>>(a);
   finish_dq_kernel<<<static_cast<unsigned>(cdiv(nq * 3, 256)), 256, 0, stream>>>(dO_part, p.nranges,
