@@ -784,13 +784,19 @@ AdjointPlan plan_waves(int64_t nblocks, int64_t nq, int64_t slots, int64_t qc) {
 // Like plan_waves, but the split between face ranges and query groups balances the
 // two partial arrays the split creates: nranges * nq * 3 doubles of dL/do partials
 // against ngroups * elem_doubles of per-element partials (elem_doubles = 9 * ld for
-// faces), for about `waves` waves of `slots` resident CTAs.
+// faces), for about `waves` waves of `slots` resident CTAs (two, if more would leave a
+// CTA less than kLeastPairs pairs: its partial sums would cost more than they).
+constexpr int64_t kBlockElems = kFaTiles * kTileFaces;
+constexpr int64_t kLeastPairs = 1 << 17;
 AdjointPlan plan_balanced(int64_t nblocks, int64_t nq, int64_t slots, int64_t qc,
                           int64_t elem_doubles, int waves = 2) {
   AdjointPlan p;
   nblocks = std::max<int64_t>(1, nblocks);
   nq = std::max<int64_t>(1, nq);
-  const int64_t target = waves * std::max<int64_t>(1, slots);
+  int64_t target = 2 * std::max<int64_t>(1, slots);
+  if (waves > 2)  // but no CTA of less than kLeastPairs for it
+    target = std::max(target, std::min<int64_t>(waves * std::max<int64_t>(1, slots),
+                                                nblocks * kBlockElems * nq / kLeastPairs));
   const double r = std::sqrt(static_cast<double>(target) * static_cast<double>(elem_doubles) /
                              (3.0 * static_cast<double>(nq)));
   const int64_t nranges =
