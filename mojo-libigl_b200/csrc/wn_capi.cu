@@ -236,12 +236,12 @@ int forward_fp64_host(const double* tri, const double* q, double* w, int64_t nf,
           (e = cudaMemcpyAsync(c->q.ptr, q, sizeof(double) * 3 * nq, cudaMemcpyHostToDevice,
                                c->stream)) != cudaSuccess)
         return cuda_fail(e, "copy of the inputs");
-      int64_t nitem = -1;
-      if ((e = exact_build(xp, tri_d, ld, q_d, c->scratch.ptr, kExactMostFp64, &nitem,
+      ExactBoundary boundary;
+      if ((e = exact_build(xp, tri_d, ld, q_d, c->scratch.ptr, kExactMostFp64, &boundary,
                            c->stream)) != cudaSuccess)
         return cuda_fail(e, "mesh preparation");
-      if (nitem >= 0) {
-        if ((e = exact_eval(xp, nitem, q_d, w_d, c->scratch.ptr, c->sms, c->stream)) != cudaSuccess)
+      if (boundary.items >= 0) {
+        if ((e = exact_eval(xp, boundary, q_d, w_d, c->scratch.ptr, c->sms, c->stream)) != cudaSuccess)
           return cuda_fail(e, "exact winding-number launch");
         if ((e = cudaMemcpyAsync(w, w_d, sizeof(double) * nq, cudaMemcpyDeviceToHost,
                                  c->stream)) != cudaSuccess)
@@ -521,12 +521,13 @@ int wn_forward_exact_device(const double* tri, int64_t ld, const double* q, doub
     cudaGetLastError();
     return WN_OK;  // the caller's all-pairs path needs less memory
   }
-  int64_t nitem = -1;
-  e = exact_build(p, tri, ld, q, scratch, mixed ? kExactMostMixed : kExactMostFp64, &nitem, st);
-  if (e == cudaSuccess && nitem >= 0) e = exact_eval(p, nitem, q, w, scratch, sms, st);
+  ExactBoundary boundary;
+  e = exact_build(p, tri, ld, q, scratch, mixed ? kExactMostMixed : kExactMostFp64, &boundary,
+                  st);
+  if (e == cudaSuccess && boundary.items >= 0) e = exact_eval(p, boundary, q, w, scratch, sms, st);
   cudaFreeAsync(scratch, st);
   if (e != cudaSuccess) return cuda_fail(e, "exact winding-number launch");
-  *taken = nitem >= 0 ? 1 : 0;
+  *taken = boundary.items >= 0 ? 1 : 0;
   return WN_OK;
 }
 

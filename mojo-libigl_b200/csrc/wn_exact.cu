@@ -57,11 +57,11 @@ constexpr int kLeaf = kExactLeafFaces;
 constexpr int kLeafEdges = 3 * kLeaf;
 constexpr int kWarps = 4;            // warps per CTA
 constexpr int kStack = 1536;         // node stack of a warp
-constexpr float kPad = 0.1f;         // near box: the leaf's box grown by kPad * diagonal
+constexpr float kPad = 0.05f;        // near box: the leaf's box grown by kPad * diagonal
 constexpr float kPadAbs = 1e-6f;     // ... and by this much of the mesh's extent
 constexpr float kSlack = 3e-7f;      // FP32 rounding of node centres (|p| <= 1)
 constexpr float kBeta = 2.5f;        // a node is far when d >= beta * r
-constexpr float kMaxBound = 0.4f;    // proven error of W_far below which k is certain
+constexpr float kMaxBound = 0.45f;   // proven error of W_far below which k is certain
 constexpr int kBetaTries = 4;        // beta = 2.5, 3.25, 4.55, 9.1
 constexpr int kDirTries = 4;
 constexpr int kMinExp = (1023 - 7) << 20;  // |z_e| >= ~2^-7, else try another direction
@@ -116,11 +116,18 @@ static_assert(sizeof(Face32) == 64, "a leaf's faces are one 16-byte word per lan
 // boxes of the edges' leaves, and the edges.
 struct alignas(16) Group {
   float lo[3], hi[3];
-  int32_t first, count;
+  int32_t first, count, triangle, pad[3];  // first edge, edges, first triangle of its fan
 };
 struct Root {
   double u[3], v[3];
 };
+// Triangle (A, A + e1, A + e2) of a loop's fan, with n = e1 x e2 and the sides' products:
+// with a = A - o the pair needs |a|^2, a.e1, a.e2 and a.n only (50 FP64 operations with
+// the product; 63 from the corners).
+struct alignas(16) Triangle {
+  double a[3], e1[3], e2[3], n[3], e11, e22, e12, pad;
+};
+static_assert(sizeof(Triangle) == 128, "eight 16-byte words");
 
 __device__ __forceinline__ unsigned long long okey(double x) {
   const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(x));
@@ -421,6 +428,16 @@ __global__ void exact_partner_kernel(const Face64* __restrict__ faces, int64_t n
   nb[e] = rank < nopp && other != leaf ? static_cast<int32_t>(other) : -1;
 }
 
+// What a leaf's sides lead, and (exclusive sums) what comes before it.
+struct Counts {
+  int32_t groups, edges, triangles;
+};
+struct AddCounts {
+  __host__ __device__ __forceinline__ Counts operator()(const Counts& a, const Counts& b) const {
+    return Counts{a.groups + b.groups, a.edges + b.edges, a.triangles + b.triangles};
+  }
+};
+
 __device__ __forceinline__ uint32_t point_slot(const double* v, uint32_t mask) {
   return (point_hash(v) * 0x9e3779b1u >> 7) & mask;
 }
@@ -513,14 +530,14 @@ __global__ void exact_successor_kernel(const Face64* __restrict__ faces, int64_t
   succ[e] = s;
 }
 
-// Per leaf: the groups it leads and their edges, packed (groups << 32 | edges); and
+// Per leaf: the groups it leads, their edges and their triangles (Counts); and
 // per side how many edges the group it leads has (0: leads none). A loop's leader
 // is its side of the smallest number. As many root edges enter a point as leave it,
 // so a loop is left and entered at one place each.
 __global__ void exact_loops_kernel(const uint32_t* __restrict__ partner,
                                    const uint32_t* __restrict__ succ, int64_t nedge,
                                    uint8_t* __restrict__ lead,
-                                   unsigned long long* __restrict__ counts, Info* info) {
+                                   Counts* __restrict__ counts, Info* info) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const uint32_t e = static_cast<uint32_t>(i);
   int count = 0;
@@ -538,7 +555,12 @@ __global__ void exact_loops_kernel(const uint32_t* __restrict__ partner,
     }
     if (count < 3) count = 1;
     else if (!smallest) count = 0;
-    if (count) atomicAdd(counts + e / kLeafEdges, (1ull << 32) | static_cast<unsigned>(count));
+    if (count) {
+      Counts* c = counts + e / kLeafEdges;
+      atomicAdd(&c->groups, 1);
+      atomicAdd(&c->edges, count);
+      if (count > 1) atomicAdd(&c->triangles, count - 2);
+    }
   }
   if (i < nedge) lead[e] = static_cast<uint8_t>(count);
   const int edges = __reduce_add_sync(~0u, count);
@@ -698,55 +720,70 @@ __global__ void __launch_bounds__(64) exact_leaf_kernel(
   moments[leaf] = m;
 }
 
-// A node from its children: areas and boxes unite, moments shift to the common
-// centre.
+// A node from its children, by one warp: areas and boxes unite, moments shift to the
+// common centre. A lane takes a component (a thread per node took the whole
+// chain of loads alone: 83 us for the last six levels of a 20,480-face mesh).
 __device__ __forceinline__ void merge_node(int64_t first, int count, Moments* moments,
                                            NodeTest* test, int64_t node) {
-  Moments m = {};
-  NodeTest t;
-  for (int x = 0; x < 3; ++x) {
-    t.lo[x] = INFINITY;
-    t.hi[x] = -INFINITY;
-  }
-  double mean[3] = {0, 0, 0};
+  const int lane = threadIdx.x & 31;
+  double area = 0.0, p[3] = {0, 0, 0}, mean[3] = {0, 0, 0};
   for (int k = 0; k < count; ++k) {
     const Moments& c = moments[first + k];
-    m.area += c.area;
+    area += c.area;
     for (int x = 0; x < 3; ++x) {
-      m.p[x] += c.area * c.p[x];
+      p[x] += c.area * c.p[x];
       mean[x] += c.p[x];
-      t.lo[x] = fminf(t.lo[x], test[first + k].lo[x]);
-      t.hi[x] = fmaxf(t.hi[x], test[first + k].hi[x]);
     }
   }
-  for (int x = 0; x < 3; ++x) {
-    m.p[x] = m.area > 0.0 ? m.p[x] / m.area : mean[x] / count;
-    t.p[x] = static_cast<float>(m.p[x]);
-  }
-  for (int k = 0; k < count; ++k) {
-    const Moments& c = moments[first + k];
-    const double s[3] = {c.p[0] - m.p[0], c.p[1] - m.p[1], c.p[2] - m.p[2]};
-    for (int i = 0; i < 3; ++i) {
-      m.m0[i] += c.m0[i];
-      for (int j = 0; j < 3; ++j) m.m1[j][i] += c.m1[j][i] + s[j] * c.m0[i];
-      for (int j = 0; j < 3; ++j)
-        for (int k2 = j; k2 < 3; ++k2)
-          m.m2[kSym[j][k2]][i] += c.m2[kSym[j][k2]][i] +
-                                  0.5 * (s[j] * c.m1[k2][i] + s[k2] * c.m1[j][i]) +
-                                  0.5 * s[j] * s[k2] * c.m0[i];
+  for (int x = 0; x < 3; ++x) p[x] = area > 0.0 ? p[x] / area : mean[x] / count;
+  Moments& out = moments[node];
+  if (lane < 3) {  // m0
+    double v = 0.0;
+    for (int k = 0; k < count; ++k) v += moments[first + k].m0[lane];
+    out.m0[lane] = v;
+    out.p[lane] = p[lane];
+    if (lane == 0) out.area = area;
+  } else if (lane < 12) {  // m1[j][i]
+    const int j = (lane - 3) / 3, i = (lane - 3) % 3;
+    double v = 0.0;
+    for (int k = 0; k < count; ++k) {
+      const Moments& c = moments[first + k];
+      v += c.m1[j][i] + (c.p[j] - p[j]) * c.m0[i];
     }
+    out.m1[j][i] = v;
+  } else if (lane < 30) {  // m2[jk][i]
+    const int jk = (lane - 12) / 3, i = (lane - 12) % 3;
+    const int j = jk < 3 ? 0 : (jk < 5 ? 1 : 2), l = jk < 3 ? jk : (jk < 5 ? jk - 2 : 2);
+    double v = 0.0;
+    for (int k = 0; k < count; ++k) {
+      const Moments& c = moments[first + k];
+      const double sj = c.p[j] - p[j], sl = c.p[l] - p[l];
+      v += c.m2[jk][i] + 0.5 * (sj * c.m1[l][i] + sl * c.m1[j][i]) + 0.5 * sj * sl * c.m0[i];
+    }
+    out.m2[jk][i] = v;
+  } else if (lane == 30) {
+    NodeTest t;
+    for (int x = 0; x < 3; ++x) {
+      t.lo[x] = INFINITY;
+      t.hi[x] = -INFINITY;
+      t.p[x] = static_cast<float>(p[x]);
+    }
+    for (int k = 0; k < count; ++k)
+      for (int x = 0; x < 3; ++x) {
+        t.lo[x] = fminf(t.lo[x], test[first + k].lo[x]);
+        t.hi[x] = fmaxf(t.hi[x], test[first + k].hi[x]);
+      }
+    t.r = 0.0f;
+    t.area = 0.0f;
+    t.child = static_cast<int32_t>(first << 2) | (count - 1);
+    test[node] = t;
   }
-  t.r = 0.0f;
-  t.area = 0.0f;
-  t.child = static_cast<int32_t>(first << 2) | (count - 1);
-  test[node] = t;
-  moments[node] = m;
 }
 
-__global__ void __launch_bounds__(64) exact_level_kernel(int64_t child_off, int64_t child_n,
-                                                         int64_t off, int64_t n,
-                                                         Moments* moments, NodeTest* test) {
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(128) exact_level_kernel(int64_t child_off, int64_t child_n,
+                                                          int64_t off, int64_t n,
+                                                          Moments* moments, NodeTest* test) {
+  const int64_t i = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / 32;
   if (i >= n) return;
   const int64_t c0 = i * kExactArity;
   merge_node(child_off + c0, static_cast<int>(min(static_cast<int64_t>(kExactArity), child_n - c0)),
@@ -758,10 +795,10 @@ struct Levels {
   int64_t off[kExactMaxLevels], n[kExactMaxLevels];
 };
 // The few nodes of the top levels, one CTA level by level.
-__global__ void __launch_bounds__(256) exact_top_kernel(const Levels a, int first_level,
-                                                        Moments* moments, NodeTest* test) {
+__global__ void __launch_bounds__(1024) exact_top_kernel(const Levels a, int first_level,
+                                                         Moments* moments, NodeTest* test) {
   for (int l = first_level; l < a.nlevel; ++l) {
-    for (int64_t i = threadIdx.x; i < a.n[l]; i += blockDim.x) {
+    for (int64_t i = threadIdx.x / 32; i < a.n[l]; i += blockDim.x / 32) {
       const int64_t c0 = i * kExactArity;
       merge_node(a.off[l - 1] + c0,
                  static_cast<int>(min(static_cast<int64_t>(kExactArity), a.n[l - 1] - c0)),
@@ -815,52 +852,74 @@ __global__ void __launch_bounds__(64) exact_finish_kernel(int64_t nnode,
   finish_node(moments[i], r, eval + i);
 }
 
-// The groups that a leaf's sides lead and their edges, in face order behind each
-// other; `first` is the exclusive sum of the leaves' packed counts.
-__global__ void exact_groups_kernel(const Face64* __restrict__ faces, int64_t nf, int64_t nleaf,
+// The groups, a thread per side: what a leaf's sides lead lies behind each other in side
+// order, from `first` (the exclusive sum of the leaves' counts).
+__global__ void exact_groups_kernel(const Face64* __restrict__ faces, int64_t nedge, int64_t nleaf,
                                     const uint32_t* __restrict__ succ,
                                     const uint8_t* __restrict__ lead,
-                                    const unsigned long long* __restrict__ counts,
-                                    const unsigned long long* __restrict__ first,
-                                    int64_t max_roots, const NodeTest* __restrict__ test,
-                                    Group* __restrict__ groups, Root* __restrict__ roots,
-                                    int32_t* __restrict__ root_leaf, Info* info) {
-  const int64_t leaf = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (leaf >= nleaf) return;
-  const unsigned long long n = counts[leaf], at0 = first[leaf];
-  if (leaf == nleaf - 1) info->ngroup = static_cast<int32_t>((at0 + n) >> 32);
-  if (n == 0) return;
-  int64_t g = static_cast<int64_t>(at0 >> 32), at = static_cast<int64_t>(at0 & 0xffffffffull);
-  const int64_t e1 = min((leaf + 1) * kLeafEdges, 3 * nf);
-  for (int64_t e = leaf * kLeafEdges; e < e1; ++e) {
-    const int count = lead[e];
-    if (count == 0) continue;
-    if (at + count <= max_roots) {  // more than that: the result is not used
-      Group o;
-      for (int x = 0; x < 3; ++x) {
-        o.lo[x] = INFINITY;
-        o.hi[x] = -INFINITY;
-      }
-      o.first = static_cast<int32_t>(at);
-      o.count = count;
-      uint32_t s = static_cast<uint32_t>(e);
-      for (int k = 0; k < count; ++k) {
-        const double *u = corner_of(faces, s, 0), *v = corner_of(faces, s, 1);
-        const uint32_t l = s / kLeafEdges;
-        for (int x = 0; x < 3; ++x) {
-          roots[at + k].u[x] = u[x];
-          roots[at + k].v[x] = v[x];
-          o.lo[x] = fminf(o.lo[x], test[l].lo[x]);
-          o.hi[x] = fmaxf(o.hi[x], test[l].hi[x]);
-        }
-        root_leaf[at + k] = static_cast<int32_t>(l);
-        if (k + 1 < count) s = succ[s];
-      }
-      groups[g] = o;
-    }
-    ++g;
-    at += count;
+                                    const Counts* __restrict__ counts,
+                                    const Counts* __restrict__ first, int64_t max_roots,
+                                    const NodeTest* __restrict__ test, Group* __restrict__ groups,
+                                    Root* __restrict__ roots, int32_t* __restrict__ root_leaf,
+                                    Triangle* __restrict__ triangles, Info* info) {
+  const int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (e == 0) info->ngroup = first[nleaf - 1].groups + counts[nleaf - 1].groups;
+  if (e >= nedge) return;
+  const int count = lead[e];
+  if (count == 0) return;
+  const int64_t leaf = e / kLeafEdges;
+  Counts at = first[leaf];
+  for (int64_t o = leaf * kLeafEdges; o < e; ++o) {
+    const int c = lead[o];
+    if (c == 0) continue;
+    ++at.groups;
+    at.edges += c;
+    at.triangles += c > 1 ? c - 2 : 0;
   }
+  if (at.edges + count > max_roots) return;  // more than that: the result is not used
+  Group g;
+  for (int x = 0; x < 3; ++x) {
+    g.lo[x] = INFINITY;
+    g.hi[x] = -INFINITY;
+  }
+  g.first = at.edges;
+  g.count = count;
+  g.triangle = at.triangles;
+  g.pad[0] = g.pad[1] = g.pad[2] = 0;
+  uint32_t s = static_cast<uint32_t>(e);
+  double a[3] = {0.0, 0.0, 0.0};
+  for (int k = 0; k < count; ++k) {
+    const double *u = corner_of(faces, s, 0), *v = corner_of(faces, s, 1);
+    const uint32_t l = s / kLeafEdges;
+    for (int x = 0; x < 3; ++x) {
+      roots[at.edges + k].u[x] = u[x];
+      roots[at.edges + k].v[x] = v[x];
+      g.lo[x] = fminf(g.lo[x], test[l].lo[x]);
+      g.hi[x] = fmaxf(g.hi[x], test[l].hi[x]);
+    }
+    root_leaf[at.edges + k] = static_cast<int32_t>(l);
+    if (k == 0) {
+      for (int x = 0; x < 3; ++x) a[x] = u[x];
+    } else if (k + 1 < count) {
+      // Triangle k of the fan: the loop's first vertex and this edge.
+      Triangle t;
+      for (int x = 0; x < 3; ++x) {
+        t.a[x] = a[x];
+        t.e1[x] = u[x] - a[x];
+        t.e2[x] = v[x] - a[x];
+      }
+      t.n[0] = t.e1[1] * t.e2[2] - t.e1[2] * t.e2[1];
+      t.n[1] = t.e1[2] * t.e2[0] - t.e1[0] * t.e2[2];
+      t.n[2] = t.e1[0] * t.e2[1] - t.e1[1] * t.e2[0];
+      t.e11 = t.e1[0] * t.e1[0] + t.e1[1] * t.e1[1] + t.e1[2] * t.e1[2];
+      t.e22 = t.e2[0] * t.e2[0] + t.e2[1] * t.e2[1] + t.e2[2] * t.e2[2];
+      t.e12 = t.e1[0] * t.e2[0] + t.e1[1] * t.e2[1] + t.e1[2] * t.e2[2];
+      t.pad = 0.0;
+      triangles[at.triangles + k - 1] = t;
+    }
+    if (k + 1 < count) s = succ[s];
+  }
+  groups[at.groups] = g;
 }
 
 // ---- evaluation ------------------------------------------------------------------
@@ -874,6 +933,7 @@ struct EvalArgs {
   const Group* groups;
   const Root* roots;
   const int32_t* root_leaf;
+  const Triangle* triangles;
   const double* q;
   const uint32_t* perm;
   double* w;
@@ -1028,40 +1088,26 @@ __device__ __forceinline__ void push_edge(EdgeProduct& p, const Dir& D, double q
   multiply(p, 1.0 + uv * s + du * ru + dv * rv, (px * wy - py * wx) * (s * D.z));
 }
 
-struct Corner64 {
-  double x, y, z, r;  // corner - query, 1 / length
-};
-__device__ __forceinline__ Corner64 corner64(double qx, double qy, double qz, double x, double y,
-                                             double z) {
-  x -= qx; y -= qy; z -= qz;
-  return Corner64{x, y, z, rsqrt64(x * x + y * y + z * z)};
-}
-__device__ __forceinline__ double dot64(const Corner64& a, const Corner64& b) {
-  return a.x * b.x + a.y * b.y + a.z * b.z;
-}
-__device__ __forceinline__ void push_triangle(EdgeProduct& p, const Corner64& a, const Corner64& b,
-                                              const Corner64& c) {
-  const double det = a.x * (b.y * c.z - b.z * c.y) - a.y * (b.x * c.z - b.z * c.x) +
-                     a.z * (b.x * c.y - b.y * c.x);
-  const double rab = a.r * b.r;
-  multiply(p, 1.0 + dot64(a, b) * rab + dot64(b, c) * (b.r * c.r) + dot64(c, a) * (c.r * a.r),
-           det * (rab * c.r));
-}
-// Multiplies in triangle k (from 1) of the fan of a loop from its first vertex.
-__device__ __forceinline__ void push_fan(EdgeProduct& p, double qx, double qy, double qz,
-                                         const Root* r, int k) {
-  const double2* s = reinterpret_cast<const double2*>(r);
-  const double2 a0 = __ldg(s);
-  const double a1 = __ldg(&r->u[2]);
-  const double2* t = reinterpret_cast<const double2*>(r + k);
-  const double2 b0 = __ldg(t), bc = __ldg(t + 1), c1 = __ldg(t + 2);
-  push_triangle(p, corner64(qx, qy, qz, a0.x, a0.y, a1), corner64(qx, qy, qz, b0.x, b0.y, bc.x),
-                corner64(qx, qy, qz, bc.y, c1.x, c1.y));
+// Multiplies in the pair term of a fan triangle, scaled by its lengths.
+__device__ __forceinline__ void push_triangle(EdgeProduct& p, double qx, double qy, double qz,
+                                              const Triangle* t) {
+  const double2* s = reinterpret_cast<const double2*>(t);
+  const double2 s0 = s[0], s1 = s[1], s2 = s[2], s3 = s[3], s4 = s[4], s5 = s[5], s6 = s[6];
+  const double e12 = t->e12;
+  const double ax = s0.x - qx, ay = s0.y - qy, az = s1.x - qz;
+  const double aa = ax * ax + ay * ay + az * az;
+  const double a1 = ax * s1.y + ay * s2.x + az * s2.y;
+  const double a2 = ax * s3.x + ay * s3.y + az * s4.x;
+  const double an = ax * s4.y + ay * s5.x + az * s5.y;
+  const double ab = aa + a1, ac = aa + a2;
+  const double ra = rsqrt64(aa), rb = rsqrt64(ab + a1 + s6.x), rc = rsqrt64(ac + a2 + s6.y);
+  const double rab = ra * rb;
+  multiply(p, 1.0 + ab * rab + (ab + a2 + e12) * (rb * rc) + ac * (rc * ra), an * (rab * rc));
 }
 
 enum WalkMode : int { kWalkFar = 1, kWalkNear = 2, kWalkEdges = 4 };
 
-constexpr int kStage = 32 * 7;  // 16-byte words: 32 expansions, or one leaf's faces
+constexpr int kStage = 32 * 8;  // 16-byte words: 32 triangles or expansions, a leaf's faces
 
 struct WarpMem {
   float4 stage[kStage];
@@ -1078,14 +1124,18 @@ struct WarpMem {
 // read: the launch chooses by the queries' spacing.
 //
 // 327,680 faces x 2^20 queries: a warp of 16 queries takes ~550 expansions, ~48 leaves
-// in FP32, ~10 near leaves and ~60 edges in place of 327,680 faces; 5.6 ms with the
+// in FP32, ~10 near leaves and ~60 edges in place of 327,680 faces; 4.6 ms with the
 // preparation, where the all-pairs kernels take 410 (mixed) and 1,884 (FP64). 18,842
-// faces with 1,638 holes x 2^20 queries: ~1,607 fan triangles a query, 11.0 ms against
-// 108 (FP64 pairs). Bound there by FP64 and its latency (ncu, 131,072 queries: FP64 pipe
-// 47 %, issue 48 %, 20 warps per SM at 96 registers). Reading each expansion's seven
-// words with every lane instead of staging 32 of them cost 11.6 against 6.4 ms.
+// faces with 1,638 holes x 2^20 queries: ~1,607 fan triangles a query, 9.2 ms against
+// 108 (FP64 pairs). Bound by FP64 and latency there (ncu, 131,072 queries: FP64 pipe
+// 44 %, issue 49 %). Reading each expansion's seven words with every lane instead of
+// staging 32 of them cost 11.6 against 6.4 ms. Four CTAs per SM of 128 registers: with
+// five of 96 spills cost 5.7 against 5.4 ms, with six of 80 6.3. kPad: 0.2 / 0.1 / 0.05 /
+// 0.03 of the diagonal 6.1 / 5.7 / 5.5 / 5.4 ms, at the price of nearer FP32 leaves; kBeta
+// 2.25 / 2.5 / 2.75 7.3 / 5.7 / 5.3 ms (too many second walks below), with kMaxBound 0.45
+// in place of 0.4 5.1 at 2.5; 18,842 faces prefer the smaller kBeta (9.5 / 9.8 / 10.0).
 template <int SUB>
-__global__ void __launch_bounds__(32 * kWarps, 5) exact_eval_kernel(const EvalArgs a) {
+__global__ void __launch_bounds__(32 * kWarps, 4) exact_eval_kernel(const EvalArgs a) {
   __shared__ WarpMem mem[kWarps];
   constexpr int kQueries = 32 / SUB;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1269,13 +1319,14 @@ __global__ void __launch_bounds__(32 * kWarps, 5) exact_eval_kernel(const EvalAr
       for (int32_t g0 = 0; g0 < ngroup; g0 += 32) {
         // A lane's group: as a fan when it is not near; else its edges one by one, but
         // for those of near leaves (bit j of `edges`: edge j).
-        int fan = 0, first = 0;
+        int fan = 0, first = 0, triangle = 0;
         unsigned edges = 0;
         if (g0 + lane < ngroup) {
           const Group* g = a.groups + g0 + lane;
           const bool near = box_near(g, box);
           const int2 fc = __ldg(reinterpret_cast<const int2*>(&g->first));
           first = fc.x;
+          triangle = __ldg(&g->triangle);
           if (fc.y == 1) {
             edges = near ? 0u : 1u;
           } else if (!near) {
@@ -1285,9 +1336,8 @@ __global__ void __launch_bounds__(32 * kWarps, 5) exact_eval_kernel(const EvalAr
               edges |= box_near(a.test + __ldg(a.root_leaf + first + j), box) ? 0u : 1u << j;
           }
         }
-        // Both kinds as lists in shared memory, 64 entries at a time: triangles
-        // (first edge << 3 | triangle) and edges. `mine` places a lane's entries behind
-        // those of the lanes before it.
+        // Both kinds as lists in shared memory, 64 entries at a time. `mine` places a
+        // lane's entries behind those of the lanes before it.
         auto place = [&](int count, int& total) {
           int upto = count;
           for (int o = 1; o < 32; o <<= 1) {
@@ -1302,17 +1352,36 @@ __global__ void __launch_bounds__(32 * kWarps, 5) exact_eval_kernel(const EvalAr
         for (int t0 = 0; t0 < total; t0 += 64) {
           for (int k = 0; k < fan; ++k) {
             const int to = mine + k - t0;
-            if (to >= 0 && to < 64) m.farl[to] = static_cast<uint32_t>(first) << 3 | (k + 1);
+            if (to >= 0 && to < 64) m.farl[to] = static_cast<uint32_t>(triangle + k);
           }
           __syncwarp();
           const int n = min(total - t0, 64);
+          if constexpr (SUB >= 4) {
+            // Few queries to a warp: every lane reads its own.
 #pragma unroll 2
-          for (int k = sub; k < n; k += SUB) {
-            const uint32_t ft = m.farl[k];
-            push_fan(fans, qx, qy, qz, a.roots + (ft >> 3), ft & 7u);
+            for (int k = sub; k < n; k += SUB)
+              push_triangle(fans, qx, qy, qz, a.triangles + m.farl[k]);
+            __syncwarp();
+          } else {
+            // Through shared memory, 32 at a time (read by every lane from L1 they cost
+            // 12.3 ms instead of 9.8, 18,842 F with 1,638 holes x 2^20 Q).
+            for (int u0 = 0; u0 < n; u0 += 32) {
+              const int cnt = min(n - u0, 32);
+#pragma unroll
+              for (int k = 0; k < 8; ++k) {
+                const int word = 32 * k + lane;
+                if (word / 8 < cnt)
+                  m.stage[word] = __ldg(reinterpret_cast<const float4*>(
+                                            a.triangles + m.farl[u0 + word / 8]) + word % 8);
+              }
+              __syncwarp();
+#pragma unroll 2
+              for (int k = sub; k < cnt; k += SUB)
+                push_triangle(fans, qx, qy, qz, reinterpret_cast<const Triangle*>(m.stage) + k);
+              __syncwarp();
+            }
           }
           rescale(fans);
-          __syncwarp();
         }
         mine = place(__popc(edges), total);
         for (int t0 = 0; t0 < total; t0 += 64) {
@@ -1429,7 +1498,7 @@ unsigned blocks(int64_t n, int threads) {
 // Where the method starts to pay (one B200, meshes of 1,280 to 327,680 faces, closed,
 // open and terrain grids; ms, the faster all-pairs kernel -> this one): 20,480 F x
 // 8,192 Q 1.21 -> 0.54, 81,920 F x 4,096 Q 2.4 -> 0.8, 28,322 F (grid) x 8,192 Q 1.6 ->
-// 1.0; below the line 28,322 F x 4,096 Q 0.83 -> 1.09, 5,120 F x 8,192 Q 0.37 -> 0.38.
+// 0.58; below the line 5,120 F x 8,192 Q 0.37 -> 0.38.
 // Fewer queries than 4,096 leave too few warps and wide boxes: 243,602 F (grid) x
 // 2,048 Q 3.5 -> 4.1.
 bool exact_pays(int64_t nf, int64_t nq) {
@@ -1472,11 +1541,12 @@ ExactPlan plan_exact(int64_t nf, int64_t nq) {
   p.moments = take(sizeof(Moments) * node);
   p.test = take(sizeof(NodeTest) * node);
   p.eval = take(sizeof(NodeEval) * node);
-  p.counts = take(sizeof(unsigned long long) * leaf);
-  p.first = take(sizeof(unsigned long long) * leaf);
+  p.counts = take(sizeof(Counts) * leaf);
+  p.first = take(sizeof(Counts) * leaf);
   p.groups = take(sizeof(Group) * static_cast<size_t>(p.max_roots + 1));
   p.roots = take(sizeof(Root) * static_cast<size_t>(p.max_roots + 1));
   p.root_leaf = take(sizeof(int32_t) * static_cast<size_t>(p.max_roots + 1));
+  p.triangles = take(sizeof(Triangle) * static_cast<size_t>(p.max_roots + 1));
   p.perm = take(sizeof(uint32_t) * q);
   p.list = take(sizeof(uint32_t) * q);
   const size_t m = std::max(f, q);
@@ -1492,9 +1562,9 @@ ExactPlan plan_exact(int64_t nf, int64_t nq) {
   cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, static_cast<uint32_t*>(nullptr),
                                   static_cast<uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr),
                                   static_cast<uint32_t*>(nullptr), static_cast<int>(m), 0, 30);
-  cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, static_cast<unsigned long long*>(nullptr),
-                                static_cast<unsigned long long*>(nullptr),
-                                static_cast<int>(p.nleaf));
+  cub::DeviceScan::ExclusiveScan(nullptr, scan_bytes, static_cast<Counts*>(nullptr),
+                                 static_cast<Counts*>(nullptr), AddCounts(), Counts{0, 0, 0},
+                                 static_cast<int>(p.nleaf));
   p.cub_bytes = std::max(sort_bytes, scan_bytes);
   p.cub = take(p.cub_bytes);
   p.bytes = at;
@@ -1509,15 +1579,14 @@ T* at(void* scratch, size_t offset) {
 }  // namespace
 
 cudaError_t exact_build(const ExactPlan& p, const double* tri, int64_t ld, const double* q,
-                        void* scratch, double most, int64_t* nitem, cudaStream_t stream) {
-  using u64 = unsigned long long;
+                        void* scratch, double most, ExactBoundary* boundary, cudaStream_t stream) {
   Info* info = at<Info>(scratch, p.info);
   Face64* faces = at<Face64>(scratch, p.faces64);
   uint32_t* partner = at<uint32_t>(scratch, p.partner);
   uint8_t* lead = at<uint8_t>(scratch, p.lead);
   Moments* moments = at<Moments>(scratch, p.moments);
   NodeTest* test = at<NodeTest>(scratch, p.test);
-  u64 *counts = at<u64>(scratch, p.counts), *first = at<u64>(scratch, p.first);
+  Counts *counts = at<Counts>(scratch, p.counts), *first = at<Counts>(scratch, p.first);
   uint32_t *keys_in = at<uint32_t>(scratch, p.keys_in), *keys_out = at<uint32_t>(scratch, p.keys_out);
   uint32_t *vals_in = at<uint32_t>(scratch, p.vals_in), *vals_out = at<uint32_t>(scratch, p.vals_out);
   uint32_t *heads = at<uint32_t>(scratch, p.heads), *next = at<uint32_t>(scratch, p.next);
@@ -1534,7 +1603,7 @@ cudaError_t exact_build(const ExactPlan& p, const double* tri, int64_t ld, const
   cudaError_t e;
   exact_init_kernel<<<1, 32, 0, stream>>>(info);
   if ((e = cudaMemsetAsync(heads, 0xff, sizeof(uint32_t) * p.hash_slots, stream)) != cudaSuccess ||
-      (e = cudaMemsetAsync(counts, 0, sizeof(u64) * p.nleaf, stream)) != cudaSuccess)
+      (e = cudaMemsetAsync(counts, 0, sizeof(Counts) * p.nleaf, stream)) != cudaSuccess)
     return e;
   exact_face_box_kernel<<<std::min(blocks(p.nf, th), 592u), th, 0, stream>>>(tri, ld, p.nf, info);
   exact_face_keys_kernel<<<blocks(p.nf, th), th, 0, stream>>>(tri, ld, p.nf, info, keys_in,
@@ -1566,32 +1635,33 @@ cudaError_t exact_build(const ExactPlan& p, const double* tri, int64_t ld, const
     return e;
   const bool fit = !host.bad && host.nroot <= p.max_roots &&
                    static_cast<double>(host.nitem) <= most * static_cast<double>(p.nf);
-  *nitem = fit ? host.nitem : -1;
+  boundary->items = fit ? host.nitem : -1;
+  boundary->loops = (host.nroot - host.nitem) / 2;  // a loop of n edges: n - 2 triangles
   if (!fit) return cudaSuccess;
   tb = p.cub_bytes;
-  if ((e = cub::DeviceScan::ExclusiveSum(temp, tb, counts, first, static_cast<int>(p.nleaf),
-                                         stream)) != cudaSuccess)
+  if ((e = cub::DeviceScan::ExclusiveScan(temp, tb, counts, first, AddCounts(), Counts{0, 0, 0},
+                                          static_cast<int>(p.nleaf), stream)) != cudaSuccess)
     return e;
   exact_leaf_kernel<<<blocks(p.nleaf, 64), 64, 0, stream>>>(faces, p.nf, p.nleaf, info, moments,
                                                             test, at<Face32>(scratch, p.faces32));
   int l = 1;
-  for (; l < p.nlevel && p.level_n[l] > 1024; ++l) {
-    exact_level_kernel<<<blocks(p.level_n[l], 64), 64, 0, stream>>>(
+  for (; l < p.nlevel && p.level_n[l] > 64; ++l) {
+    exact_level_kernel<<<blocks(p.level_n[l], 4), 128, 0, stream>>>(
         p.level_off[l - 1], p.level_n[l - 1], p.level_off[l], p.level_n[l], moments, test);
     g_launches.fetch_add(1, std::memory_order_relaxed);
   }
   if (l < p.nlevel) {
-    exact_top_kernel<<<1, 256, 0, stream>>>(levels, l, moments, test);
+    exact_top_kernel<<<1, 1024, 0, stream>>>(levels, l, moments, test);
     g_launches.fetch_add(1, std::memory_order_relaxed);
   }
   exact_radius_kernel<<<blocks(p.nf, th), th, 0, stream>>>(faces, p.nf, levels, info, moments,
                                                            test);
   exact_finish_kernel<<<blocks(p.nnode, 64), 64, 0, stream>>>(p.nnode, moments, test,
                                                               at<NodeEval>(scratch, p.eval));
-  exact_groups_kernel<<<blocks(p.nleaf, 128), 128, 0, stream>>>(
-      faces, p.nf, p.nleaf, succ, lead, counts, first, p.max_roots, test,
+  exact_groups_kernel<<<blocks(3 * p.nf, th), th, 0, stream>>>(
+      faces, 3 * p.nf, p.nleaf, succ, lead, counts, first, p.max_roots, test,
       at<Group>(scratch, p.groups), at<Root>(scratch, p.roots), at<int32_t>(scratch, p.root_leaf),
-      info);
+      at<Triangle>(scratch, p.triangles), info);
   exact_query_box_kernel<<<std::min(blocks(p.nq, th), 592u), th, 0, stream>>>(q, p.nq, info);
   exact_query_keys_kernel<<<blocks(p.nq, th), th, 0, stream>>>(q, p.nq, info, keys_in, vals_in);
   tb = p.cub_bytes;
@@ -1612,21 +1682,26 @@ void launch_eval(const EvalArgs& a, cudaStream_t stream) {
 }  // namespace
 
 // Lanes per query. More of them shrink the warp's box and fill the GPU where queries
-// are few, but every warp walks the tree and reads the mesh's boundary for itself. With
-// one lane per query as the start: without a boundary, enough warps for two waves (s7,
-// 65,536 Q: 3.4 / 2.5 / 1.9 / 1.7 ms at 1 / 2 / 4 / 8 lanes; 16,384 Q: 6.2 / 2.8 / 1.7 /
-// 1.2) and still two lanes while queries are sparse against the faces (327,680 F x 2^20
-// Q: 6.4 / 5.7 ms; 20,480 F x 2^20 Q: 2.6 / 2.8); with one, a single wave (28,322 F grid
-// x 65,536 Q: 1.9 / 1.7 / 1.9 / 2.8 ms; 2^20 Q: 8.6 / 11.8).
-static int lanes_per_query(const ExactPlan& p, int64_t nitem) {
-  const bool closed = nitem < 64;
-  const int64_t enough = closed ? 262144 : 131072;
+// are few, but every warp walks the tree and reads the mesh's boundary for itself.
+// Measured at 1 / 2 / 4 / 8 lanes, ms:
+//   closed   327,680 F x 16,384 Q 4.4 / 2.5 / 1.5 / 1.1   x 131,072 3.1 / 2.0 / 1.8 / 1.8
+//            x 2^20 5.1 / 4.6 / 5.6 / 7.8; 20,480 F x 2^20 2.3 / 2.5 / 3.4 / 5.3
+//   edges    28,322 F (terrain) x 16,384 1.5 / 0.86 / 0.68 / 0.70   x 65,536 1.4 / 1.0 /
+//            1.1 / 1.4   x 2^20 6.7 / 7.3 / 9.6 / 14.9;
+//            243,602 F x 131,072 5.7 / 4.8, x 262,144 8.2 / 7.2
+//   holes    19,456 F x 16,384 1.05 / 0.77 / 0.78 / 0.99   x 65,536 1.2 / 1.1 / 1.6 / 2.6
+//            x 2^20 6.5 / 7.8 / 18.3 / 34.4
+static int lanes_per_query(const ExactPlan& p, const ExactBoundary& boundary) {
+  const bool closed = boundary.items < 64, holes = 4 * boundary.loops > boundary.items;
+  const int64_t enough = closed ? 262144 : (holes ? 32768 : 131072);
   int sub = 1;
   while (sub < 8 && p.nq * sub < enough) sub *= 2;
-  return closed && sub == 1 && p.nq < 8 * p.nf ? 2 : sub;
+  if (closed && sub < 8 && 2 * p.nq < p.nf) sub *= 2;
+  if (sub == 1 && p.nq < (closed ? 8 * p.nf : std::max<int64_t>(100000, holes ? 0 : p.nf + p.nf / 8))) sub = 2;
+  return sub;
 }
 
-cudaError_t exact_eval(const ExactPlan& p, int64_t nitem, const double* q, double* w,
+cudaError_t exact_eval(const ExactPlan& p, const ExactBoundary& boundary, const double* q, double* w,
                        void* scratch, int sms, cudaStream_t stream) {
   EvalArgs a;
   a.faces = at<Face64>(scratch, p.faces64);
@@ -1637,6 +1712,7 @@ cudaError_t exact_eval(const ExactPlan& p, int64_t nitem, const double* q, doubl
   a.groups = at<Group>(scratch, p.groups);
   a.roots = at<Root>(scratch, p.roots);
   a.root_leaf = at<int32_t>(scratch, p.root_leaf);
+  a.triangles = at<Triangle>(scratch, p.triangles);
   a.q = q;
   a.perm = at<uint32_t>(scratch, p.perm);
   a.w = w;
@@ -1645,7 +1721,7 @@ cudaError_t exact_eval(const ExactPlan& p, int64_t nitem, const double* q, doubl
   a.nf = p.nf;
   a.nq = p.nq;
   a.top = p.nnode - 1;
-  switch (lanes_per_query(p, nitem)) {
+  switch (lanes_per_query(p, boundary)) {
     case 1: launch_eval<1>(a, stream); break;
     case 2: launch_eval<2>(a, stream); break;
     case 4: launch_eval<4>(a, stream); break;

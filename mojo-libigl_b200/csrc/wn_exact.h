@@ -22,7 +22,7 @@ struct ExactPlan {
   int64_t max_roots = 0;   // root edges kept; more than this and the method is not taken
   uint32_t hash_slots = 0;  // a power of two
   size_t info, faces64, faces32, partner, nb, lead, moments, test, eval, counts, first, groups,
-      roots, root_leaf;
+      roots, root_leaf, triangles;
   size_t keys_in, keys_out, vals_in, vals_out, heads, next, pick, succ, perm, list, cub;
   size_t cub_bytes = 0, bytes = 0;
 };
@@ -38,15 +38,21 @@ ExactPlan plan_exact(int64_t nf, int64_t nq);
 // 262,144 queries: 47 ms against 440 and 94).
 constexpr double kExactMostFp64 = 0.55, kExactMostMixed = 0.13;
 
-// Pairs the mesh's edges, waits for the stream and reports in *nitem the triangles and
-// single edges of the boundary; -1 if they are more than `most` per face or the mesh is
-// not fit for the method (nothing further is done then). Else builds the tree and the
-// query order in `scratch` (plan.bytes).
+// What the boundary costs a query: triangles and single edges, and the loops that the
+// triangles fan.
+struct ExactBoundary {
+  int64_t items = -1, loops = 0;
+};
+
+// Pairs the mesh's edges, waits for the stream and reports the boundary; items = -1 if
+// they are more than `most` per face or the mesh is not fit for the method (nothing
+// further is done then). Else builds the tree and the query order in `scratch`
+// (plan.bytes).
 cudaError_t exact_build(const ExactPlan& p, const double* tri, int64_t ld, const double* q,
-                        void* scratch, double most, int64_t* nitem, cudaStream_t stream);
+                        void* scratch, double most, ExactBoundary* boundary, cudaStream_t stream);
 
 // W of the queries (in the order given) after exact_build on the same stream.
-cudaError_t exact_eval(const ExactPlan& p, int64_t nitem, const double* q, double* w,
-                       void* scratch, int sms, cudaStream_t stream);
+cudaError_t exact_eval(const ExactPlan& p, const ExactBoundary& boundary, const double* q,
+                       double* w, void* scratch, int sms, cudaStream_t stream);
 
 }  // namespace wn
