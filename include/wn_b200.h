@@ -275,6 +275,34 @@ int wn_gather_vertex_grad_device(const double* grad, int64_t ld, int corners,
                                  const int64_t* indptr, const int64_t* entries, int64_t nv,
                                  double* dV, void* stream);
 
+/* The edges of a mesh in device memory, for the edge adjoints above. F (nf,3) int64 and
+ * V (nv,3) double; 1 <= nf <= 2^28, 1 <= nv <= 2^29. Counting and writing are two calls
+ * on one scratch block (device memory, 256-byte aligned, kept unchanged in between); the
+ * counts wait for the stream, so they are refused under capture.
+ * wn_edges_scratch_bytes: kind 0 boundary, 1 weld, 2 gather of nf edges, 3 gather of nf
+ * faces; 0 for sizes out of range.
+ * boundary: *ne edges {u < v} whose sides do not cancel, or -1 for an index outside
+ * [0, nv); then edges (7, le) as above and ends (ne,2), in the order of (u, v).
+ * weld: sides of equal endpoint coordinates share an edge. counts[0] edges with net count
+ * 0 (-1 for a bad index), counts[1] others; the write gives (7, counts[0]) and behind it
+ * (7, counts[1]). The scratch keeps each side's edge for wn_gather_welded_device, whose
+ * dedge is (6, counts[0]) and behind it (6, counts[1]), from unit-weight adjoints.
+ * gather: dV (nv,3), each vertex's terms added in a fixed order. */
+int64_t wn_edges_scratch_bytes(int kind, int64_t nf, int64_t nv);
+int wn_boundary_count_device(const int64_t* F, int64_t nf, int64_t nv, void* scratch,
+                             int64_t* ne, void* stream);
+int wn_boundary_write_device(const double* V, int64_t nf, int64_t nv, const void* scratch,
+                             double* edges, int64_t le, int64_t* ends, void* stream);
+int wn_weld_count_device(const double* V, const int64_t* F, int64_t nf, int64_t nv,
+                         void* scratch, int64_t* counts, void* stream);
+int wn_weld_write_device(const double* V, int64_t nf, int64_t nv, int64_t cancelled,
+                         int64_t others, void* scratch, double* edges, void* stream);
+int wn_gather_edges_device(const double* dedge, int64_t le, const int64_t* ends, int64_t ne,
+                           int64_t nv, void* scratch, double* dV, void* stream);
+int wn_gather_welded_device(const double* dedge, int64_t cancelled, int64_t others,
+                            const int64_t* F, int64_t nf, int64_t nv,
+                            const void* weld_scratch, void* scratch, double* dV, void* stream);
+
 /* ---- closest points over the median-split hierarchy ---------------------
  * V: nv x 3 doubles; F: nf x 3 int64; P: np x 3 doubles. Tree arrays as the
  * reference's python/igl/__init__.py:286-319 `_build_aabb` returns them:

@@ -21,6 +21,7 @@
 #include "../../include/wn_b200.h"
 #include "wn_aabb.h"
 #include "wn_adjoint.h"
+#include "wn_edges.h"
 #include "wn_exact.h"
 #include "wn_fwn.h"
 #include "wn_normals.h"
@@ -843,6 +844,82 @@ int wn_gather_vertex_grad_device(const double* dtri, int64_t ld, int corners,
     return fail(WN_EINVAL, "bad nv=%lld or corners=%d", (long long)nv, corners);
   cudaError_t e = gather_vertex_grad(dtri, ld, corners, indptr, entries, nv, dV,
                                      static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? WN_OK : cuda_fail(e, "vertex gradient gather");
+}
+
+int64_t wn_edges_scratch_bytes(int kind, int64_t nf, int64_t nv) {
+  if (!edges_fit(nf, nv)) return 0;
+  switch (kind) {
+    case 0: return static_cast<int64_t>(boundary_scratch_bytes(nf, nv));
+    case 1: return static_cast<int64_t>(weld_scratch_bytes(nf, nv));
+    default: return static_cast<int64_t>(gather_scratch_bytes(kind == 2 ? 2 * nf : 3 * nf));
+  }
+}
+
+int wn_boundary_count_device(const int64_t* F, int64_t nf, int64_t nv, void* scratch, int64_t* ne,
+                             void* stream) {
+  WN_NVTX_RANGE();
+  if (!edges_fit(nf, nv) || !F || !scratch || !ne)
+    return fail(WN_EINVAL, "bad nf=%lld or nv=%lld, or a null pointer", (long long)nf,
+                (long long)nv);
+  cudaError_t e = boundary_count(F, nf, nv, scratch, ne, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? WN_OK : cuda_fail(e, "boundary edges");
+}
+
+int wn_boundary_write_device(const double* V, int64_t nf, int64_t nv, const void* scratch,
+                             double* edges, int64_t le, int64_t* ends, void* stream) {
+  WN_NVTX_RANGE();
+  if (!edges_fit(nf, nv) || !V || !scratch || !edges || !ends || le < 1)
+    return fail(WN_EINVAL, "bad nf=%lld, nv=%lld or le=%lld, or a null pointer", (long long)nf,
+                (long long)nv, (long long)le);
+  cudaError_t e =
+      boundary_write(V, nf, nv, scratch, edges, le, ends, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? WN_OK : cuda_fail(e, "boundary edges");
+}
+
+int wn_weld_count_device(const double* V, const int64_t* F, int64_t nf, int64_t nv, void* scratch,
+                         int64_t* counts, void* stream) {
+  WN_NVTX_RANGE();
+  if (!edges_fit(nf, nv) || !V || !F || !scratch || !counts)
+    return fail(WN_EINVAL, "bad nf=%lld or nv=%lld, or a null pointer", (long long)nf,
+                (long long)nv);
+  cudaError_t e =
+      weld_count(V, F, nf, nv, scratch, counts, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? WN_OK : cuda_fail(e, "welded edges");
+}
+
+int wn_weld_write_device(const double* V, int64_t nf, int64_t nv, int64_t cancelled,
+                         int64_t others, void* scratch, double* edges, void* stream) {
+  WN_NVTX_RANGE();
+  if (!edges_fit(nf, nv) || cancelled < 0 || others < 0 || !V || !scratch || !edges)
+    return fail(WN_EINVAL, "bad nf=%lld, nv=%lld or counts, or a null pointer", (long long)nf,
+                (long long)nv);
+  cudaError_t e = weld_write(V, nf, nv, cancelled, others, scratch, edges,
+                             static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? WN_OK : cuda_fail(e, "welded edges");
+}
+
+int wn_gather_edges_device(const double* dedge, int64_t le, const int64_t* ends, int64_t ne,
+                           int64_t nv, void* scratch, double* dV, void* stream) {
+  WN_NVTX_RANGE();
+  if (!edges_fit(ne, nv) || le < ne || !dedge || !ends || !scratch || !dV)
+    return fail(WN_EINVAL, "bad ne=%lld, nv=%lld or le=%lld, or a null pointer", (long long)ne,
+                (long long)nv, (long long)le);
+  cudaError_t e =
+      gather_edges(dedge, le, ends, ne, nv, scratch, dV, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? WN_OK : cuda_fail(e, "vertex gradient gather");
+}
+
+int wn_gather_welded_device(const double* dedge, int64_t cancelled, int64_t others,
+                            const int64_t* F, int64_t nf, int64_t nv, const void* weld_scratch,
+                            void* scratch, double* dV, void* stream) {
+  WN_NVTX_RANGE();
+  if (!edges_fit(nf, nv) || cancelled < 0 || others < 0 || !dedge || !F || !weld_scratch ||
+      !scratch || !dV)
+    return fail(WN_EINVAL, "bad nf=%lld, nv=%lld or counts, or a null pointer", (long long)nf,
+                (long long)nv);
+  cudaError_t e = gather_welded(dedge, cancelled, others, F, nf, nv, weld_scratch, scratch, dV,
+                                static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? WN_OK : cuda_fail(e, "vertex gradient gather");
 }
 

@@ -74,6 +74,13 @@ _WN_SIGNATURES = {
     "wn_mixed_stats": ([ctypes.POINTER(I), ctypes.POINTER(I), C_INT], C_INT),
     "wn_backward_fp64_device": ([P, I, I, P, I, P, P, P, P], C_INT),
     "wn_gather_vertex_grad_device": ([P, I, C_INT, P, P, I, P, P], C_INT),
+    "wn_edges_scratch_bytes": ([C_INT, I, I], I),
+    "wn_boundary_count_device": ([P, I, I, P, ctypes.POINTER(I), P], C_INT),
+    "wn_boundary_write_device": ([P, I, I, P, P, I, P, P], C_INT),
+    "wn_weld_count_device": ([P, P, I, I, P, ctypes.POINTER(I), P], C_INT),
+    "wn_weld_write_device": ([P, I, I, I, I, P, P, P], C_INT),
+    "wn_gather_edges_device": ([P, I, P, I, I, P, P, P], C_INT),
+    "wn_gather_welded_device": ([P, I, I, P, I, I, P, P, P, P], C_INT),
     "wn_backward_edges_device": ([P, I, I, P, I, P, P, P, P], C_INT),
     "wn_backward_edges_mixed_device": ([P, I, I, P, I, P, ctypes.c_double, C_INT, P, P, P],
                                        C_INT),

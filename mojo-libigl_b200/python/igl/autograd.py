@@ -180,11 +180,56 @@ def gather_vertices(dtri, ld, nf, F, nv, corners=3):
     return dV
 
 
+class _Boundary(tuple):
+    """boundary_edges' result from the library's kernels: its vertices are in [0, nv)."""
+
+    nv = -1
+
+
+def _scratch(kind: int, nf: int, V: torch.Tensor) -> torch.Tensor | None:
+    """Scratch of the mesh-edge kernels (wn_edges.cu); None off the GPU and for sizes
+    that they do not take."""
+    if not V.is_cuda:
+        return None
+    size = _lib.lib().wn_edges_scratch_bytes(kind, nf, V.shape[0])
+    return torch.empty(size, dtype=torch.uint8, device=V.device) if size else None
+
+
+def _boundary_edges_device(V, F):
+    """boundary_edges by the library's kernels; None where they do not apply."""
+    scratch = _scratch(0, F.shape[0], V) if F.device == V.device else None
+    if scratch is None:
+        return None
+    handle, nf, nv = _lib.lib(), F.shape[0], V.shape[0]
+    F64 = F.to(torch.int64).contiguous()
+    Vd = V.detach().to(torch.float64).contiguous()
+    count = ctypes.c_int64(-1)
+    _check(handle.wn_boundary_count_device(F64.data_ptr(), nf, nv, scratch.data_ptr(),
+                                           ctypes.byref(count), _stream()))
+    ne = count.value
+    if ne < 0:
+        return None  # an index out of range: the general path's answer
+    ends = torch.empty((ne, 2), dtype=torch.int64, device=V.device)
+    if not ne:
+        edges = torch.zeros((7, 1), dtype=torch.float64, device=V.device)
+    else:
+        edges = torch.empty((7, ne), dtype=torch.float64, device=V.device)
+        _check(handle.wn_boundary_write_device(Vd.data_ptr(), nf, nv, scratch.data_ptr(),
+                                               edges.data_ptr(), ne, ends.data_ptr(),
+                                               _stream()))
+    out = _Boundary((edges, ne, ends))
+    out.nv = nv
+    return out
+
+
 def boundary_edges(V: torch.Tensor, F: torch.Tensor):
     """Undirected edges {u < v} with net multiplicity m = #(u->v) - #(v->u) != 0.
 
     Returns (edges (7, le) float64 SoA: V[u], V[v], m; ne; endpoints (ne, 2) int64).
     """
+    found = _boundary_edges_device(V, F)
+    if found is not None:
+        return found
     nv = V.shape[0]
     e = torch.cat([F[:, [0, 1]], F[:, [1, 2]], F[:, [2, 0]]]).to(torch.int64)
     e = e[e[:, 0] != e[:, 1]]
@@ -216,7 +261,8 @@ def backward_edges(V, F, O, gW, edges=None, precision: str = "fp64", kappa: floa
     q = O.to(torch.float64).contiguous()
     gw = gW.to(torch.float64).contiguous()
     nq, nv = q.shape[0], V.shape[0]
-    edges, ne, ends = edges if edges is not None else boundary_edges(V, F)
+    found = edges if edges is not None else boundary_edges(V, F)
+    edges, ne, ends = found
     le = edges.shape[1]
     dq = torch.empty((nq, 3), dtype=torch.float64, device=q.device)
     dedge = torch.zeros((6, le), dtype=torch.float64, device=q.device)
@@ -228,7 +274,13 @@ def backward_edges(V, F, O, gW, edges=None, precision: str = "fp64", kappa: floa
         _check(handle.wn_backward_edges_device(edges.data_ptr(), le, ne, q.data_ptr(), nq,
                                                gw.data_ptr(), dq.data_ptr(), dedge.data_ptr(),
                                                _stream()))
-    return gather_vertices(dedge, le, ne, ends, nv, corners=2), dq
+    scratch = _scratch(2, ne, V) if getattr(found, "nv", -1) == nv else None
+    if scratch is None:
+        return gather_vertices(dedge, le, ne, ends, nv, corners=2), dq
+    dV = torch.empty((nv, 3), dtype=torch.float64, device=q.device)
+    _check(handle.wn_gather_edges_device(dedge.data_ptr(), le, ends.data_ptr(), ne, nv,
+                                         scratch.data_ptr(), dV.data_ptr(), _stream()))
+    return dV, dq
 
 
 def welded_edges(V: torch.Tensor, F: torch.Tensor):
@@ -271,6 +323,72 @@ def welded_edges(V: torch.Tensor, F: torch.Tensor):
     return edges, ng, side_edge, sigma, torch.stack([a, b], 1)
 
 
+class _Weld:
+    """The sides welded by position, by the library's kernels: `cancelled` edges with
+    m = 0, then `others`. The scratch block keeps each side's edge."""
+
+    def __init__(self, V, F, scratch):
+        handle = _lib.lib()
+        self.F = F.to(torch.int64).contiguous()
+        self.V = V.detach().to(torch.float64).contiguous()
+        self.scratch = scratch
+        counts = (ctypes.c_int64 * 2)()
+        _check(handle.wn_weld_count_device(self.V.data_ptr(), self.F.data_ptr(), F.shape[0],
+                                           V.shape[0], scratch.data_ptr(), counts, _stream()))
+        self.cancelled, self.others = counts
+
+    def __getitem__(self, i):  # [1]: the number of edges, as in welded_edges' result
+        return (None, self.cancelled + self.others)[i]
+
+
+def _weld(V, F):
+    """The welded sides of (V, F) for backward_welded_edges."""
+    scratch = _scratch(1, F.shape[0], V) if F.device == V.device else None
+    weld = _Weld(V, F, scratch) if scratch is not None else None
+    if weld is None or weld.cancelled < 0:  # off the GPU, or an index out of range
+        return welded_edges(V, F)
+    return weld
+
+
+def _backward_weld(weld, O, gW, kappa):
+    """(dL/dV, dL/dO) from a _Weld."""
+    handle = _lib.lib()
+    q = O.to(torch.float64).contiguous()
+    gw = gW.to(torch.float64).contiguous()
+    nf, nv, nq = weld.F.shape[0], weld.V.shape[0], q.shape[0]
+    n0, n1 = weld.cancelled, weld.others
+    dq = torch.zeros((nq, 3), dtype=torch.float64, device=q.device)
+    dV = torch.zeros((nv, 3), dtype=torch.float64, device=q.device)
+    if not n0 + n1:
+        return dV, dq
+    edges = torch.empty(7 * (n0 + n1), dtype=torch.float64, device=q.device)
+    dedge = torch.empty(6 * (n0 + n1), dtype=torch.float64, device=q.device)
+    _check(handle.wn_weld_write_device(weld.V.data_ptr(), nf, nv, n0, n1,
+                                       weld.scratch.data_ptr(), edges.data_ptr(), _stream()))
+
+    def run(n, first, with_dq, stream):
+        _check(handle.wn_backward_edges_mixed_device(
+            edges[7 * first:].data_ptr(), n, n, q.data_ptr(), nq, gw.data_ptr(), kappa, 1,
+            dq.data_ptr() if with_dq else None, dedge[6 * first:].data_ptr(), stream))
+
+    if not n0 or not n1:
+        run(n0 + n1, 0, not n0, _stream())
+    else:
+        main = torch.cuda.current_stream(q.device)
+        side = torch.cuda.Stream(q.device)
+        side.wait_stream(main)
+        run(n1, n0, True, ctypes.c_void_p(side.cuda_stream))
+        run(n0, 0, False, _stream())
+        main.wait_stream(side)
+        for t in (edges, dedge, dq, q, gw):  # made on the main stream, used on both
+            t.record_stream(side)
+    scratch = _scratch(3, nf, weld.V)
+    _check(handle.wn_gather_welded_device(dedge.data_ptr(), n0, n1, weld.F.data_ptr(), nf, nv,
+                                          weld.scratch.data_ptr(), scratch.data_ptr(),
+                                          dV.data_ptr(), _stream()))
+    return dV, dq
+
+
 def backward_welded_edges(V, F, O, gW, welded=None, kappa: float = 4.0):
     """(dL/dV, dL/dO) of a triangle soup from its sides welded by position.
 
@@ -283,11 +401,15 @@ def backward_welded_edges(V, F, O, gW, welded=None, kappa: float = 4.0):
     dL/dO (a leaner kernel) and only the others (an open soup's boundary) through the
     full one; a closed soup (every m = 0) gets dL/dO = 0 from one lean launch.
     """
+    if welded is None:
+        welded = _weld(V, F)
+    if isinstance(welded, _Weld):
+        return _backward_weld(welded, O, gW, kappa)
     handle = _lib.lib()
     q = O.to(torch.float64).contiguous()
     gw = gW.to(torch.float64).contiguous()
     nq, nv = q.shape[0], V.shape[0]
-    edges, ng, side_edge, sigma, ends = welded if welded is not None else welded_edges(V, F)
+    edges, ng, side_edge, sigma, ends = welded
     le = edges.shape[1]
     dq = torch.zeros((nq, 3), dtype=torch.float64, device=q.device)
     dedge = torch.zeros((6, le), dtype=torch.float64, device=q.device)
@@ -380,6 +502,9 @@ class WindingNumberFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gW):
         V, F, O = ctx.saved_tensors
+        dtypes = V.dtype, O.dtype
+        # Converted here, ahead of the waits for the edges' counts.
+        V, O, gW = (x.to(torch.float64).contiguous() for x in (V, O, gW))
         adjoint = ctx.adjoint
         edges = None
         welded = None
@@ -387,7 +512,7 @@ class WindingNumberFunction(torch.autograd.Function):
             edges = boundary_edges(V, F)
             adjoint = "edges"
             if ctx.precision == "mixed" and edges[1] > FACE_COST * ctx.nf:
-                welded = welded_edges(V, F)
+                welded = _weld(V, F)
                 adjoint = "welded" if welded[1] < FACE_COST * ctx.nf else "faces"
             if adjoint != "faces" and ctx.mesh is not None:
                 ctx.mesh.close()
@@ -407,7 +532,7 @@ class WindingNumberFunction(torch.autograd.Function):
             mesh.close()
         else:
             dV, dq = backward_fp64(ctx.tri, ctx.ld, ctx.nf, O, gW, F, V.shape[0])
-        return dV.to(V.dtype), None, dq.to(O.dtype), None, None
+        return dV.to(dtypes[0]), None, dq.to(dtypes[1]), None, None
 
 
 def winding_number_torch(V: torch.Tensor, F: torch.Tensor, O: torch.Tensor,
