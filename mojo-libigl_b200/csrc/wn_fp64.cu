@@ -3,18 +3,21 @@
 // Replaces the reference's two-kernel GPU path (lee101/mojo-libigl,
 // src/capi.mojo:297-398: one thread per (face, query) writing an nf x nq FP64
 // angle buffer, then one thread per query summing it). Here one fused kernel:
-//   * each CTA owns THREADS*QPT queries, QPT per thread, held in registers;
-//   * the CTA streams the face SoA (9 rows x ld doubles) through a STAGES-deep
-//     ring of shared-memory tiles filled by 1-D bulk copies (cp.async.bulk,
-//     completion on an mbarrier; no cluster multicast);
-//   * every thread evaluates its QPT queries against each face of the tile,
-//     reading the face by shared-memory broadcast;
-//   * pair terms are bit-identical to the reference (wn_pair.cuh); the angles
-//     are summed either by the argument-of-product accumulator (default) or by
-//     one atan2 per pair;
+//   * each CTA owns 128 queries, one per thread, held in registers;
+//   * the CTA streams the face SoA (9 rows x ld doubles) through a ring of
+//     shared-memory tiles filled by 1-D bulk copies (cp.async.bulk, completion on
+//     an mbarrier; no cluster multicast);
+//   * every thread evaluates its query against each face of the tile, reading the
+//     face by shared-memory broadcast;
+//   * pair terms are bit-identical to the reference (wn_pair.cuh) wherever their
+//     last bits can matter, and rounded about as well where they cannot
+//     (pair_terms_far); the angles are summed either by the argument-of-product
+//     accumulator (default) or by one atan2 per pair, bit-identical terms only;
 //   * no nf x nq buffer exists. When there are too few queries to fill the
 //     GPU the face range is split over grid.y and a second kernel sums the
-//     per-split partial angles in split order (deterministic, no atomics).
+//     per-split partial angles in a fixed order (deterministic, no atomics);
+//   * few queries (fp64_few_kernel) leave most threads of such a CTA idle: there
+//     the threads stand for faces and the queries are common to the CTA.
 #include <algorithm>
 
 #include "wn_common.cuh"
@@ -52,27 +55,62 @@ __device__ double direct_sum_global(const Fp64Args& a, int64_t f_begin, int64_t 
   return s;
 }
 
-template <int THREADS, int QPT, int TF, int STAGES, int MODE>
-__global__ void __launch_bounds__(THREADS) fp64_forward_kernel(const Fp64Args a) {
+// Adds two faces to a query's product. Both factors far: their arguments lie within
+// (-pi/2, pi/2), so they multiply without a turn and go in as one.
+__device__ __forceinline__ void push_two(ArgAcc& acc, double ox, double oy, double oz,
+                                         const double (&u)[9], const double (&v)[9]) {
+  double t0, d0, t1, d1;
+  const bool far0 = pair_terms_far(ox, oy, oz, u[0], u[1], u[2], u[3], u[4], u[5], u[6], u[7],
+                                   u[8], t0, d0);
+  const bool far1 = pair_terms_far(ox, oy, oz, v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7],
+                                   v[8], t1, d1);
+  if (far0 && far1) {
+    argacc_push(acc, fma(d0, d1, -(t0 * t1)), fma(d0, t1, t0 * d1));
+    return;
+  }
+  if (!far0)
+    pair_terms_exact(ox, oy, oz, u[0], u[1], u[2], u[3], u[4], u[5], u[6], u[7], u[8], t0, d0);
+  argacc_push(acc, d0, t0);
+  if (!far1)
+    pair_terms_exact(ox, oy, oz, v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8], t1, d1);
+  argacc_push(acc, d1, t1);
+}
+
+__device__ __forceinline__ void push_one(ArgAcc& acc, double ox, double oy, double oz,
+                                         const double (&v)[9]) {
+  double t, d;
+  if (!pair_terms_far(ox, oy, oz, v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8], t, d))
+    pair_terms_exact(ox, oy, oz, v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8], t, d);
+  argacc_push(acc, d, t);
+}
+
+constexpr int kFwdThreads = 128, kFwdStages = 3;
+constexpr int kFwdTileBytes = 9 * kTileFaces * 8;
+
+// Bound by the FP64 pipe: about 115 operations a bit-identical pair (three correctly
+// rounded roots among them), 65 one of pair_terms_far. Two
+// faces a step: their far factors are multiplied first, which saves half of the product's
+// bookkeeping (120 -> 95 instructions a pair) and gives every warp a second chain (92
+// registers, 20 warps an SM). One query a thread and 64-face tiles keep the split fine.
+// On one B200, before (two queries a thread, bit-identical terms only) and now, us:
+// 28,322 F x 1,024 Q 235 -> 159, 20,480 F x 1,024 Q 196 -> 121, 243,602 F x 2,048 Q
+// 3,491 -> 2,448; one face a step 182, 137, 2,996. Corners shared with the face before
+// were tried instead: a third of them at best in a mesh's own order, no gain.
+template <int MODE>
+__global__ void __launch_bounds__(kFwdThreads) fp64_forward_kernel(const Fp64Args a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  double* tiles = reinterpret_cast<double*>(smem_raw);  // [STAGES][9][TF]
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + sizeof(double) * STAGES * 9 * TF);
+  constexpr int TF = kTileFaces, STAGES = kFwdStages;
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + STAGES * kFwdTileBytes);
 
   const int tid = threadIdx.x;
-  const int64_t q_base = static_cast<int64_t>(blockIdx.x) * (THREADS * QPT);
+  const int64_t qi = static_cast<int64_t>(blockIdx.x) * kFwdThreads + tid;
   const int64_t f_begin = static_cast<int64_t>(blockIdx.y) * a.f_chunk;
   const int64_t f_end = min(a.nf, f_begin + a.f_chunk);
   const int ntiles = f_end > f_begin ? static_cast<int>((f_end - f_begin + TF - 1) / TF) : 0;
-
-  double ox[QPT], oy[QPT], oz[QPT];
-#pragma unroll
-  for (int k = 0; k < QPT; ++k) {
-    const int64_t qi = q_base + tid + k * THREADS;
-    const bool valid = qi < a.nq;
-    ox[k] = valid ? a.q[3 * qi] : 0.0;
-    oy[k] = valid ? a.q[3 * qi + 1] : 0.0;
-    oz[k] = valid ? a.q[3 * qi + 2] : 0.0;
-  }
+  const bool valid = qi < a.nq;
+  const double ox = valid ? a.q[3 * qi] : 0.0;
+  const double oy = valid ? a.q[3 * qi + 1] : 0.0;
+  const double oz = valid ? a.q[3 * qi + 2] : 0.0;
 
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) mbar_init(&full[s], 1);
@@ -91,20 +129,17 @@ __global__ void __launch_bounds__(THREADS) fp64_forward_kernel(const Fp64Args a)
     mbar_arrive_expect_tx(&full[slot], 9u * bytes);
 #pragma unroll
     for (int r = 0; r < 9; ++r)
-      bulk_g2s(tiles + (slot * 9 + r) * TF, a.tri + r * a.ld + f0, bytes, &full[slot]);
+      bulk_g2s(smem_raw + slot * kFwdTileBytes + r * TF * 8, a.tri + r * a.ld + f0, bytes,
+               &full[slot]);
   };
   int issued = 0;
   if (tid == 0) {
     for (; issued < min(STAGES, ntiles); ++issued) issue(issued);
   }
 
-  ArgAcc acc[QPT];
-  double sum[QPT];
-#pragma unroll
-  for (int k = 0; k < QPT; ++k) {
-    argacc_init(acc[k]);
-    sum[k] = 0.0;
-  }
+  ArgAcc acc;
+  argacc_init(acc);
+  double sum = 0.0;
 
   bool failed = false;
   int t = 0;
@@ -118,22 +153,34 @@ __global__ void __launch_bounds__(THREADS) fp64_forward_kernel(const Fp64Args a)
     }
     if (tid == 0 && t >= 1 && issued < ntiles) issue(issued++);
 
-    const double* s = tiles + slot * 9 * TF;
+    const double* s = reinterpret_cast<const double*>(smem_raw + slot * kFwdTileBytes);
     const int64_t f0 = f_begin + static_cast<int64_t>(t) * TF;
     const int n = static_cast<int>(min(static_cast<int64_t>(TF), f_end - f0));
-#pragma unroll 1
-    for (int j = 0; j < n; ++j) {
-      const double Ax = s[j], Ay = s[TF + j], Az = s[2 * TF + j];
-      const double Bx = s[3 * TF + j], By = s[4 * TF + j], Bz = s[5 * TF + j];
-      const double Cx = s[6 * TF + j], Cy = s[7 * TF + j], Cz = s[8 * TF + j];
+    auto face = [&](int j, double(&v)[9]) {
 #pragma unroll
-      for (int k = 0; k < QPT; ++k) {
+      for (int r = 0; r < 9; ++r) v[r] = s[r * TF + j];
+    };
+    double u[9], v[9];
+    if (MODE == kFp64ArgProd) {
+      int j = 0;
+#pragma unroll 1
+      for (; j + 1 < n; j += 2) {
+        face(j, u);
+        face(j + 1, v);
+        push_two(acc, ox, oy, oz, u, v);
+      }
+      if (j < n) {
+        face(j, u);
+        push_one(acc, ox, oy, oz, u);
+      }
+    } else {
+#pragma unroll 1
+      for (int j = 0; j < n; ++j) {
+        face(j, u);
         double det, denom;
-        pair_terms_exact(ox[k], oy[k], oz[k], Ax, Ay, Az, Bx, By, Bz, Cx, Cy, Cz, det, denom);
-        if (MODE == kFp64ArgProd)
-          argacc_push(acc[k], denom, det);
-        else
-          sum[k] += atan2(det, denom);
+        pair_terms_exact(ox, oy, oz, u[0], u[1], u[2], u[3], u[4], u[5], u[6], u[7], u[8], det,
+                         denom);
+        sum += atan2(det, denom);
       }
     }
   }
@@ -146,31 +193,142 @@ __global__ void __launch_bounds__(THREADS) fp64_forward_kernel(const Fp64Args a)
     return;
   }
 
-#pragma unroll
-  for (int k = 0; k < QPT; ++k) {
-    const int64_t qi = q_base + tid + k * THREADS;
-    if (qi >= a.nq) continue;
-    double angle;
-    if (MODE == kFp64ArgProd) {
-      angle = acc[k].bad ? direct_sum_global(a, f_begin, f_end, ox[k], oy[k], oz[k])
-                         : atan2(acc[k].zi, acc[k].zr) + static_cast<double>(acc[k].k) * kTwoPi;
-    } else {
-      angle = sum[k];
-    }
-    if (gridDim.y == 1)
-      a.w[qi] = angle / kTwoPi;
-    else
-      a.partial[static_cast<int64_t>(blockIdx.y) * a.nq + qi] = angle;
-  }
+  if (!valid) return;
+  double angle = sum;
+  if (MODE == kFp64ArgProd)
+    angle = acc.bad ? direct_sum_global(a, f_begin, f_end, ox, oy, oz)
+                    : atan2(acc.zi, acc.zr) + static_cast<double>(acc.k) * kTwoPi;
+  if (gridDim.y == 1)
+    a.w[qi] = angle / kTwoPi;
+  else
+    a.partial[static_cast<int64_t>(blockIdx.y) * a.nq + qi] = angle;
 }
 
-__global__ void sum_splits_kernel(const double* __restrict__ partial, int64_t nsplit, int64_t nq,
-                                  double* __restrict__ w) {
-  const int64_t qi = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (qi >= nq) return;
+// Few queries: kFewQueries of them a CTA, common to its threads, which take faces
+// f_begin + tid, + kFewThreads, ... The threads' products are multiplied pairwise in a
+// fixed order (their turns add; a product that went bad makes the CTA sum one atan2 per
+// pair). Bound by latency at the few: 1,178 F x 1 Q 78 -> 24 us on one B200 (with the sum
+// of the splits), 28,322 F x 64 Q 105 -> 27, 243,602 F x 64 Q 532 -> 102.
+constexpr int kFewThreads = 128, kFewQueries = 4;
+
+__device__ void argacc_join(ArgAcc& s, double zr, double zi, int k, int bad) {
+  argacc_push(s, zr, zi);
+  s.k += k;
+  s.bad |= bad;
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kFewThreads) fp64_few_kernel(const Fp64Args a) {
+  __shared__ double part[kFewThreads / 32][kFewQueries][2];
+  __shared__ int turns[kFewThreads / 32][kFewQueries];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t q0 = static_cast<int64_t>(blockIdx.x) * kFewQueries;
+  const int64_t f_begin = static_cast<int64_t>(blockIdx.y) * a.f_chunk;
+  const int64_t f_end = min(a.nf, f_begin + a.f_chunk);
+  const int nq = static_cast<int>(min(static_cast<int64_t>(kFewQueries), a.nq - q0));
+  double o[kFewQueries][3];
+  ArgAcc acc[kFewQueries];
+  double sum[kFewQueries];
+#pragma unroll
+  for (int k = 0; k < kFewQueries; ++k) {
+    for (int x = 0; x < 3; ++x) o[k][x] = k < nq ? a.q[3 * (q0 + k) + x] : 0.0;
+    argacc_init(acc[k]);
+    sum[k] = 0.0;
+  }
+  auto walk = [&](bool product) {
+    for (int64_t f = f_begin + tid; f < f_end; f += kFewThreads) {
+      double v[9];
+#pragma unroll
+      for (int r = 0; r < 9; ++r) v[r] = a.tri[r * a.ld + f];
+#pragma unroll
+      for (int k = 0; k < kFewQueries; ++k) {
+        if (k >= nq) break;
+        if (product) {
+          push_one(acc[k], o[k][0], o[k][1], o[k][2], v);
+        } else {
+          double det, denom;
+          pair_terms_exact(o[k][0], o[k][1], o[k][2], v[0], v[1], v[2], v[3], v[4], v[5], v[6],
+                           v[7], v[8], det, denom);
+          sum[k] += atan2(det, denom);
+        }
+      }
+    }
+  };
+  bool product = MODE == kFp64ArgProd;
+  walk(product);
+  if (product) {
+    int bad = 0;
+#pragma unroll
+    for (int k = 0; k < kFewQueries; ++k) {
+      if (k >= nq) break;
+      for (int off = 16; off; off >>= 1)
+        argacc_join(acc[k], __shfl_down_sync(0xffffffffu, acc[k].zr, off),
+                    __shfl_down_sync(0xffffffffu, acc[k].zi, off),
+                    __shfl_down_sync(0xffffffffu, acc[k].k, off),
+                    __shfl_down_sync(0xffffffffu, acc[k].bad, off));
+      bad |= acc[k].bad;
+      if (lane == 0) {
+        part[warp][k][0] = acc[k].zr;
+        part[warp][k][1] = acc[k].zi;
+        turns[warp][k] = acc[k].k;
+      }
+    }
+    if (__syncthreads_or(bad)) {
+      product = false;
+      walk(false);
+      __syncthreads();  // part is read by no one: it is written again below
+    }
+  }
+  if (!product) {
+#pragma unroll
+    for (int k = 0; k < kFewQueries; ++k) {
+      for (int off = 16; off; off >>= 1) sum[k] += __shfl_down_sync(0xffffffffu, sum[k], off);
+      if (lane == 0) part[warp][k][0] = sum[k];
+    }
+    __syncthreads();
+  }
+  if (tid >= nq) return;
+  double angle = 0.0;
+  bool done = false;
+  if (product) {
+    ArgAcc s;
+    argacc_init(s);
+    for (int w = 0; w < kFewThreads / 32; ++w)
+      argacc_join(s, part[w][tid][0], part[w][tid][1], turns[w][tid], 0);
+    angle = atan2(s.zi, s.zr) + static_cast<double>(s.k) * kTwoPi;
+    done = true;
+  }
+  if (!done)
+    for (int w = 0; w < kFewThreads / 32; ++w) angle += part[w][tid][0];
+  if (gridDim.y == 1)
+    a.w[q0 + tid] = angle / kTwoPi;
+  else
+    a.partial[static_cast<int64_t>(blockIdx.y) * a.nq + q0 + tid] = angle;
+}
+
+// 32 queries x 8 slices of the splits a CTA: one thread for all of a query's splits is a
+// chain of their loads.
+__global__ void __launch_bounds__(256) sum_splits_kernel(const double* __restrict__ partial,
+                                                         int64_t nsplit, int64_t nq,
+                                                         double* __restrict__ w) {
+  __shared__ double slice[8][32];
+  const int64_t qi = static_cast<int64_t>(blockIdx.x) * 32 + threadIdx.x;
   double s = 0.0;
-  for (int64_t y = 0; y < nsplit; ++y) s += partial[y * nq + qi];
+  if (qi < nq)
+    for (int64_t y = threadIdx.y; y < nsplit; y += 8) s += partial[y * nq + qi];
+  slice[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.y != 0 || qi >= nq) return;
+  for (int k = 1; k < 8; ++k) s += slice[k][threadIdx.x];
   w[qi] = s / kTwoPi;
+}
+
+cudaError_t launch_sum_splits(const double* partial, int64_t nsplit, int64_t nq, double* w,
+                              cudaStream_t stream) {
+  sum_splits_kernel<<<static_cast<unsigned>((nq + 31) / 32), dim3(32, 8), 0, stream>>>(
+      partial, nsplit, nq, w);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return cudaGetLastError();
 }
 
 // ---- FP64 over a prepared mesh, with corner reuse ---------------------------
@@ -372,36 +530,54 @@ __global__ void __launch_bounds__(THREADS) fp64_tiled_kernel(const Fp64TiledArgs
   }
 }
 
-template <int THREADS, int QPT, int TF, int STAGES, int MODE>
+template <int MODE>
 cudaError_t launch_variant(const Fp64Plan& p, const Fp64Args& a, cudaStream_t stream) {
-  auto kernel = fp64_forward_kernel<THREADS, QPT, TF, STAGES, MODE>;
-  const size_t smem = sizeof(double) * STAGES * 9 * TF + sizeof(uint64_t) * STAGES;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(smem));
-  if (e != cudaSuccess) return e;
-  dim3 grid(static_cast<unsigned>(p.qblocks), static_cast<unsigned>(p.nsplit));
-  kernel<<<grid, THREADS, smem, stream>>>(a);
+  const dim3 grid(static_cast<unsigned>(p.qblocks), static_cast<unsigned>(p.nsplit));
+  if (p.few) {
+    fp64_few_kernel<MODE><<<grid, kFewThreads, 0, stream>>>(a);
+  } else {
+    const int smem = kFwdStages * (kFwdTileBytes + static_cast<int>(sizeof(uint64_t)));
+    fp64_forward_kernel<MODE><<<grid, kFwdThreads, smem, stream>>>(a);
+  }
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return cudaGetLastError();
 }
 
 }  // namespace
 
+// The shape that leaves the busiest SM the least to do. A CTA costs its tiles and half of
+// one for its start; fewer than kFwdLeast CTAs an SM do not fill the FP64 pipe, and more
+// than some waves of them need no better split.
 Fp64Plan plan_fp64(int64_t nf, int64_t nq, int sms, int force_nsplit) {
+  constexpr int64_t kFwdLeast = 8, kFwdMost = 16;
   Fp64Plan p;
-  const int64_t per_block = static_cast<int64_t>(p.threads) * p.qpt;
-  p.qblocks = std::max<int64_t>(1, (nq + per_block - 1) / per_block);
-  const int64_t tiles = std::max<int64_t>(1, (nf + p.tile_faces - 1) / p.tile_faces);
-  // Aim for >= 4 resident-CTA waves' worth of CTAs across the SMs.
-  const int64_t target = static_cast<int64_t>(std::max(sms, 1)) * 8;
-  int64_t nsplit = 1;
-  if (force_nsplit > 0)
-    nsplit = force_nsplit;
-  else if (p.qblocks < target)
-    nsplit = (target + p.qblocks - 1) / p.qblocks;
-  nsplit = std::max<int64_t>(1, std::min(nsplit, tiles));
-  const int64_t tiles_per_split = (tiles + nsplit - 1) / nsplit;
-  p.f_chunk = tiles_per_split * p.tile_faces;
+  auto round_up = [](int64_t n, int64_t m) { return (std::max<int64_t>(n, 1) + m - 1) / m * m; };
+  // A few-query CTA pads the queries to 4, the other to 128, but spends up to 1.5 times as
+  // long on a pair (28,322 F, us: 80 Q 30 against 42 padded, 150 Q 42 against 52; 96 Q
+  // would tie, 200 Q 56 against 52).
+  p.few = 3 * round_up(nq, kFewQueries) <= 2 * round_up(nq, kFwdThreads);
+  p.tile_faces = p.few ? kFewThreads : kTileFaces;
+  p.qblocks = round_up(nq, p.few ? kFewQueries : kFwdThreads) / (p.few ? kFewQueries : kFwdThreads);
+  const int64_t tiles = round_up(nf, p.tile_faces) / p.tile_faces;
+  sms = std::max(sms, 1);
+  int64_t per = tiles;  // tiles of a CTA
+  if (force_nsplit > 0) {
+    per = (tiles + force_nsplit - 1) / force_nsplit;
+  } else if (p.qblocks < kFwdMost * sms) {
+    double best = 0.0;
+    const int64_t most = (kFwdMost * sms + p.qblocks - 1) / p.qblocks;
+    for (int64_t n = 1; n <= std::min(most, tiles); n += 1 + n / 16) {
+      const int64_t t = (tiles + n - 1) / n;
+      const int64_t ctas = p.qblocks * ((tiles + t - 1) / t);
+      const double cost = static_cast<double>(std::max<int64_t>((ctas + sms - 1) / sms, kFwdLeast)) *
+                          (static_cast<double>(t) + 0.5);
+      if (best == 0.0 || cost < best) {
+        best = cost;
+        per = t;
+      }
+    }
+  }
+  p.f_chunk = per * p.tile_faces;
   p.nsplit = std::max<int64_t>(1, (nf + p.f_chunk - 1) / p.f_chunk);
   p.scratch_doubles = p.nsplit > 1 ? p.nsplit * nq : 0;
   return p;
@@ -441,10 +617,7 @@ cudaError_t launch_fp64_tiled(const Fp64TiledPlan& p, const MixedMesh& m, const 
            smem, stream>>>(a);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   if ((e = cudaGetLastError()) != cudaSuccess || p.nsplit == 1) return e;
-  sum_splits_kernel<<<static_cast<unsigned>((nq + 255) / 256), 256, 0, stream>>>(scratch,
-                                                                             p.nsplit, nq, w);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return cudaGetLastError();
+  return launch_sum_splits(scratch, p.nsplit, nq, w, stream);
 }
 
 cudaError_t launch_fp64(const Fp64Plan& p, int mode, const double* tri, int64_t ld, int64_t nf,
@@ -457,19 +630,13 @@ cudaError_t launch_fp64(const Fp64Plan& p, int mode, const double* tri, int64_t 
     return cudaErrorInvalidValue;
   Fp64Args a{tri, ld, nf, q, nq, p.f_chunk, w, scratch, err};
   cudaError_t e;
-  if (p.threads != 128 || p.qpt != 2 || p.tile_faces != 128 || p.stages != 3)
-    return cudaErrorInvalidConfiguration;
+  if (p.tile_faces != (p.few ? kFewThreads : kTileFaces)) return cudaErrorInvalidConfiguration;
   if (mode == kFp64Direct)
-    e = launch_variant<128, 2, 128, 3, kFp64Direct>(p, a, stream);
+    e = launch_variant<kFp64Direct>(p, a, stream);
   else
-    e = launch_variant<128, 2, 128, 3, kFp64ArgProd>(p, a, stream);
+    e = launch_variant<kFp64ArgProd>(p, a, stream);
   if (e != cudaSuccess || p.nsplit == 1) return e;
-  const int threads = 256;
-  const int64_t blocks = (nq + threads - 1) / threads;
-  sum_splits_kernel<<<static_cast<unsigned>(blocks), threads, 0, stream>>>(scratch, p.nsplit, nq,
-                                                                          w);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return cudaGetLastError();
+  return launch_sum_splits(scratch, p.nsplit, nq, w, stream);
 }
 
 }  // namespace wn

@@ -60,10 +60,8 @@ enum Fp64Mode : int {
 };
 
 struct Fp64Plan {
-  int threads = 128;      // threads per CTA
-  int qpt = 2;            // queries held per thread
-  int tile_faces = 128;   // faces per shared-memory tile
-  int stages = 3;         // bulk-copy ring depth
+  bool few = false;       // threads stand for faces, not queries
+  int tile_faces = 64;    // faces per shared-memory tile, or per step of a few-query CTA
   int64_t nsplit = 1;     // face-range splits (grid.y)
   int64_t f_chunk = 0;    // faces per split (multiple of tile_faces)
   int64_t qblocks = 0;    // grid.x
