@@ -87,31 +87,4 @@ __device__ __forceinline__ double rsqrt64(double x) {
   return fma(y * e, fma(e, 0.375, 0.5), y);
 }
 
-// det and denom of a pair (wn_pair.cuh) with contracted products and rsqrt64's roots: 65
-// FP64 operations instead of 115. True if denom is certain to be positive by a margin
-// (above |a||b||c| / 4, and between 2^-300 and 2^300): then no branch of the angle is
-// near, its error stays within a few roundings, and neither term's last bits decide
-// anything. Else, and for anything not finite, the caller takes the bit-identical terms.
-__device__ __forceinline__ bool pair_terms_far(double ox, double oy, double oz, double Ax,
-                                               double Ay, double Az, double Bx, double By,
-                                               double Bz, double Cx, double Cy, double Cz,
-                                               double& det, double& denom) {
-  const double ax = Ax - ox, ay = Ay - oy, az = Az - oz;
-  const double bx = Bx - ox, by = By - oy, bz = Bz - oz;
-  const double cx = Cx - ox, cy = Cy - oy, cz = Cz - oz;
-  const double aa = fma(ax, ax, fma(ay, ay, az * az));
-  const double bb = fma(bx, bx, fma(by, by, bz * bz));
-  const double cc = fma(cx, cx, fma(cy, cy, cz * cz));
-  const double la = aa * rsqrt64(aa), lb = bb * rsqrt64(bb), lc = cc * rsqrt64(cc);
-  const double nx = fma(by, cz, -(bz * cy)), ny = fma(bz, cx, -(bx * cz)),
-               nz = fma(bx, cy, -(by * cx));
-  det = fma(ax, nx, fma(ay, ny, az * nz));
-  const double lll = la * lb * lc;
-  double d = fma(fma(ax, bx, fma(ay, by, az * bz)), lc, lll);
-  d = fma(fma(bx, cx, fma(by, cy, bz * cz)), la, d);
-  denom = fma(fma(cx, ax, fma(cy, ay, cz * az)), lb, d);
-  const int hd = __double2hiint(denom);  // high words order positive numbers
-  return hd > 0x2d300000 && hd < 0x52b00000 && hd > __double2hiint(lll) - 0x00200000;
-}
-
 }  // namespace wn

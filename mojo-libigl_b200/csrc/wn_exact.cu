@@ -49,6 +49,7 @@
 #include "wn_exact.h"
 #include "wn_internal.h"
 #include "wn_pair.cuh"
+#include "wn_pair_device.cuh"
 
 namespace wn {
 namespace {
@@ -1253,10 +1254,8 @@ __global__ void __launch_bounds__(32 * kWarps, 4) exact_eval_kernel(const EvalAr
               const double2* s = reinterpret_cast<const double2*>(f + k);
               const double2 s0 = __ldg(s), s1 = __ldg(s + 1), s2 = __ldg(s + 2), s3 = __ldg(s + 3);
               const double s4 = __ldg(&f[k].v[8]);
-              double det, denom;
-              pair_terms_exact(qx, qy, qz, s0.x, s0.y, s1.x, s1.y, s2.x, s2.y, s3.x, s3.y, s4,
-                               det, denom);
-              argacc_push(acc, denom, det);
+              const double v[9] = {s0.x, s0.y, s1.x, s1.y, s2.x, s2.y, s3.x, s3.y, s4};
+              push_one(acc, qx, qy, qz, v);
             }
           }
           // The sides towards leaves that are not near, reversed.

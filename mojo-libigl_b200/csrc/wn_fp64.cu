@@ -24,6 +24,7 @@
 #include "wn_internal.h"
 #include "wn_mixed.h"
 #include "wn_pair.cuh"
+#include "wn_pair_device.cuh"
 
 namespace wn {
 namespace {
@@ -53,35 +54,6 @@ __device__ double direct_sum_global(const Fp64Args& a, int64_t f_begin, int64_t 
     s += atan2(det, denom);
   }
   return s;
-}
-
-// Adds two faces to a query's product. Both factors far: their arguments lie within
-// (-pi/2, pi/2), so they multiply without a turn and go in as one.
-__device__ __forceinline__ void push_two(ArgAcc& acc, double ox, double oy, double oz,
-                                         const double (&u)[9], const double (&v)[9]) {
-  double t0, d0, t1, d1;
-  const bool far0 = pair_terms_far(ox, oy, oz, u[0], u[1], u[2], u[3], u[4], u[5], u[6], u[7],
-                                   u[8], t0, d0);
-  const bool far1 = pair_terms_far(ox, oy, oz, v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7],
-                                   v[8], t1, d1);
-  if (far0 && far1) {
-    argacc_push(acc, fma(d0, d1, -(t0 * t1)), fma(d0, t1, t0 * d1));
-    return;
-  }
-  if (!far0)
-    pair_terms_exact(ox, oy, oz, u[0], u[1], u[2], u[3], u[4], u[5], u[6], u[7], u[8], t0, d0);
-  argacc_push(acc, d0, t0);
-  if (!far1)
-    pair_terms_exact(ox, oy, oz, v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8], t1, d1);
-  argacc_push(acc, d1, t1);
-}
-
-__device__ __forceinline__ void push_one(ArgAcc& acc, double ox, double oy, double oz,
-                                         const double (&v)[9]) {
-  double t, d;
-  if (!pair_terms_far(ox, oy, oz, v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8], t, d))
-    pair_terms_exact(ox, oy, oz, v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8], t, d);
-  argacc_push(acc, d, t);
 }
 
 constexpr int kFwdThreads = 128, kFwdStages = 3;
