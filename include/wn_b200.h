@@ -92,6 +92,15 @@ int wn_version(void);                 /* 100 * major + minor */
 const char* wn_last_error(void);      /* message of this thread's last failure */
 int wn_device_count(void);            /* CUDA devices visible (0 if none) */
 int wn_device_memory(int64_t* free_bytes, int64_t* total_bytes); /* current device */
+
+/* Host arrays, checked and packed on the host's own threads (no device involved).
+ * finite / in_range / same: 1 if every value is finite / lies in [0, limit) / the bytes
+ * are equal, else 0. soup: the (9, nf) triangle soup of V (nv,3) and F (nf,3);
+ * WN_EINVAL if an index lies outside [0, nv) (tri is then unspecified). */
+int wn_host_finite(const double* x, int64_t n);
+int wn_host_in_range(const int64_t* x, int64_t n, int64_t limit);
+int wn_host_same(const void* a, const void* b, int64_t bytes);
+int wn_host_soup(const double* V, int64_t nv, const int64_t* F, int64_t nf, double* tri);
 /* Synchronise `stream` and report (then clear) device-side errors raised by
  * device entry points launched on it since the last check. */
 int wn_stream_check(void* stream);

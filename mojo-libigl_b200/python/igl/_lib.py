@@ -74,6 +74,10 @@ _WN_SIGNATURES = {
     "wn_mixed_stats": ([ctypes.POINTER(I), ctypes.POINTER(I), C_INT], C_INT),
     "wn_backward_fp64_device": ([P, I, I, P, I, P, P, P, P], C_INT),
     "wn_gather_vertex_grad_device": ([P, I, C_INT, P, P, I, P, P], C_INT),
+    "wn_host_finite": ([P, I], C_INT),
+    "wn_host_in_range": ([P, I, I], C_INT),
+    "wn_host_same": ([P, P, I], C_INT),
+    "wn_host_soup": ([P, I, P, I, P], C_INT),
     "wn_edges_scratch_bytes": ([C_INT, I, I], I),
     "wn_boundary_count_device": ([P, I, I, P, ctypes.POINTER(I), P], C_INT),
     "wn_boundary_write_device": ([P, I, I, P, P, I, P, P], C_INT),
