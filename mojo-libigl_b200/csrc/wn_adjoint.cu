@@ -1090,11 +1090,21 @@ __device__ __noinline__ void refine_edge_grad(const double* __restrict__ e64, in
   const double qx = v[3] - o.x, qy = v[4] - o.y, qz = v[5] - o.z;
   const double pp = px * px + py * py + pz * pz;
   const double qq = qx * qx + qy * qy + qz * qz;
-  const double rp = rsqrt(pp), rq = rsqrt(qq);
-  const double rpq = rp * rq;
-  const double d = 1.0 + (px * qx + py * qy + pz * qz) * rpq;
+  const double pq = px * qx + py * qy + pz * qz;
+  double rp = rsqrt64(pp), rq = rsqrt64(qq);
+  double rpq = rp * rq;
+  double d = 1.0 + pq * rpq, rd = rcp64(d);
+  // All but on the edge d keeps few digits and its last ones matter: the library there
+  // (everywhere before: 4,572 edges x 262,144 near-surface queries 4.72 ms, 4.28 so).
+  if (!(d > 1e-2)) {
+    rp = rsqrt(pp);
+    rq = rsqrt(qq);
+    rpq = rp * rq;
+    d = 1.0 + pq * rpq;
+    rd = 1.0 / d;
+  }
   const bool ok = (unit || v[6] != 0.0) && pp > 0.0 && qq > 0.0 && d > 0.0;
-  const double w = ok ? o.w * (unit ? 1.0 : v[6]) * rpq / d : 0.0;
+  const double w = ok ? o.w * (unit ? 1.0 : v[6]) * rpq * rd : 0.0;
   const double cp = ok ? rp * w : 0.0, cq = ok ? rq * w : 0.0;
   const double x0 = py * qz - pz * qy, x1 = pz * qx - px * qz, x2 = px * qy - py * qx;
   acc_col[0] -= cp * x0;
@@ -1131,6 +1141,7 @@ struct EdgeAdjSmem {
   double4 q64[QC];
   float4 frame[QC][kFaTiles][2];  // (-x, -x, -y, -y), (-z, -z, gs, gs) as FP32x2 operands
   int flag[QC][kFaTiles];
+  uint8_t near[kFaTiles][64];  // a query's near edges of each warp's tile
   TileHeader th[kFaTiles];
 };
 
@@ -1434,12 +1445,21 @@ __device__ __forceinline__ void edge_adjoint_cta(const EdgeWork& a,
            pending &= pending - 1u) {
         const int jq = __ffs(pending) - 1;
         double go[3] = {0.0, 0.0, 0.0};
-        if ((near0 >> jq) & 1u)
-          refine_edge_grad(a.e64, a.ld64, slot0, sm.q64[jq], &sm.acc64[0][tid], kFaThreads, go,
-                           UNIT);
-        if ((near1 >> jq) & 1u)
-          refine_edge_grad(a.e64, a.ld64, slot0 + 32, sm.q64[jq], &sm.acc64[6][tid], kFaThreads,
-                           go, UNIT);
+        // The query's near edges side by side over the lanes: a tile's 64 seldom need
+        // more than one pass (4,572 edges x 262,144 near-surface queries 4.28 -> 4.08 ms).
+        const bool n0 = (near0 >> jq) & 1u, n1 = (near1 >> jq) & 1u;
+        const unsigned b0 = __ballot_sync(0xffffffffu, n0), b1 = __ballot_sync(0xffffffffu, n1);
+        const unsigned below = (1u << lane) - 1u;
+        const int c0n = __popc(b0), total = c0n + __popc(b1);
+        if (n0) sm.near[warp][__popc(b0 & below)] = static_cast<uint8_t>(lane);
+        if (n1) sm.near[warp][c0n + __popc(b1 & below)] = static_cast<uint8_t>(lane + 32);
+        __syncwarp();
+        for (int k = lane; k < total; k += 32) {
+          const int e = sm.near[warp][k];
+          refine_edge_grad(a.e64, a.ld64, slot0 - lane + e, sm.q64[jq],
+                           &sm.acc64[6 * (e >> 5)][tid - lane + (e & 31)], kFaThreads, go, UNIT);
+        }
+        __syncwarp();
         for (int off = 16; off; off >>= 1) {
           go[0] += __shfl_xor_sync(0xffffffffu, go[0], off);
           go[1] += __shfl_xor_sync(0xffffffffu, go[1], off);

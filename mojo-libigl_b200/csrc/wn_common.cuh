@@ -87,4 +87,12 @@ __device__ __forceinline__ double rsqrt64(double x) {
   return fma(y * e, fma(e, 0.375, 0.5), y);
 }
 
+// 1 / x likewise: with e = 1 - x y, y (1 + e + e^2) leaves e^3.
+__device__ __forceinline__ double rcp64(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
 }  // namespace wn
