@@ -261,6 +261,12 @@ int wn_backward_mixed_device(void* mesh, const double* q, int64_t nq, const doub
 int wn_backward_edges_device(const double* edges, int64_t le, int64_t ne, const double* q,
                              int64_t nq, const double* gw, double* dq, double* dedge,
                              void* stream);
+/* The same for edges that do not cancel one another (the boundary of an open mesh): pair
+ * terms within rounding, by cheaper square roots and reciprocals. The call above keeps the
+ * CUDA library's: where sides meet their reverses, dL/do is nothing but their rounding. */
+int wn_backward_edges_open_device(const double* edges, int64_t le, int64_t ne, const double* q,
+                             int64_t nq, const double* gw, double* dq, double* dedge,
+                             void* stream);
 /* The boundary-edge adjoint in mixed precision: the same arguments and outputs,
  * plus kappa (>= 3). Edges are Morton-ordered into 64-edge tiles inside the call;
  * pairs with both endpoints at least kappa * |edge| from the query run in FP32 in

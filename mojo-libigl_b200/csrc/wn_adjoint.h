@@ -35,11 +35,11 @@ cudaError_t adjoint_mixed(const AdjointPlan& p, const MixedMesh& m, const double
 
 // Boundary-edge adjoint (indexed meshes): edges 7 x le (P, Q, net multiplicity m), outputs
 // dq (nq x 3) and dedge (6 x le: dL/dP, dL/dQ).
-AdjointPlan plan_adjoint_edges(int64_t ne, int64_t nq, int sms);
+AdjointPlan plan_adjoint_edges(int64_t ne, int64_t nq, int sms, bool soup);
 size_t adjoint_edges_scratch_bytes(const AdjointPlan& p, int64_t le, int64_t nq);
 cudaError_t adjoint_edges(const AdjointPlan& p, const double* edges, int64_t le, int64_t ne,
                           const double* q, int64_t nq, const double* gw, double* dq,
-                          double* dedge, void* scratch, size_t scratch_bytes,
+                          double* dedge, bool soup, void* scratch, size_t scratch_bytes,
                           cudaStream_t stream);
 
 // Mixed-precision boundary-edge adjoint: the same inputs and outputs as

@@ -303,6 +303,26 @@ int forward_fp64_host(const double* tri, const double* q, double* w, int64_t nf,
   return collect_device_error(c, c->stream);
 }
 
+int backward_edges(const double* edges, int64_t le, int64_t ne, const double* q, int64_t nq,
+                   const double* gw, double* dq, double* dedge, bool soup, void* stream) {
+  if (ne < 0 || nq < 0 || le < ne)
+    return fail(WN_EINVAL, "bad sizes (ne=%lld, nq=%lld, le=%lld)", (long long)ne,
+                (long long)nq, (long long)le);
+  std::lock_guard<std::mutex> lock(g_mutex);
+  int code = WN_OK;
+  DeviceCtx* c = context(&code);
+  if (!c) return code;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const AdjointPlan p = plan_adjoint_edges(ne, nq, c->sms, soup);
+  const size_t sb = adjoint_edges_scratch_bytes(p, le, nq);
+  void* scratch = nullptr;
+  cudaError_t e = dev_malloc_async(&scratch, sb, st);
+  if (e != cudaSuccess) return cuda_fail(e, "device allocation");
+  e = adjoint_edges(p, edges, le, ne, q, nq, gw, dq, dedge, soup, scratch, sb, st);
+  cudaFreeAsync(scratch, st);
+  return e == cudaSuccess ? WN_OK : cuda_fail(e, "boundary-edge adjoint launch");
+}
+
 constexpr double kMinKappa = 3.0;  // the 64-face tile angle bound needs kappa >= 3
 
 struct MeshHandle {
@@ -793,22 +813,14 @@ int wn_backward_edges_device(const double* edges, int64_t le, int64_t ne, const 
                              int64_t nq, const double* gw, double* dq, double* dedge,
                              void* stream) {
   WN_NVTX_RANGE();
-  if (ne < 0 || nq < 0 || le < ne)
-    return fail(WN_EINVAL, "bad sizes (ne=%lld, nq=%lld, le=%lld)", (long long)ne,
-                (long long)nq, (long long)le);
-  std::lock_guard<std::mutex> lock(g_mutex);
-  int code = WN_OK;
-  DeviceCtx* c = context(&code);
-  if (!c) return code;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const AdjointPlan p = plan_adjoint_edges(ne, nq, c->sms);
-  const size_t sb = adjoint_edges_scratch_bytes(p, le, nq);
-  void* scratch = nullptr;
-  cudaError_t e = dev_malloc_async(&scratch, sb, st);
-  if (e != cudaSuccess) return cuda_fail(e, "device allocation");
-  e = adjoint_edges(p, edges, le, ne, q, nq, gw, dq, dedge, scratch, sb, st);
-  cudaFreeAsync(scratch, st);
-  return e == cudaSuccess ? WN_OK : cuda_fail(e, "boundary-edge adjoint launch");
+  return backward_edges(edges, le, ne, q, nq, gw, dq, dedge, true, stream);
+}
+
+int wn_backward_edges_open_device(const double* edges, int64_t le, int64_t ne, const double* q,
+                                  int64_t nq, const double* gw, double* dq, double* dedge,
+                                  void* stream) {
+  WN_NVTX_RANGE();
+  return backward_edges(edges, le, ne, q, nq, gw, dq, dedge, false, stream);
 }
 
 int wn_backward_edges_mixed_device(const double* edges, int64_t le, int64_t ne, const double* q,

@@ -86,6 +86,7 @@ _WN_SIGNATURES = {
     "wn_gather_edges_device": ([P, I, P, I, I, P, P, P], C_INT),
     "wn_gather_welded_device": ([P, I, I, P, I, I, P, P, P, P], C_INT),
     "wn_backward_edges_device": ([P, I, I, P, I, P, P, P, P], C_INT),
+    "wn_backward_edges_open_device": ([P, I, I, P, I, P, P, P, P], C_INT),
     "wn_backward_edges_mixed_device": ([P, I, I, P, I, P, ctypes.c_double, C_INT, P, P, P],
                                        C_INT),
     "wn_batch_create": ([I, P, P, P, P, ctypes.c_double, C_INT, I, C_INT, C_INT,

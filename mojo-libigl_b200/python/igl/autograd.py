@@ -271,9 +271,11 @@ def backward_edges(V, F, O, gW, edges=None, precision: str = "fp64", kappa: floa
                                                      gw.data_ptr(), kappa, 0, dq.data_ptr(),
                                                      dedge.data_ptr(), _stream()))
     else:
-        _check(handle.wn_backward_edges_device(edges.data_ptr(), le, ne, q.data_ptr(), nq,
-                                               gw.data_ptr(), dq.data_ptr(), dedge.data_ptr(),
-                                               _stream()))
+        # More edges than faces have sides of their own: a soup's, whose terms cancel.
+        adjoint = (handle.wn_backward_edges_device if ne > FACE_COST * F.shape[0]
+                   else handle.wn_backward_edges_open_device)
+        _check(adjoint(edges.data_ptr(), le, ne, q.data_ptr(), nq, gw.data_ptr(), dq.data_ptr(),
+                       dedge.data_ptr(), _stream()))
     scratch = _scratch(2, ne, V) if getattr(found, "nv", -1) == nv else None
     if scratch is None:
         return gather_vertices(dedge, le, ne, ends, nv, corners=2), dq
