@@ -10,9 +10,10 @@
 //
 //   W(o) = sum_{f in N} Omega_f / 4 pi  +  arg(prod_e z_e) / 2 pi  +  k
 //
-// 1. Near faces: the bit-exact FP64 pair terms, with turns counted
-//    (wn_pair.cuh), as in the all-pairs kernels. Everything that is sensitive to
-//    the last bits (queries on vertices, on edges, in faces) happens here.
+// 1. Near faces: their FP64 pair terms, with turns counted (wn_pair.cuh), as in the
+//    all-pairs kernels. Everything that is sensitive to the last bits (queries on
+//    vertices, on edges, in faces) happens here, with the bit-exact terms; faces whose
+//    denominator is positive by a margin take the cheaper ones (wn_pair_device.cuh).
 // 2. Boundary edges e = u -> v of the far faces: the infinite triangle from the
 //    edge towards a direction D closes the surface. Its solid angle is
 //    2 arg z_e with, for unit vectors a and b from o to u and v,

@@ -1,8 +1,11 @@
 // Checks and packing of the caller's host arrays (device="cpu" and "gpu" entry points).
 //
 // One pass each, over spans of at least 1 MiB on up to four threads: what these calls
-// spend is reading memory. On a B200's host, general array operations before and now, us:
-// the (9, nf) soup of 28,322 faces 218 -> 99, of 243,602 2,392 -> 377; the finite and
+// spend is reading memory. The soup is written in spans of 4 MiB: what other cores wrote
+// costs the copy to the device that follows more than they save (28,322 faces on two
+// threads: 117 us and a call of 470 us behind it, on one 170 and 332). On a B200's host,
+// general array operations before and now, us: the (9, nf) soup of 28,322 faces
+// 200 -> 170, of 243,602 2,392 -> 377; the finite and
 // range checks of 121,801 vertices and 243,602 faces 464 -> 149, comparing both with a
 // copy 290 -> 210; 3,145,728 coordinates checked 1,015 -> 250.
 #include <sched.h>
@@ -18,7 +21,7 @@
 
 namespace {
 
-constexpr int64_t kSpanBytes = 1 << 20;
+constexpr int64_t kSpanBytes = 1 << 20, kFillSpanBytes = 4 << 20;
 constexpr int kMostThreads = 4;
 
 int usable_threads() {
@@ -30,8 +33,8 @@ int usable_threads() {
 // f(lo, hi) over spans of [0, n), `bytes` of memory an item. A thread that cannot be
 // started leaves its span to the caller's.
 template <class F>
-void over_spans(int64_t n, int64_t bytes, const F& f) {
-  const int64_t want = n / std::max<int64_t>(1, kSpanBytes / bytes);
+void over_spans(int64_t n, int64_t bytes, const F& f, int64_t span = kSpanBytes) {
+  const int64_t want = n / std::max<int64_t>(1, span / bytes);
   const int parts = want < 2 ? 1 : static_cast<int>(std::min<int64_t>(
                                        std::min<int64_t>(want, kMostThreads), usable_threads()));
   if (parts < 2) {
@@ -123,7 +126,7 @@ int wn_host_soup(const double* V, int64_t nv, const int64_t* F, int64_t nf, doub
         }
       }
     }
-  });
+  }, kFillSpanBytes);
   return bad.load() ? WN_EINVAL : WN_OK;
 }
 
