@@ -1496,11 +1496,12 @@ unsigned blocks(int64_t n, int threads) {
 }  // namespace
 
 // Where the method starts to pay (one B200, meshes of 1,280 to 327,680 faces, closed,
-// open and terrain grids; ms, the faster all-pairs kernel -> this one): 20,480 F x
-// 8,192 Q 1.21 -> 0.54, 81,920 F x 4,096 Q 2.4 -> 0.8, 28,322 F (grid) x 8,192 Q 1.6 ->
-// 0.58; below the line 5,120 F x 8,192 Q 0.37 -> 0.38.
+// open and terrain grids; ms, the streaming all-pairs kernel -> this one): 1,280 F x
+// 131,072 Q 0.88 -> 0.42, 20,480 F x 8,192 Q 0.86 -> 0.43, 19,456 F with holes x 8,192 Q
+// 0.85 -> 0.65, 28,322 F (grid) x 8,192 Q 1.16 -> 0.57, 77,824 F with holes x 4,096 Q
+// 1.58 -> 1.30; below the line 5,120 F x 8,192 Q 0.24 -> 0.38.
 // Fewer queries than 4,096 leave too few warps and wide boxes: 243,602 F (grid) x
-// 2,048 Q 3.5 -> 4.1.
+// 2,048 Q 2.4 -> 4.1.
 bool exact_pays(int64_t nf, int64_t nq) {
   return nf >= 1024 && nf <= (int64_t(1) << 29) && nq >= 4096 && nq <= 0x7fffffffLL &&
          static_cast<double>(nf) * static_cast<double>(nq) >= 1.5e8;
