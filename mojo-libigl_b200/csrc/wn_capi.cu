@@ -203,11 +203,7 @@ int forward_fp64_host(const double* tri, const double* q, double* w, int64_t nf,
   if (nf < 0 || nq < 0) return fail(WN_EINVAL, "negative size (nf=%lld, nq=%lld)",
                                     (long long)nf, (long long)nq);
   const bool automatic = mode == kFp64Auto;
-  if (automatic)
-    mode = nf >= 4096 && nf <= 0x7fffffffLL &&
-                   static_cast<double>(nf) * static_cast<double>(nq) >= 1e9
-               ? kFp64Tiled
-               : kFp64ArgProd;
+  if (automatic) mode = kFp64ArgProd;
   if (mode != kFp64ArgProd && mode != kFp64Direct && mode != kFp64Tiled)
     return fail(WN_EINVAL, "bad mode %d", mode);
   if (mode == kFp64Tiled && nf > 0x7fffffffLL) return fail(WN_EINVAL, "more than 2^31-1 faces");
@@ -1701,10 +1697,10 @@ int wn_signed_distance_fast_device(void* tree, void* fast, double beta, const do
   return e == cudaSuccess ? WN_OK : cuda_fail(e, "signed-distance launch");
 }
 
-// src/capi.mojo:945-947: 1 on success, 0 on failure (the shim raises). Large
-// problems go through the prepared-mesh FP64 kernel (its ~2 ms preparation is
-// repaid above ~1e9 pairs), small ones through the streaming FP64 kernel; both
-// give pair terms bit-identical to the reference.
+// src/capi.mojo:945-947: 1 on success, 0 on failure (the shim raises). Large problems
+// take the exact path without all pairs where the mesh's edges allow it, all others the
+// streaming FP64 kernel (which the prepared mesh's no longer beats: 301,466 F x 262,144 Q
+// 472 ms prepared, 385 streamed; 57,344 F x 65,536 Q 25.6 and 18.4).
 int64_t mli_winding_gpu(int64_t tri, int64_t q, int64_t dst, int64_t nf, int64_t nq) {
   WN_NVTX_RANGE();
   return forward_fp64_host(reinterpret_cast<const double*>(tri),

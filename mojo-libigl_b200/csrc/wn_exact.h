@@ -33,9 +33,10 @@ bool exact_pays(int64_t nf, int64_t nq);
 ExactPlan plan_exact(int64_t nf, int64_t nq);
 
 // The boundary's triangles and single edges that the method may take per face. Each costs
-// every query about 7e-12 s, a pair 5.5e-12 s in the FP64 all-pairs kernels and 1.2e-12 s
+// every query about 5.5e-12 s, a pair 4.9e-12 s in the FP64 streaming kernel and 1.2e-12 s
 // in the mixed one (327,680-face mesh with 8 % of its faces deleted, 0.087 per face, x
-// 262,144 queries: 47 ms against 440 and 94).
+// 262,144 queries: 38 ms against 385 and 100; 81,920 faces with 20 % deleted x 65,536: 15.5
+// against 21.0 and 11.6).
 constexpr double kExactMostFp64 = 0.55, kExactMostMixed = 0.13;
 
 // What the boundary costs a query: triangles and single edges, and the loops that the

@@ -56,7 +56,7 @@ enum Fp64Mode : int {
   kFp64Direct = 1,   // bit-exact pair terms, one atan2 per pair
   kFp64Tiled = 2,    // kFp64ArgProd over a prepared mesh, repeated corners reused
   kFp64Auto = 3,     // internal: near faces + boundary (wn_exact.cu) where that pays, else
-                     // kFp64Tiled above 1e9 pairs and kFp64ArgProd below
+                     // kFp64ArgProd
 };
 
 struct Fp64Plan {

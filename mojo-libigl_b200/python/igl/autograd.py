@@ -80,8 +80,9 @@ def forward_fp64(tri: torch.Tensor, ld: int, nf: int, O: torch.Tensor) -> torch.
 
 
 def use_prepared_fp64(nf: int, nq: int) -> bool:
-    """The drop-in's rule (mli_winding_gpu): above 1e9 pairs the prepared-mesh
-    FP64 kernel, whose ~2 ms preparation its corner reuse repays."""
+    """Whether a mesh's preparation (~2 ms) is small beside one FP64 forward. The
+    streaming kernel is the faster one at every size all the same; a prepared mesh
+    serves callers that keep it."""
     return 4096 <= nf <= 0x7FFFFFFF and float(nf) * nq >= 1e9
 
 
@@ -492,8 +493,6 @@ class WindingNumberFunction(torch.autograd.Function):
                 ctx.mesh = mesh
             else:
                 mesh.close()
-        elif use_prepared_fp64(nf, O.shape[0]):
-            w = forward_fp64_prepared(tri, ld, nf, O)
         else:
             w = forward_fp64(tri, ld, nf, O)
         ctx.save_for_backward(V, F, O)

@@ -85,8 +85,6 @@ def gpu_forward(V, F, O, precision: str = "mixed"):
     tri, ld, nf = wa.triangle_soa(V, F)
     if precision == "mixed":
         return wa.forward_mixed(tri, ld, nf, O)
-    if wa.use_prepared_fp64(nf, O.shape[0]):
-        return wa.forward_fp64_prepared(tri, ld, nf, O)
     return wa.forward_fp64(tri, ld, nf, O)
 
 
