@@ -663,7 +663,7 @@ __global__ void __launch_bounds__(THREADS, 2) adjoint_edges_kernel(const EdgeAdj
           const double qx = ev[k][3] - ox, qy = ev[k][4] - oy, qz = ev[k][5] - oz;
           const double pp = px * px + py * py + pz * pz;
           const double qq = qx * qx + qy * qy + qz * qz;
-          double rp, rq, rpq, d, rd = 0.0;
+          double rp, rq, rpq, d = 0.0, rd = 0.0;
           if constexpr (!SOUP) {
             rp = rsqrt64(pp);
             rq = rsqrt64(qq);
