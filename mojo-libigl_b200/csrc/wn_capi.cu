@@ -1140,28 +1140,30 @@ int wn_aabb_create(const double* V, int64_t nv, const int64_t* F, int64_t nf,
     AabbSpan* spans_d = nullptr;
     int32_t* big_d = nullptr;
     int32_t thin = 0;
+    // On the stream that the disc kernels run on: cudaMemcpy from pageable memory may
+    // return before the data are on the device, and only the legacy stream waits for it.
+    auto upload = [&](void* dst, const void* src, size_t bytes) {
+      return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream);
+    };
     cudaError_t e;
     if ((e = dev_malloc(&h->t.nodes, sizeof(AabbNodeRec) * nrec.size())) != cudaSuccess ||
         (e = dev_malloc(&h->t.tris, sizeof(AabbTriRec) * trec.size())) != cudaSuccess ||
-        (e = cudaMemcpy(h->t.nodes, nrec.data(), sizeof(AabbNodeRec) * nrec.size(),
-                        cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaMemcpy(h->t.tris, trec.data(), sizeof(AabbTriRec) * trec.size(),
-                        cudaMemcpyHostToDevice)) != cudaSuccess ||
+        (e = upload(h->t.nodes, nrec.data(), sizeof(AabbNodeRec) * nrec.size())) != cudaSuccess ||
+        (e = upload(h->t.tris, trec.data(), sizeof(AabbTriRec) * trec.size())) != cudaSuccess ||
         (regular &&
          ((e = dev_malloc(&h->t.walk, sizeof(AabbWalkRec) * wrec.size())) != cudaSuccess ||
-          (e = cudaMemcpy(h->t.walk, wrec.data(), sizeof(AabbWalkRec) * wrec.size(),
-                          cudaMemcpyHostToDevice)) != cudaSuccess ||
           (e = dev_malloc(&h->t.face_discs, sizeof(AabbDisc) * trec.size())) != cudaSuccess ||
           (e = dev_malloc(&spans_d, sizeof(AabbSpan) * spans.size())) != cudaSuccess ||
-          (e = cudaMemcpy(spans_d, spans.data(), sizeof(AabbSpan) * spans.size(),
-                          cudaMemcpyHostToDevice)) != cudaSuccess ||
           (e = dev_malloc(&big_d, sizeof(int32_t) * big.size())) != cudaSuccess ||
-          (e = cudaMemcpy(big_d, big.data(), sizeof(int32_t) * big.size(),
-                          cudaMemcpyHostToDevice)) != cudaSuccess ||
+          (e = upload(h->t.walk, wrec.data(), sizeof(AabbWalkRec) * wrec.size())) !=
+              cudaSuccess ||
+          (e = upload(spans_d, spans.data(), sizeof(AabbSpan) * spans.size())) != cudaSuccess ||
+          (e = upload(big_d, big.data(), sizeof(int32_t) * big.size())) != cudaSuccess ||
           (e = aabb_discs(h->t, spans_d, big_d, nbig, big_d + nbig, c->stream)) != cudaSuccess ||
           (e = cudaMemcpyAsync(&thin, big_d + nbig, sizeof(int32_t), cudaMemcpyDeviceToHost,
-                               c->stream)) != cudaSuccess ||
-          (e = cudaStreamSynchronize(c->stream)) != cudaSuccess))) {
+                               c->stream)) != cudaSuccess)) ||
+        (e = cudaStreamSynchronize(c->stream)) != cudaSuccess) {
+      cudaStreamSynchronize(c->stream);  // the host arrays' last readers
       cudaFree(spans_d);
       cudaFree(big_d);
       cudaFree(h->t.nodes);
