@@ -51,6 +51,10 @@ constexpr int kTies = 8;
 // the rest of the GPU then waits for (327,680 faces x 2^20 points, stack in local memory:
 // 32 3.17 ms, 16 2.64, 8 2.87, 4 2.95).
 constexpr int kGroup = 16;
+// Shared memory that a launch gets without asking for more: 48 levels of the any-order
+// walk's stack. The library's own trees have at most 30 (2^31 faces); a caller-made one may
+// have 63, and takes the reference's walk, whose stack is in local memory.
+constexpr size_t kStackBytes = 48 << 10;
 // A face is thin below |n|^2 = kThin * (longest side)^4: thinner than about 1 : 1000.
 constexpr double kThin = 1e-6;
 
@@ -494,9 +498,9 @@ cudaError_t aabb_query(const AabbDeviceTree& t, const double* P, int64_t np, con
   for (int k = 0; k < 6; ++k) a.root[k] = t.root[k];
   const int64_t blocks = (np + kAabbThreads - 1) / kAabbThreads;
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  if (t.any_order && t.nnodes > 0)
-    aabb_any_order_kernel<<<static_cast<unsigned>(blocks), kAabbThreads,
-                            sizeof(uint2) * kAabbThreads * t.depth, stream>>>(a);
+  const size_t stack_bytes = sizeof(uint2) * kAabbThreads * t.depth;
+  if (t.any_order && t.nnodes > 0 && stack_bytes <= kStackBytes)
+    aabb_any_order_kernel<<<static_cast<unsigned>(blocks), kAabbThreads, stack_bytes, stream>>>(a);
   else
     aabb_query_kernel<<<static_cast<unsigned>(blocks), kAabbThreads, 0, stream>>>(a);
   g_launches.fetch_add(1, std::memory_order_relaxed);
