@@ -72,8 +72,26 @@ struct AabbArgs {
   int64_t np, nnodes;
   double root[6];
   double scale;
+  AabbFrame frame;
   int levels;  // depth of the tree
 };
+
+// A point in the tree's frame, with the margin of its bounds; `ok` where they hold (not
+// for huge or non-finite points, nor where the coordinates are so large beside the mesh
+// that their own rounding outweighs it).
+struct Local {
+  float x, y, z, margin;
+  bool ok;
+};
+__device__ __forceinline__ Local local_of(const AabbArgs& a, double px, double py, double pz) {
+  const double x = (px - a.frame.c[0]) * a.frame.s, y = (py - a.frame.c[1]) * a.frame.s,
+               z = (pz - a.frame.c[2]) * a.frame.s;
+  const double size = a.frame.ext + fabs(x) + fabs(y) + fabs(z);
+  const double round = kWalkRound * (a.scale + fabs(px) + fabs(py) + fabs(pz)) * a.frame.s;
+  return Local{static_cast<float>(x), static_cast<float>(y), static_cast<float>(z),
+               kWalkMargin * __double2float_ru(size) + __double2float_ru(round),
+               size < 1e15 && round < 1e-3 * size};
+}
 
 struct Best {
   double d2, x, y, z;
@@ -113,10 +131,8 @@ __device__ __forceinline__ float disc_bound2(float px, float py, float pz, const
 // the disc bound where that is larger: such a child holds no face that the reference
 // would take. The order is decided by the box distances alone.
 __device__ __noinline__ Best ordered_walk(const AabbArgs& a, double px, double py, double pz) {
-  const double size = a.scale + fabs(px) + fabs(py) + fabs(pz);
-  const float margin = size < 1e15 ? kWalkMargin * __double2float_ru(size) : INFINITY;
-  const float fx = static_cast<float>(px), fy = static_cast<float>(py),
-              fz = static_cast<float>(pz);
+  const Local p = local_of(a, px, py, pz);
+  const double unit = a.frame.s > 0.0 ? 1.0 / a.frame.s : 0.0;
   Best r{1.0e300, 0.0, 0.0, 0.0, -1};
   int stack_node[kAabbStack];
   double stack_d2[kAabbStack];
@@ -141,13 +157,13 @@ __device__ __noinline__ Best ordered_walk(const AabbArgs& a, double px, double p
     } else {
       const double dl = box_of(nd->lbox, px, py, pz), dr = box_of(nd->rbox, px, py, pz);
       double kl = dl, kr = dr;
-      if (a.walk) {
+      if (a.walk && p.ok) {
         const float4* disc = reinterpret_cast<const float4*>(a.walk + (nd - a.nodes)) + 1;
         float v2;
-        kl = fmax(kl, static_cast<double>(disc_bound2(fx, fy, fz, __ldg(disc), __ldg(disc + 1),
-                                                      margin, v2)));
-        kr = fmax(kr, static_cast<double>(disc_bound2(fx, fy, fz, __ldg(disc + 2),
-                                                      __ldg(disc + 3), margin, v2)));
+        const float l = disc_bound2(p.x, p.y, p.z, __ldg(disc), __ldg(disc + 1), p.margin, v2);
+        const float r = disc_bound2(p.x, p.y, p.z, __ldg(disc + 2), __ldg(disc + 3), p.margin, v2);
+        kl = fmax(kl, static_cast<double>(l) * unit * unit);
+        kr = fmax(kr, static_cast<double>(r) * unit * unit);
       }
       // Farther child first, so the nearer one is popped next (capi.mojo:571-586).
       const bool left_near = dl < dr;
@@ -225,16 +241,13 @@ __global__ void __launch_bounds__(kAabbThreads) aabb_any_order_kernel(const Aabb
   if (t >= a.np) return;
   const int64_t qi = a.perm ? static_cast<int64_t>(a.perm[t]) : t;
   const double px = a.P[3 * qi], py = a.P[3 * qi + 1], pz = a.P[3 * qi + 2];
-  // No bound skips anything for huge or non-finite input.
-  const double size = a.scale + fabs(px) + fabs(py) + fabs(pz);
-  const float margin = size < 1e15 ? kWalkMargin * __double2float_ru(size) : INFINITY;
-  const float fx = static_cast<float>(px), fy = static_cast<float>(py),
-              fz = static_cast<float>(pz);
+  const Local p = local_of(a, px, py, pz);
+  const float fx = p.x, fy = p.y, fz = p.z, margin = p.margin;
   Best r{1.0e300, 0.0, 0.0, 0.0, -1};
-  float bestf = INFINITY;  // r.d2, rounded up
+  float bestf = INFINITY;  // r.d2 in the tree's frame, rounded up
   int tie[kTies], tie_slot[kTies], nties = 0;  // face records that evaluate to r.d2
   uint2* stack = s_stack + threadIdx.x;
-  int sp = 0, node = 0;
+  int sp = 0, node = p.ok ? 0 : -1;
   while (node >= 0) {
     const float4* rec = reinterpret_cast<const float4*>(a.walk + node);
     const int4 meta = __ldg(reinterpret_cast<const int4*>(rec));
@@ -259,7 +272,7 @@ __global__ void __launch_bounds__(kAabbThreads) aabb_any_order_kernel(const Aabb
           const ClosestHit h = closest_on_record(a.tris + k, px, py, pz, face);
           if (h.d2 < r.d2) {
             r = Best{h.d2, h.x, h.y, h.z, face};
-            bestf = __double2float_ru(h.d2);
+            bestf = __double2float_ru(h.d2 * a.frame.s * a.frame.s);
             nties = 0;
           }
           if (h.d2 == r.d2) {
@@ -340,17 +353,22 @@ __device__ __forceinline__ T block_reduce(T v, T* part, F f) {
   return v;
 }
 
+__device__ __forceinline__ double3 local_corner(const AabbTriRec& t, int j, const AabbFrame& f) {
+  const double* x = j == 0 ? t.a : (j == 1 ? t.b : t.c);
+  return make_double3((x[0] - f.c[0]) * f.s, (x[1] - f.c[1]) * f.s, (x[2] - f.c[2]) * f.s);
+}
+
 // The disc of one node per CTA: of node list[blockIdx.x], or of node blockIdx.x unless
 // it has more than kDiscBig faces. Three passes over its vertices: normal and shape of
 // the faces; ranges along the normal and two axes across it (the centre); thickness and
 // radius about the centre as rounded to FP32.
 __global__ void aabb_disc_kernel(const AabbTriRec* __restrict__ tris,
                                  const AabbSpan* __restrict__ spans, const int32_t* list,
-                                 double scale, AabbWalkRec* nodes) {
+                                 const AabbFrame f, AabbWalkRec* nodes) {
   __shared__ double part[32];
   const int64_t node = list ? list[blockIdx.x] : static_cast<int64_t>(blockIdx.x);
   const AabbSpan s = spans[node];
-  if (s.slot < 0 || s.last <= s.first || !(scale < 1e100)) return;
+  if (s.slot < 0 || s.last <= s.first) return;
   if (!list && s.last - s.first > kDiscBig) return;
   const int step = static_cast<int>(blockDim.x);
   const auto add = [](double a, double b) { return a + b; };
@@ -359,8 +377,10 @@ __global__ void aabb_disc_kernel(const AabbTriRec* __restrict__ tris,
   double nx = 0.0, ny = 0.0, nz = 0.0, thin = 0.0;
   for (int k = s.first + threadIdx.x; k < s.last; k += step) {
     const AabbTriRec& t = tris[k];
-    const double ux = t.b[0] - t.a[0], uy = t.b[1] - t.a[1], uz = t.b[2] - t.a[2];
-    const double wx = t.c[0] - t.a[0], wy = t.c[1] - t.a[1], wz = t.c[2] - t.a[2];
+    const double ux = (t.b[0] - t.a[0]) * f.s, uy = (t.b[1] - t.a[1]) * f.s,
+                 uz = (t.b[2] - t.a[2]) * f.s;
+    const double wx = (t.c[0] - t.a[0]) * f.s, wy = (t.c[1] - t.a[1]) * f.s,
+                 wz = (t.c[2] - t.a[2]) * f.s;
     const double ex = wx - ux, ey = wy - uy, ez = wz - uz;
     const double cx = uy * wz - uz * wy, cy = uz * wx - ux * wz, cz = ux * wy - uy * wx;
     const double l2 = fmax(fmax(ux * ux + uy * uy + uz * uz, wx * wx + wy * wy + wz * wz),
@@ -392,9 +412,9 @@ __global__ void aabb_disc_kernel(const AabbTriRec* __restrict__ tris,
   double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
   for (int k = s.first + threadIdx.x; k < s.last; k += step)
     for (int j = 0; j < 3; ++j) {
-      const double* x = j == 0 ? tris[k].a : (j == 1 ? tris[k].b : tris[k].c);
-      const double d[3] = {nx * x[0] + ny * x[1] + nz * x[2], ux * x[0] + uy * x[1] + uz * x[2],
-                           wx * x[0] + wy * x[1] + wz * x[2]};
+      const double3 x = local_corner(tris[k], j, f);
+      const double d[3] = {nx * x.x + ny * x.y + nz * x.z, ux * x.x + uy * x.y + uz * x.z,
+                           wx * x.x + wy * x.y + wz * x.z};
       for (int i = 0; i < 3; ++i) {
         lo[i] = fmin(lo[i], d[i]);
         hi[i] = fmax(hi[i], d[i]);
@@ -409,8 +429,8 @@ __global__ void aabb_disc_kernel(const AabbTriRec* __restrict__ tris,
   double t = 0.0, r2 = 0.0, w2 = 0.0;
   for (int k = s.first + threadIdx.x; k < s.last; k += step)
     for (int j = 0; j < 3; ++j) {
-      const double* x = j == 0 ? tris[k].a : (j == 1 ? tris[k].b : tris[k].c);
-      const double dx = x[0] - cx, dy = x[1] - cy, dz = x[2] - cz;
+      const double3 x = local_corner(tris[k], j, f);
+      const double dx = x.x - cx, dy = x.y - cy, dz = x.z - cz;
       const double h = static_cast<double>(fx) * dx + static_cast<double>(fy) * dy +
                        static_cast<double>(fz) * dz;
       const double q = dx * dx + dy * dy + dz * dz;
@@ -424,7 +444,7 @@ __global__ void aabb_disc_kernel(const AabbTriRec* __restrict__ tris,
   if (threadIdx.x != 0) return;
   AabbWalkRec& parent = nodes[s.slot >> 1];
   AabbDisc& out = s.slot & 1 ? parent.rdisc : parent.ldisc;
-  const double pad = 1e-12 * scale;  // >> the rounding of the sums above
+  const double pad = 1e-12;  // >> the rounding of the sums above
   out.n[0] = fx;
   out.n[1] = fy;
   out.n[2] = fz;
@@ -437,13 +457,15 @@ __global__ void aabb_disc_kernel(const AabbTriRec* __restrict__ tris,
 
 // The disc of every face: about its centroid, along its own normal.
 __global__ void aabb_face_disc_kernel(const AabbTriRec* __restrict__ tris, int64_t n,
-                                      double scale, AabbDisc* __restrict__ out,
+                                      const AabbFrame f, AabbDisc* __restrict__ out,
                                       int32_t* __restrict__ thin) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const AabbTriRec& t = tris[i];
-  const double ux = t.b[0] - t.a[0], uy = t.b[1] - t.a[1], uz = t.b[2] - t.a[2];
-  const double wx = t.c[0] - t.a[0], wy = t.c[1] - t.a[1], wz = t.c[2] - t.a[2];
+  const double ux = (t.b[0] - t.a[0]) * f.s, uy = (t.b[1] - t.a[1]) * f.s,
+               uz = (t.b[2] - t.a[2]) * f.s;
+  const double wx = (t.c[0] - t.a[0]) * f.s, wy = (t.c[1] - t.a[1]) * f.s,
+               wz = (t.c[2] - t.a[2]) * f.s;
   const double ex = wx - ux, ey = wy - uy, ez = wz - uz;
   double nx = uy * wz - uz * wy, ny = uz * wx - ux * wz, nz = ux * wy - uy * wx;
   const double l2 = fmax(fmax(ux * ux + uy * uy + uz * uz, wx * wx + wy * wy + wz * wz),
@@ -456,23 +478,23 @@ __global__ void aabb_face_disc_kernel(const AabbTriRec* __restrict__ tris, int64
   d.n[0] = static_cast<float>(nx * inv);
   d.n[1] = static_cast<float>(ny * inv);
   d.n[2] = static_cast<float>(nz * inv);
-  d.t = d.r = INFINITY;
-  for (int j = 0; j < 3; ++j) d.c[j] = static_cast<float>((t.a[j] + t.b[j] + t.c[j]) / 3.0);
-  if (scale < 1e100) {
-    double h = 0.0, r2 = 0.0, w2 = 0.0;
-    for (int j = 0; j < 3; ++j) {
-      const double* x = j == 0 ? t.a : (j == 1 ? t.b : t.c);
-      const double dx = x[0] - d.c[0], dy = x[1] - d.c[1], dz = x[2] - d.c[2];
-      const double p = d.n[0] * dx + d.n[1] * dy + d.n[2] * dz;
-      const double q = dx * dx + dy * dy + dz * dz;
-      h = fmax(h, fabs(p));
-      r2 = fmax(r2, q - p * p);
-      w2 = fmax(w2, q);
-    }
-    const double pad = 1e-12 * scale;
-    d.t = __double2float_ru(h + pad);
-    if (!is_thin) d.r = __double2float_ru(sqrt(r2 + 1e-14 * w2) * (1.0 + 1e-9) + pad);
+  double3 x[3];
+  for (int j = 0; j < 3; ++j) x[j] = local_corner(t, j, f);
+  d.c[0] = static_cast<float>((x[0].x + x[1].x + x[2].x) / 3.0);
+  d.c[1] = static_cast<float>((x[0].y + x[1].y + x[2].y) / 3.0);
+  d.c[2] = static_cast<float>((x[0].z + x[1].z + x[2].z) / 3.0);
+  double h = 0.0, r2 = 0.0, w2 = 0.0;
+  for (int j = 0; j < 3; ++j) {
+    const double dx = x[j].x - d.c[0], dy = x[j].y - d.c[1], dz = x[j].z - d.c[2];
+    const double p = d.n[0] * dx + d.n[1] * dy + d.n[2] * dz;
+    const double q = dx * dx + dy * dy + dz * dz;
+    h = fmax(h, fabs(p));
+    r2 = fmax(r2, q - p * p);
+    w2 = fmax(w2, q);
   }
+  const double pad = 1e-12;
+  d.t = __double2float_ru(h + pad);
+  d.r = is_thin ? INFINITY : __double2float_ru(sqrt(r2 + 1e-14 * w2) * (1.0 + 1e-9) + pad);
   float4* dst = reinterpret_cast<float4*>(out + i);
   dst[0] = make_float4(d.n[0], d.n[1], d.n[2], d.t);
   dst[1] = make_float4(d.c[0], d.c[1], d.c[2], d.r);
@@ -494,7 +516,7 @@ cudaError_t aabb_query(const AabbDeviceTree& t, const double* P, int64_t np, con
   if (np <= 0) return cudaSuccess;
   if (t.depth + 1 > kAabbStack) return cudaErrorInvalidValue;
   AabbArgs a{t.nodes, t.walk, t.tris, t.face_discs, P, perm, sqrd, index, closest, err, np,
-             t.nnodes, {}, t.scale, t.depth};
+             t.nnodes, {}, t.scale, t.frame, t.depth};
   for (int k = 0; k < 6; ++k) a.root[k] = t.root[k];
   const int64_t blocks = (np + kAabbThreads - 1) / kAabbThreads;
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
@@ -511,12 +533,12 @@ cudaError_t aabb_discs(const AabbDeviceTree& t, const AabbSpan* spans, const int
                        int64_t nbig, int32_t* thin, cudaStream_t stream) {
   if (t.nnodes <= 0) return cudaSuccess;
   aabb_disc_kernel<<<static_cast<unsigned>(t.nnodes), 32, 0, stream>>>(t.tris, spans, nullptr,
-                                                                       t.scale, t.walk);
+                                                                       t.frame, t.walk);
   if (nbig > 0)
-    aabb_disc_kernel<<<static_cast<unsigned>(nbig), 512, 0, stream>>>(t.tris, spans, big, t.scale,
+    aabb_disc_kernel<<<static_cast<unsigned>(nbig), 512, 0, stream>>>(t.tris, spans, big, t.frame,
                                                                       t.walk);
   aabb_face_disc_kernel<<<static_cast<unsigned>((t.nleaf_faces + 255) / 256), 256, 0, stream>>>(
-      t.tris, t.nleaf_faces, t.scale, t.face_discs, thin);
+      t.tris, t.nleaf_faces, t.frame, t.face_discs, thin);
   g_launches.fetch_add(nbig > 0 ? 3 : 2, std::memory_order_relaxed);
   return cudaGetLastError();
 }

@@ -16,7 +16,8 @@
 // cylinder, so with h = n.(p - c) and l the distance of p from the axis,
 // max(|h| - t, 0)^2 + max(l - r, 0)^2 bounds the squared distance from p to any of
 // them from below. A child is skipped when that bound, less a rounding margin, exceeds
-// the best squared distance. Points away from a curved surface reach many boxes but
+// the best squared distance. All of this is in the tree's own frame (AabbFrame), so that
+// neither a distant origin nor the unit of length costs the bounds their digits. Points away from a curved surface reach many boxes but
 // few discs: inside a 327,680-face sphere the reference's walk tests 595 faces a point
 // with the boxes alone, 367 with the range of n.x (a slab) beside them, 46 with the
 // discs, 29 when the order is by the discs' centres.
@@ -55,6 +56,13 @@ struct AabbSpan {
   int32_t first, last, slot;
 };
 
+// Where the discs and FP32 boxes live: x' = (x - c) s with the vertices in [-1, 1]^3, s a
+// power of two (the products are exact), ext the largest |x'|; s = 0 for a mesh whose
+// extent is 0 or out of range: no bounds then.
+struct AabbFrame {
+  double c[3] = {}, s = 0.0, ext = 0.0;
+};
+
 struct __align__(16) AabbTriRec {
   double a[3], b[3], c[3];
   int64_t face;
@@ -71,6 +79,7 @@ struct AabbDeviceTree {
   int depth = 0;       // levels, root = 1
   double root[6] = {};  // root box (the traversal tests it when the root is popped)
   double scale = 0.0;   // largest |coordinate| of the mesh (sets the rounding margin)
+  AabbFrame frame;
   bool any_order = false;  // aabb_pack's *regular, and no thin face (aabb_discs)
 };
 
@@ -117,19 +126,22 @@ int64_t aabb_build(const double* V, int64_t nv, const int64_t* F, int64_t nf, in
 // Validates caller-supplied tree arrays and converts them to the device
 // records (host memory, caller-sized: nnodes node and walk records and spans, nf face
 // records); the discs are left without bounds, for aabb_discs to fill in on the device.
-// *scale receives the largest |coordinate| of the mesh; *regular whether every box holds
+// *scale receives the largest |coordinate| of the mesh and *frame its frame; *regular whether every box holds
 // its children's boxes or its faces and every face lies in one leaf, as in the trees
 // that aabb_build makes. Returns the depth (root = 1), or a negative value with the
 // reason in *why.
 int64_t aabb_pack(const double* V, int64_t nv, const int64_t* F, int64_t nf, const double* boxes,
                   const int64_t* nodes, const int64_t* order, int64_t nnodes,
                   AabbNodeRec* node_out, AabbWalkRec* walk_out, AabbSpan* span_out,
-                  AabbTriRec* tri_out, double* scale, bool* regular, const char** why);
+                  AabbTriRec* tri_out, double* scale, AabbFrame* frame, bool* regular,
+                  const char** why);
 
-// The walk's bounds are computed in FP32 from p - c: kWalkMargin * (scale + |px| + |py| +
-// |pz|) covers the rounding of p, of the differences and of their products (under 20
-// units of 2^-24 of the coordinates), kWalkRel the relative rest; both are far above
-// the rounding of the reference's own FP64 closest-point arithmetic.
+// The walk's bounds are computed in FP32 in the tree's frame: kWalkMargin * (ext + |px'| +
+// |py'| + |pz'|) covers the rounding of p', of the differences and of their products (under
+// 20 units of 2^-24), kWalkRel the relative rest. kWalkRound * (scale + |px| + |py| + |pz|),
+// brought into the frame, covers the rounding of the closest points' own coordinates in the
+// reference's FP64 arithmetic (a few units of 2^-53 of them).
 constexpr float kWalkMargin = 2e-6f, kWalkRel = 1e-5f;
+constexpr double kWalkRound = 1e-14;
 
 }  // namespace wn

@@ -232,6 +232,22 @@ bool node_spans(const int64_t* nodes, int64_t nnodes, AabbSpan* span) {
   return whole;
 }
 
+// Extents outside [2^-400, 2^400] have no frame: s^2 and its inverse times a squared
+// distance stay within FP64.
+AabbFrame frame_of(const double* lo, const double* hi) {
+  AabbFrame f;
+  double ext = 0.0;
+  for (int k = 0; k < 3; ++k) {
+    f.c[k] = 0.5 * lo[k] + 0.5 * hi[k];
+    ext = std::max(ext, 0.5 * hi[k] - 0.5 * lo[k]);
+  }
+  int e = 0;
+  std::frexp(ext, &e);  // ext <= 2^e
+  if (ext > 0.0 && e > -400 && e < 400) f.s = std::ldexp(1.0, -e);
+  f.ext = ext * f.s;
+  return f;
+}
+
 // Whether `box` holds the n points.
 bool holds(const double* box, const double* points, int64_t n) {
   for (int64_t k = 0; k < n; ++k, points += 3)
@@ -245,14 +261,17 @@ bool holds(const double* box, const double* points, int64_t n) {
 int64_t aabb_pack(const double* V, int64_t nv, const int64_t* F, int64_t nf, const double* boxes,
                   const int64_t* nodes, const int64_t* order, int64_t nnodes,
                   AabbNodeRec* node_out, AabbWalkRec* walk_out, AabbSpan* span_out,
-                  AabbTriRec* tri_out, double* scale, bool* regular, const char** why) {
+                  AabbTriRec* tri_out, double* scale, AabbFrame* frame, bool* regular,
+                  const char** why) {
   *regular = false;
   *scale = 0.0;
+  *frame = AabbFrame{};
   if (nnodes == 0) return 0;
   if (nnodes < 0 || nnodes > 0x7fffffffLL || nf <= 0 || nf > 0x7fffffffLL) {
     *why = "node or face count out of range";
     return -1;
   }
+  double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
   for (int64_t i = 0; i < nf; ++i) {
     const int64_t f = order[i];
     if (f < 0 || f >= nf) {
@@ -274,10 +293,13 @@ int64_t aabb_pack(const double* V, int64_t nv, const int64_t* F, int64_t nf, con
           return -1;
         }
         *scale = std::max(*scale, std::fabs(dst[k]));
+        lo[k] = std::min(lo[k], dst[k]);
+        hi[k] = std::max(hi[k], dst[k]);
       }
     }
     r.face = f;
   }
+  *frame = frame_of(lo, hi);
   // Depth of every node, walking in index order: children must come after
   // their parent (true of any preorder numbering), which also rules out cycles.
   std::vector<int32_t> level(static_cast<size_t>(nnodes), 0);
@@ -323,7 +345,9 @@ int64_t aabb_pack(const double* V, int64_t nv, const int64_t* F, int64_t nf, con
     return -1;
   }
   bool sound = node_spans(nodes, nnodes, span_out);
+  sound = sound && frame->s > 0.0;
   const AabbDisc none{{0.f, 0.f, 0.f}, INFINITY, {0.f, 0.f, 0.f}, INFINITY};
+  auto local = [&](double x, int k) { return (x - frame->c[k]) * frame->s; };
   for (int64_t i = 0; i < nnodes; ++i) {
     const AabbNodeRec& r = node_out[i];
     AabbWalkRec& w = walk_out[i];
@@ -344,10 +368,10 @@ int64_t aabb_pack(const double* V, int64_t nv, const int64_t* F, int64_t nf, con
     w.start = span_out[r.right].first;
     sound = sound && holds(box, r.lbox, 2) && holds(box, r.rbox, 2);
     for (int k = 0; k < 3; ++k) {
-      w.lbox[k] = round_down(r.lbox[k]);
-      w.rbox[k] = round_down(r.rbox[k]);
-      w.lbox[3 + k] = round_up(r.lbox[3 + k]);
-      w.rbox[3 + k] = round_up(r.rbox[3 + k]);
+      w.lbox[k] = round_down(local(r.lbox[k], k));
+      w.rbox[k] = round_down(local(r.rbox[k], k));
+      w.lbox[3 + k] = round_up(local(r.lbox[3 + k], k));
+      w.rbox[3 + k] = round_up(local(r.rbox[3 + k], k));
     }
   }
   *regular = sound;

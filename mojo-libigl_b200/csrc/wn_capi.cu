@@ -1115,9 +1115,11 @@ int wn_aabb_create(const double* V, int64_t nv, const int64_t* F, int64_t nf,
   std::vector<AabbSpan> spans(static_cast<size_t>(nnodes));
   const char* why = "";
   double scale = 0.0;
+  AabbFrame frame;
   bool regular = false;
   const int64_t depth = aabb_pack(V, nv, F, nf, boxes, nodes, order, nnodes, nrec.data(),
-                                  wrec.data(), spans.data(), trec.data(), &scale, &regular, &why);
+                                  wrec.data(), spans.data(), trec.data(), &scale, &frame,
+                                  &regular, &why);
   if (depth < 0) return fail(WN_EINVAL, "invalid tree: %s", why);
   std::lock_guard<std::mutex> lock(g_mutex);
   int code = WN_OK;
@@ -1129,6 +1131,7 @@ int wn_aabb_create(const double* V, int64_t nv, const int64_t* F, int64_t nf,
   h->t.nleaf_faces = static_cast<int64_t>(trec.size());
   h->t.depth = static_cast<int>(depth);
   h->t.scale = scale;
+  h->t.frame = frame;
   if (nnodes > 0) {
     for (int k = 0; k < 6; ++k) h->t.root[k] = boxes[k];
     std::vector<int32_t> big;  // nodes whose discs take a CTA each
