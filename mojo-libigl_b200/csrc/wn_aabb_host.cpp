@@ -208,12 +208,12 @@ float round_up(double x) {
   return f;
 }
 
-// Every node's run of face records and its place beside its parent; false unless every
-// internal node's run is its left child's followed by its right child's and every node
-// but the root has one parent (else, possible only in a caller-made tree, the runs mean
-// nothing).
+// Every node's run of face records (empty where its children's are not one run, possible
+// only in a caller-made tree) and its place beside its parent; true if every internal
+// node's run is its left child's followed by its right child's and every node but the root
+// has one parent.
 bool node_spans(const int64_t* nodes, int64_t nnodes, AabbSpan* span) {
-  bool whole = true;
+  bool ordered = true;
   for (int64_t i = 0; i < nnodes; ++i) span[i].slot = -1;
   for (int64_t i = nnodes - 1; i >= 0; --i) {  // children come after their parent
     const int64_t* nd = nodes + 4 * i;
@@ -223,13 +223,16 @@ bool node_spans(const int64_t* nodes, int64_t nnodes, AabbSpan* span) {
       continue;
     }
     AabbSpan &l = span[nd[0]], &r = span[nd[1]];
-    whole = whole && nd[0] != nd[1] && l.slot < 0 && r.slot < 0 && l.last == r.first;
+    const bool runs = l.first < l.last && r.first < r.last;
+    const bool follows = runs && l.last == r.first;
+    ordered = ordered && nd[0] != nd[1] && l.slot < 0 && r.slot < 0 && follows;
     l.slot = static_cast<int32_t>(2 * i);
     r.slot = static_cast<int32_t>(2 * i + 1);
-    span[i].first = l.first;
-    span[i].last = r.last;
+    const bool whole = follows || (runs && r.last == l.first);
+    span[i].first = whole ? std::min(l.first, r.first) : 0;
+    span[i].last = whole ? std::max(l.last, r.last) : 0;
   }
-  return whole;
+  return ordered;
 }
 
 // Extents outside [2^-400, 2^400] have no frame: s^2 and its inverse times a squared

@@ -1134,8 +1134,9 @@ int wn_aabb_create(const double* V, int64_t nv, const int64_t* F, int64_t nf,
   h->t.frame = frame;
   if (nnodes > 0) {
     for (int k = 0; k < 6; ++k) h->t.root[k] = boxes[k];
+    const bool discs = frame.s > 0.0;
     std::vector<int32_t> big;  // nodes whose discs take a CTA each
-    if (regular)
+    if (discs)
       for (int64_t i = 0; i < nnodes; ++i)
         if (spans[i].last - spans[i].first > kDiscBig) big.push_back(static_cast<int32_t>(i));
     const int64_t nbig = static_cast<int64_t>(big.size());
@@ -1153,7 +1154,7 @@ int wn_aabb_create(const double* V, int64_t nv, const int64_t* F, int64_t nf,
         (e = dev_malloc(&h->t.tris, sizeof(AabbTriRec) * trec.size())) != cudaSuccess ||
         (e = upload(h->t.nodes, nrec.data(), sizeof(AabbNodeRec) * nrec.size())) != cudaSuccess ||
         (e = upload(h->t.tris, trec.data(), sizeof(AabbTriRec) * trec.size())) != cudaSuccess ||
-        (regular &&
+        (discs &&
          ((e = dev_malloc(&h->t.walk, sizeof(AabbWalkRec) * wrec.size())) != cudaSuccess ||
           (e = dev_malloc(&h->t.face_discs, sizeof(AabbDisc) * trec.size())) != cudaSuccess ||
           (e = dev_malloc(&spans_d, sizeof(AabbSpan) * spans.size())) != cudaSuccess ||
