@@ -55,6 +55,11 @@ constexpr int kGroup = 16;
 // walk's stack. The library's own trees have at most 30 (2^31 faces); a caller-made one may
 // have 63, and takes the reference's walk, whose stack is in local memory.
 constexpr size_t kStackBytes = 48 << 10;
+// The reference's walk takes the discs' bounds on meshes of at least kDiscFaces of which one
+// in kDiscShare is thin at most, else the slabs alone (131,072 points, ms, slabs and discs:
+// one thin face in 327,681 3.7 and 2.4, in 20,481 0.96 and 1.00; a tenth of 327,680 10.0 and
+// 11.3, since a disc over a thin face has no radius).
+constexpr int64_t kDiscFaces = 65536, kDiscShare = 1024;
 // A face is thin below |n|^2 = kThin * (longest side)^4: thinner than about 1 : 1000.
 constexpr double kThin = 1e-6;
 
@@ -90,7 +95,7 @@ __device__ __forceinline__ Local local_of(const AabbArgs& a, double px, double p
   const double round = kWalkRound * (a.scale + fabs(px) + fabs(py) + fabs(pz)) * a.frame.s;
   return Local{static_cast<float>(x), static_cast<float>(y), static_cast<float>(z),
                kWalkMargin * __double2float_ru(size) + __double2float_ru(round),
-               size < 1e15 && round < 1e-3 * size};
+               a.walk != nullptr && size < 1e15 && round < 1e-3 * size};
 }
 
 struct Best {
@@ -126,13 +131,31 @@ __device__ __forceinline__ float disc_bound2(float px, float py, float pz, const
   const float l = fmaxf(sqrtf(fmaxf(v2 * (1.0f - 2e-6f) - h * h, 0.0f)) - cr.w - e, 0.0f);
   return (g * g + l * l) * (1.0f - kWalkRel);
 }
+// A point in the tree's frame in FP64, the margin of its slab bounds there, and what brings
+// their squares back (kSlabMargin for their own rounding among it).
+struct Slabs {
+  double x, y, z, margin, back;
+};
+__device__ __forceinline__ double slab_bound2(const Slabs& p, float nx, float ny, float nz, float lo,
+                                              float hi) {
+  const double h = fma(static_cast<double>(nz), p.z,
+                       fma(static_cast<double>(ny), p.y, static_cast<double>(nx) * p.x));
+  const double g = fmax(static_cast<double>(lo) - h, h - static_cast<double>(hi)) - p.margin;
+  return g > 0.0 ? g * g * p.back : 0.0;
+}
+
 // The reference's walk. Each stack entry keeps the box distance computed when it was
 // pushed (the reference recomputes the same double from the same box at the pop), or
 // the disc bound where that is larger: such a child holds no face that the reference
 // would take. The order is decided by the box distances alone.
-__device__ __noinline__ Best ordered_walk(const AabbArgs& a, double px, double py, double pz) {
+template <bool DISCS>
+__device__ __forceinline__ Best walk_in_order(const AabbArgs& a, double px, double py, double pz) {
   const Local p = local_of(a, px, py, pz);
-  const double unit = a.frame.s > 0.0 ? 1.0 / a.frame.s : 0.0;
+  const double unit = p.ok ? 1.0 / a.frame.s : 0.0;
+  const Slabs s{(px - a.frame.c[0]) * a.frame.s, (py - a.frame.c[1]) * a.frame.s,
+                (pz - a.frame.c[2]) * a.frame.s,
+                p.ok ? kSlabMargin * (a.scale + fabs(px) + fabs(py) + fabs(pz)) * a.frame.s : INFINITY,
+                unit * unit * (1.0 - kSlabMargin)};
   Best r{1.0e300, 0.0, 0.0, 0.0, -1};
   int stack_node[kAabbStack];
   double stack_d2[kAabbStack];
@@ -149,21 +172,34 @@ __device__ __noinline__ Best ordered_walk(const AabbArgs& a, double px, double p
     const AabbNodeRec* nd = a.nodes + stack_node[sp];
     const int4 meta = __ldg(reinterpret_cast<const int4*>(nd));
     if (meta.w > 0) {
-      for (int k = 0; k < meta.w; ++k) {
+      const AabbTriRec* tr = a.tris + meta.z;
+      for (int k = 0; k < meta.w; ++k, ++tr) {
         int64_t face;
-        const ClosestHit h = closest_on_record(a.tris + meta.z + k, px, py, pz, face);
-        if (h.d2 < r.d2) r = Best{h.d2, h.x, h.y, h.z, face};
+        const ClosestHit h = closest_on_record(tr, px, py, pz, face);
+        if (h.d2 < r.d2) {
+          r.d2 = h.d2;
+          r.face = face;
+          r.x = h.x;
+          r.y = h.y;
+          r.z = h.z;
+        }
       }
     } else {
       const double dl = box_of(nd->lbox, px, py, pz), dr = box_of(nd->rbox, px, py, pz);
       double kl = dl, kr = dr;
-      if (a.walk && p.ok) {
+      if (DISCS && p.ok) {
         const float4* disc = reinterpret_cast<const float4*>(a.walk + (nd - a.nodes)) + 1;
         float v2;
         const float l = disc_bound2(p.x, p.y, p.z, __ldg(disc), __ldg(disc + 1), p.margin, v2);
         const float r = disc_bound2(p.x, p.y, p.z, __ldg(disc + 2), __ldg(disc + 3), p.margin, v2);
         kl = fmax(kl, static_cast<double>(l) * unit * unit);
         kr = fmax(kr, static_cast<double>(r) * unit * unit);
+      } else if (!DISCS) {
+        const float4* w = reinterpret_cast<const float4*>(&nd->lslab);
+        const float4 s0 = __ldg(w), s1 = __ldg(w + 1);
+        const float2 s2 = __ldg(reinterpret_cast<const float2*>(w + 2));
+        kl = fmax(kl, slab_bound2(s, s0.x, s0.y, s0.z, s0.w, s1.x));
+        kr = fmax(kr, slab_bound2(s, s1.y, s1.z, s1.w, s2.x, s2.y));
       }
       // Farther child first, so the nearer one is popped next (capi.mojo:571-586).
       const bool left_near = dl < dr;
@@ -189,6 +225,10 @@ __device__ __noinline__ Best ordered_walk(const AabbArgs& a, double px, double p
   return r;
 }
 
+__device__ __noinline__ Best ordered_walk(const AabbArgs& a, double px, double py, double pz) {
+  return walk_in_order<true>(a, px, py, pz);
+}
+
 __device__ __forceinline__ void store_result(const AabbArgs& a, int64_t qi, const Best& r) {
   a.sqrd[qi] = r.d2;
   a.index[qi] = r.face;
@@ -197,11 +237,12 @@ __device__ __forceinline__ void store_result(const AabbArgs& a, int64_t qi, cons
   a.closest[3 * qi + 2] = r.z;
 }
 
+template <bool DISCS>
 __global__ void __launch_bounds__(kAabbThreads) aabb_query_kernel(const AabbArgs a) {
   const int64_t t = static_cast<int64_t>(blockIdx.x) * kAabbThreads + threadIdx.x;
   if (t >= a.np) return;
   const int64_t qi = a.perm ? static_cast<int64_t>(a.perm[t]) : t;
-  store_result(a, qi, ordered_walk(a, a.P[3 * qi], a.P[3 * qi + 1], a.P[3 * qi + 2]));
+  store_result(a, qi, walk_in_order<DISCS>(a, a.P[3 * qi], a.P[3 * qi + 1], a.P[3 * qi + 2]));
 }
 
 __device__ __forceinline__ float box_bound2(float px, float py, float pz, float lx, float ly,
@@ -364,7 +405,7 @@ __device__ __forceinline__ double3 local_corner(const AabbTriRec& t, int j, cons
 // radius about the centre as rounded to FP32.
 __global__ void aabb_disc_kernel(const AabbTriRec* __restrict__ tris,
                                  const AabbSpan* __restrict__ spans, const int32_t* list,
-                                 const AabbFrame f, AabbWalkRec* nodes) {
+                                 const AabbFrame f, AabbWalkRec* walk, AabbNodeRec* nodes) {
   __shared__ double part[32];
   const int64_t node = list ? list[blockIdx.x] : static_cast<int64_t>(blockIdx.x);
   const AabbSpan s = spans[node];
@@ -426,7 +467,7 @@ __global__ void aabb_disc_kernel(const AabbTriRec* __restrict__ tris,
   const float cx = static_cast<float>(nx * mid[0] + ux * mid[1] + wx * mid[2]);
   const float cy = static_cast<float>(ny * mid[0] + uy * mid[1] + wy * mid[2]);
   const float cz = static_cast<float>(nz * mid[0] + uz * mid[1] + wz * mid[2]);
-  double t = 0.0, r2 = 0.0, w2 = 0.0;
+  double t = 0.0, r2 = 0.0, w2 = 0.0, dlo = INFINITY, dhi = -INFINITY;
   for (int k = s.first + threadIdx.x; k < s.last; k += step)
     for (int j = 0; j < 3; ++j) {
       const double3 x = local_corner(tris[k], j, f);
@@ -434,16 +475,22 @@ __global__ void aabb_disc_kernel(const AabbTriRec* __restrict__ tris,
       const double h = static_cast<double>(fx) * dx + static_cast<double>(fy) * dy +
                        static_cast<double>(fz) * dz;
       const double q = dx * dx + dy * dy + dz * dz;
+      const double d = static_cast<double>(fx) * x.x + static_cast<double>(fy) * x.y +
+                       static_cast<double>(fz) * x.z;
       t = fmax(t, fabs(h));
       r2 = fmax(r2, q - h * h);
       w2 = fmax(w2, q);
+      dlo = fmin(dlo, d);
+      dhi = fmax(dhi, d);
     }
+  dlo = block_reduce(dlo, part, low);
+  dhi = block_reduce(dhi, part, high);
   t = block_reduce(t, part, high);
   r2 = block_reduce(r2, part, high);
   w2 = block_reduce(w2, part, high);
   if (threadIdx.x != 0) return;
-  AabbWalkRec& parent = nodes[s.slot >> 1];
-  AabbDisc& out = s.slot & 1 ? parent.rdisc : parent.ldisc;
+  const bool right = s.slot & 1;
+  AabbDisc& out = right ? walk[s.slot >> 1].rdisc : walk[s.slot >> 1].ldisc;
   const double pad = 1e-12;  // >> the rounding of the sums above
   out.n[0] = fx;
   out.n[1] = fy;
@@ -453,6 +500,9 @@ __global__ void aabb_disc_kernel(const AabbTriRec* __restrict__ tris,
   out.c[2] = cz;
   out.t = __double2float_ru(t + pad);
   out.r = thin > 0.0 ? INFINITY : __double2float_ru(sqrt(r2 + 1e-14 * w2) * (1.0 + 1e-9) + pad);
+  AabbNodeRec& parent = nodes[s.slot >> 1];
+  (right ? parent.rslab : parent.lslab) =
+      AabbSlab{{fx, fy, fz}, __double2float_rd(dlo - pad), __double2float_ru(dhi + pad)};
 }
 
 // The disc of every face: about its centroid, along its own normal.
@@ -472,7 +522,7 @@ __global__ void aabb_face_disc_kernel(const AabbTriRec* __restrict__ tris, int64
                          ex * ex + ey * ey + ez * ez);
   const double nn = nx * nx + ny * ny + nz * nz;
   const bool is_thin = !(nn >= kThin * l2 * l2);
-  if (is_thin) *thin = 1;
+  if (is_thin) atomicAdd(thin, 1);
   const double inv = nn > 0.0 && nn < INFINITY ? (1.0 - 1.5e-7) / sqrt(nn) : 0.0;
   AabbDisc d;
   d.n[0] = static_cast<float>(nx * inv);
@@ -523,8 +573,10 @@ cudaError_t aabb_query(const AabbDeviceTree& t, const double* P, int64_t np, con
   const size_t stack_bytes = sizeof(uint2) * kAabbThreads * t.depth;
   if (t.any_order && t.nnodes > 0 && stack_bytes <= kStackBytes)
     aabb_any_order_kernel<<<static_cast<unsigned>(blocks), kAabbThreads, stack_bytes, stream>>>(a);
+  else if (t.nleaf_faces >= kDiscFaces && t.thin <= t.nleaf_faces / kDiscShare)
+    aabb_query_kernel<true><<<static_cast<unsigned>(blocks), kAabbThreads, 0, stream>>>(a);
   else
-    aabb_query_kernel<<<static_cast<unsigned>(blocks), kAabbThreads, 0, stream>>>(a);
+    aabb_query_kernel<false><<<static_cast<unsigned>(blocks), kAabbThreads, 0, stream>>>(a);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return cudaGetLastError();
 }
@@ -533,10 +585,10 @@ cudaError_t aabb_discs(const AabbDeviceTree& t, const AabbSpan* spans, const int
                        int64_t nbig, int32_t* thin, cudaStream_t stream) {
   if (t.nnodes <= 0) return cudaSuccess;
   aabb_disc_kernel<<<static_cast<unsigned>(t.nnodes), 32, 0, stream>>>(t.tris, spans, nullptr,
-                                                                       t.frame, t.walk);
+                                                                       t.frame, t.walk, t.nodes);
   if (nbig > 0)
     aabb_disc_kernel<<<static_cast<unsigned>(nbig), 512, 0, stream>>>(t.tris, spans, big, t.frame,
-                                                                      t.walk);
+                                                                      t.walk, t.nodes);
   aabb_face_disc_kernel<<<static_cast<unsigned>((t.nleaf_faces + 255) / 256), 256, 0, stream>>>(
       t.tris, t.nleaf_faces, t.frame, t.face_discs, thin);
   g_launches.fetch_add(nbig > 0 ? 3 : 2, std::memory_order_relaxed);

@@ -34,12 +34,21 @@ struct __align__(16) AabbDisc {
   float c[3], r;  // centre, radius; +inf: no bound across n
 };
 
-struct __align__(16) AabbNodeRec {
+// Faces between two planes: lo <= n.x' <= hi (infinite: no bound), the disc's thickness
+// without FP32's margin. The reference's walk needs that: of the leaves that a point away
+// from the surface could reach, one in ten is told apart by less than the margin.
+struct AabbSlab {
+  float n[3], lo, hi;
+};
+
+struct __align__(32) AabbNodeRec {
   int32_t left, right, start, count;  // count > 0: a leaf of faces [start, start+count)
   double lbox[6];  // left child's box (lo xyz, hi xyz); unused for a leaf
   double rbox[6];  // right child's box
+  AabbSlab lslab, rslab;
+  int32_t pad[2];
 };
-static_assert(sizeof(AabbNodeRec) == 112, "node record is seven 16-byte words");
+static_assert(sizeof(AabbNodeRec) == 160, "node record is five 32-byte sectors");
 
 struct __align__(16) AabbWalkRec {
   int32_t left, right;  // a leaf: its place beside its parent (AabbSpan::slot), unused
@@ -80,6 +89,7 @@ struct AabbDeviceTree {
   double root[6] = {};  // root box (the traversal tests it when the root is popped)
   double scale = 0.0;   // largest |coordinate| of the mesh (sets the rounding margin)
   AabbFrame frame;
+  int32_t thin = 0;    // thin faces (aabb_discs)
   bool any_order = false;  // aabb_pack's *regular, and no thin face (aabb_discs)
 };
 
@@ -99,9 +109,9 @@ cudaError_t aabb_query(const AabbDeviceTree& t, const double* P, int64_t np, con
                        double* sqrd, int64_t* index, double* closest, int* err,
                        cudaStream_t stream);
 
-// Fills in the discs of a tree, its nodes' and its faces', whose records are on the
-// device (spans: nnodes, device; big: the nbig nodes of more than kDiscBig faces,
-// device). *thin (device, set to 0 before) becomes 1 if some face is thinner than
+// Fills in the discs and slabs of a tree, its nodes' and its faces', whose records are on
+// the device (spans: nnodes, device; big: the nbig nodes of more than kDiscBig faces,
+// device). *thin (device, set to 0 before) receives the number of faces thinner than
 // 1 : 1000: the reference's closest point on such a face may lie off it (the barycentric
 // quotients lose their digits), so no bound holds for it and only the reference's own
 // order says whether it is looked at.
@@ -143,5 +153,9 @@ int64_t aabb_pack(const double* V, int64_t nv, const int64_t* F, int64_t nf, con
 // reference's FP64 arithmetic (a few units of 2^-53 of them).
 constexpr float kWalkMargin = 2e-6f, kWalkRel = 1e-5f;
 constexpr double kWalkRound = 1e-14;
+// The slabs' margin (FP64) is kSlabMargin * (scale + |px| + |py| + |pz|): the rounding of n.x'
+// and of the reference's closest points, a few units of 2^-53 of the coordinates, with a
+// factor above 1000 to spare.
+constexpr double kSlabMargin = 4e-12;
 
 }  // namespace wn

@@ -312,6 +312,8 @@ int64_t aabb_pack(const double* V, int64_t nv, const int64_t* F, int64_t nf, con
     const int64_t* nd = nodes + 4 * i;
     AabbNodeRec& r = node_out[i];
     for (int k = 0; k < 6; ++k) r.lbox[k] = r.rbox[k] = 0.0;
+    r.lslab = r.rslab = AabbSlab{{0.f, 0.f, 0.f}, -INFINITY, INFINITY};
+    r.pad[0] = r.pad[1] = 0;
     if (level[i] == 0) {
       *why = "node unreachable from the root";
       return -1;

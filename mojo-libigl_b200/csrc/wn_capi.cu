@@ -1140,7 +1140,7 @@ int wn_aabb_create(const double* V, int64_t nv, const int64_t* F, int64_t nf,
       for (int64_t i = 0; i < nnodes; ++i)
         if (spans[i].last - spans[i].first > kDiscBig) big.push_back(static_cast<int32_t>(i));
     const int64_t nbig = static_cast<int64_t>(big.size());
-    big.push_back(0);  // the flag for thin faces
+    big.push_back(0);  // the count of thin faces
     AabbSpan* spans_d = nullptr;
     int32_t* big_d = nullptr;
     int32_t thin = 0;
@@ -1179,6 +1179,7 @@ int wn_aabb_create(const double* V, int64_t nv, const int64_t* F, int64_t nf,
     }
     cudaFree(spans_d);
     cudaFree(big_d);
+    h->t.thin = thin;
     h->t.any_order = regular && thin == 0;
   }
   *tree = h;

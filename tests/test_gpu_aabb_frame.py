@@ -77,3 +77,17 @@ def test_points_beyond_any_bound(bad):
         assert (mixed[1][~keep] == -1).all()
     if not np.isnan(bad):  # the reference's walk visits every node for NaN
         assert _ms(tree, Q) < 3 * _ms(tree, P)
+
+
+@pytest.mark.parametrize("level, every", [(6, 81920), (6, 10), (4, 5120), (4, 10)])
+def test_thin_faces(level, every):
+    """Meshes with thin faces take the reference's walk, the larger ones with few of them by
+    the discs and the others by the slabs."""
+    V, F = synthetic.bumpy_icosphere(level, seed=4)
+    P = np.concatenate([synthetic.mixed_queries(V, F, 4000, 5, near_sigma=1e-3), 30 * V[:200]])
+    at = F[::every, 0]
+    F = F.copy()
+    F[::every, 1] = len(V) + np.arange(len(at))
+    V = np.concatenate([V, V[at] + 1e-6])
+    _check(V, F, P)
+    _check(V + [4.5e5, 5.2e6, 300], F, P + [4.5e5, 5.2e6, 300])
