@@ -13,15 +13,15 @@
 //    the others with the reference's FP64 arithmetic (wn_aabb.cuh). What it skips is
 //    farther than the best, so afterwards `best` is the smallest squared distance B
 //    that any face of the mesh evaluates to, and the faces that evaluate to B exactly
-//    have all been seen.
-// 2. The reference's result is the first of these in its order, if it looks at all of
-//    them: a leaf is looked at when its box distance is <= the best at that time, and
-//    that is never below B. So if every one of their leaves has a box distance <= B,
-//    the winner is the first by the walk's order, which two faces' common ancestor
-//    decides: the child with the smaller box distance comes first (the right one when
-//    they are equal), within a leaf the order of the records.
-// 3. Where rounding puts a leaf's box distance above B, or more than kTies faces tie,
-//    the thread does the reference's own walk.
+//    have all been seen. Of these the walk keeps the first in the reference's order,
+//    which two faces' common ancestor decides: the child with the smaller box distance
+//    comes first (the right one when they are equal), within a leaf the order of the
+//    records.
+// 2. The reference's result is that face if it looks at it: a leaf is looked at when its
+//    box distance is <= the best at that time, which before that face is above B. So a
+//    leaf whose box distance is <= B is.
+// 3. Where rounding puts the leaf's box distance above B, the thread does the reference's
+//    own walk.
 //
 // Trees that the library did not build may have boxes that do not hold their faces,
 // and closest points on very thin faces lose their digits: no bound of step 1 holds
@@ -30,9 +30,11 @@
 // Bound by the walks' divergence and load latency, not by HBM or FP64 throughput (the
 // tree sits in L2; ncu, 524,288 points inside and around the 327,680-face sphere: 8.2 of
 // 32 lanes active, issue 42 %, FP64 pipe 15 %). Measured against the reference's walk
-// with box and slab (a range of n.x) alone: 327,680 faces x 2^20 points 10.1 -> 2.4 ms,
+// with box and slab (a range of n.x) alone: 327,680 faces x 2^20 points 10.1 -> 2.3 ms,
 // 243,602 (terrain) x 2^20 1.54 -> 1.34 ms, x 10,000 0.18 -> 0.12 ms. The reference's
-// order with the discs: 5.1 ms. Keeping the warp's lanes in step, leaves held until 1, 4,
+// order with the discs: 5.1 ms. Ties kept in a list and compared at the end, from the root
+// down: 2.76 -> 2.57 ms for the whole call, and 131,072 of the mesh's own vertices 0.70 ->
+// 0.45 (the reference's walk: 0.31). Keeping the warp's lanes in step, leaves held until 1, 4,
 // 8 or more lanes have one: slower in either order (3.2 ms at best here).
 #include <cuda_runtime.h>
 
@@ -45,7 +47,6 @@ namespace wn {
 namespace {
 
 constexpr int kAabbThreads = 128;
-constexpr int kTies = 8;
 // Consecutive points of the (Morton) order that share a warp; its other lanes take
 // points from elsewhere, so that 32 of the longest walks do not meet in one warp, which
 // the rest of the GPU then waits for (327,680 faces x 2^20 points, stack in local memory:
@@ -66,6 +67,7 @@ constexpr double kThin = 1e-6;
 struct AabbArgs {
   const AabbNodeRec* __restrict__ nodes;
   const AabbWalkRec* __restrict__ walk;
+  const AabbSpan* __restrict__ spans;
   const AabbTriRec* __restrict__ tris;
   const AabbDisc* __restrict__ face_discs;
   const double* __restrict__ P;
@@ -253,22 +255,22 @@ __device__ __forceinline__ float box_bound2(float px, float py, float pz, float 
   return (x * x + y * y + z * z) * (1.0f - kWalkRel);
 }
 
-// Whether the reference's walk reaches face record i before face record j.
-__device__ __forceinline__ bool comes_first(const AabbArgs& a, int i, int j, double px, double py,
+// Whether the reference's walk reaches the leaf at slot `at` before face record j of another
+// leaf: up to the node that holds both (a vertex's faces lie in leaves a few levels apart;
+// from the root down it took three times the loads).
+__device__ __forceinline__ bool comes_first(const AabbArgs& a, int at, int j, double px, double py,
                                             double pz) {
-  int node = 0;
-  for (;;) {
-    const int4 m = __ldg(reinterpret_cast<const int4*>(a.walk + node));
-    if (m.w > 0) return i < j;
-    const bool il = i < m.z, jl = j < m.z;
-    if (il == jl) {
-      node = il ? m.x : m.y;
-      continue;
+  while (at >= 0) {
+    const int node = at >> 1;
+    const int4 s = __ldg(reinterpret_cast<const int4*>(a.spans + node));
+    if (j >= s.x && j < s.y) {
+      const AabbNodeRec* nd = a.nodes + node;
+      const bool left_near = box_of(nd->lbox, px, py, pz) < box_of(nd->rbox, px, py, pz);
+      return left_near == !(at & 1);
     }
-    const AabbNodeRec* nd = a.nodes + node;
-    const bool left_near = box_of(nd->lbox, px, py, pz) < box_of(nd->rbox, px, py, pz);
-    return il == left_near;
+    at = s.z;
   }
+  return false;  // not reached: the root holds every record
 }
 
 __global__ void __launch_bounds__(kAabbThreads) aabb_any_order_kernel(const AabbArgs a) {
@@ -286,8 +288,9 @@ __global__ void __launch_bounds__(kAabbThreads) aabb_any_order_kernel(const Aabb
   const float fx = p.x, fy = p.y, fz = p.z, margin = p.margin;
   Best r{1.0e300, 0.0, 0.0, 0.0, -1};
   float bestf = INFINITY;  // r.d2 in the tree's frame, rounded up
-  int tie[kTies], tie_slot[kTies], nties = 0;  // face records that evaluate to r.d2
+  int win = -1, win_slot = -1;  // r's face record, its leaf's place
   uint2* stack = s_stack + threadIdx.x;
+  bool complete = p.ok;
   int sp = 0, node = p.ok ? 0 : -1;
   while (node >= 0) {
     const float4* rec = reinterpret_cast<const float4*>(a.walk + node);
@@ -311,17 +314,14 @@ __global__ void __launch_bounds__(kAabbThreads) aabb_any_order_kernel(const Aabb
           todo &= todo - 1;
           int64_t face;
           const ClosestHit h = closest_on_record(a.tris + k, px, py, pz, face);
-          if (h.d2 < r.d2) {
+          // Of equal distances the one that the reference meets first; a leaf's records come
+          // in its order here too.
+          if (h.d2 < r.d2 || (h.d2 == r.d2 && meta.x != win_slot &&
+                              comes_first(a, meta.x, win, px, py, pz))) {
             r = Best{h.d2, h.x, h.y, h.z, face};
             bestf = __double2float_ru(h.d2 * a.frame.s * a.frame.s);
-            nties = 0;
-          }
-          if (h.d2 == r.d2) {
-            if (nties < kTies) {
-              tie[nties] = k;
-              tie_slot[nties] = meta.x;
-            }
-            ++nties;
+            win = k;
+            win_slot = meta.x;
           }
         }
       }
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kAabbThreads) aabb_any_order_kernel(const Aabb
                                                 __float_as_uint(left_first ? kr : kl));
           ++sp;
         } else {
-          nties = kTies + 1;  // not all seen: the reference's walk decides
+          complete = false;  // not all seen: the reference's walk decides
           atomicOr(a.err, kErrBadLaunch);
         }
       } else if (left || right) {
@@ -357,25 +357,15 @@ __global__ void __launch_bounds__(kAabbThreads) aabb_any_order_kernel(const Aabb
     }
     node = go;
   }
-  bool sure = nties >= 1 && nties <= kTies;
-  for (int k = 0; sure && k < nties; ++k) {
-    const int slot = tie_slot[k];
-    const double d = slot < 0 ? box_distance2(px, py, pz, a.root[0], a.root[1], a.root[2],
-                                              a.root[3], a.root[4], a.root[5])
-                              : box_of(slot & 1 ? a.nodes[slot >> 1].rbox : a.nodes[slot >> 1].lbox,
-                                       px, py, pz);
-    sure = d <= r.d2;
+  if (complete && win >= 0) {
+    const double d =
+        win_slot < 0 ? box_distance2(px, py, pz, a.root[0], a.root[1], a.root[2], a.root[3],
+                                     a.root[4], a.root[5])
+                     : box_of(win_slot & 1 ? a.nodes[win_slot >> 1].rbox : a.nodes[win_slot >> 1].lbox,
+                              px, py, pz);
+    complete = d <= r.d2;
   }
-  if (sure && nties > 1) {
-    int win = tie[0];
-    for (int k = 1; k < nties; ++k)
-      if (comes_first(a, tie[k], win, px, py, pz)) win = tie[k];
-    const ClosestHit h = closest_on_record(a.tris + win, px, py, pz, r.face);
-    r.x = h.x;
-    r.y = h.y;
-    r.z = h.z;
-  }
-  if (!sure) r = ordered_walk(a, px, py, pz);
+  if (!complete || win < 0) r = ordered_walk(a, px, py, pz);
   store_result(a, qi, r);
 }
 
@@ -565,7 +555,7 @@ cudaError_t aabb_query(const AabbDeviceTree& t, const double* P, int64_t np, con
                        cudaStream_t stream) {
   if (np <= 0) return cudaSuccess;
   if (t.depth + 1 > kAabbStack) return cudaErrorInvalidValue;
-  AabbArgs a{t.nodes, t.walk, t.tris, t.face_discs, P, perm, sqrd, index, closest, err, np,
+  AabbArgs a{t.nodes, t.walk, t.spans, t.tris, t.face_discs, P, perm, sqrd, index, closest, err, np,
              t.nnodes, {}, t.scale, t.frame, t.depth};
   for (int k = 0; k < 6; ++k) a.root[k] = t.root[k];
   const int64_t blocks = (np + kAabbThreads - 1) / kAabbThreads;
@@ -581,13 +571,13 @@ cudaError_t aabb_query(const AabbDeviceTree& t, const double* P, int64_t np, con
   return cudaGetLastError();
 }
 
-cudaError_t aabb_discs(const AabbDeviceTree& t, const AabbSpan* spans, const int32_t* big,
-                       int64_t nbig, int32_t* thin, cudaStream_t stream) {
+cudaError_t aabb_discs(const AabbDeviceTree& t, const int32_t* big, int64_t nbig,
+                       int32_t* thin, cudaStream_t stream) {
   if (t.nnodes <= 0) return cudaSuccess;
-  aabb_disc_kernel<<<static_cast<unsigned>(t.nnodes), 32, 0, stream>>>(t.tris, spans, nullptr,
+  aabb_disc_kernel<<<static_cast<unsigned>(t.nnodes), 32, 0, stream>>>(t.tris, t.spans, nullptr,
                                                                        t.frame, t.walk, t.nodes);
   if (nbig > 0)
-    aabb_disc_kernel<<<static_cast<unsigned>(nbig), 512, 0, stream>>>(t.tris, spans, big, t.frame,
+    aabb_disc_kernel<<<static_cast<unsigned>(nbig), 512, 0, stream>>>(t.tris, t.spans, big, t.frame,
                                                                       t.walk, t.nodes);
   aabb_face_disc_kernel<<<static_cast<unsigned>((t.nleaf_faces + 255) / 256), 256, 0, stream>>>(
       t.tris, t.nleaf_faces, t.frame, t.face_discs, thin);

@@ -61,8 +61,8 @@ static_assert(sizeof(AabbWalkRec) == 128, "walk record is one cache line");
 // A node's faces (a run [first, last) of the face records; empty if they are not one
 // run, possible only in a caller-made tree) and where its disc goes: 2 * parent + side,
 // -1 for the root.
-struct AabbSpan {
-  int32_t first, last, slot;
+struct __align__(16) AabbSpan {
+  int32_t first, last, slot, pad;
 };
 
 // Where the discs and FP32 boxes live: x' = (x - c) s with the vertices in [-1, 1]^3, s a
@@ -82,6 +82,7 @@ static_assert(sizeof(AabbTriRec) == 80, "face record is five 16-byte words");
 struct AabbDeviceTree {
   AabbNodeRec* nodes = nullptr;
   AabbWalkRec* walk = nullptr;
+  AabbSpan* spans = nullptr;
   AabbTriRec* tris = nullptr;
   AabbDisc* face_discs = nullptr;  // one per face record
   int64_t nnodes = 0, nleaf_faces = 0;
@@ -110,14 +111,14 @@ cudaError_t aabb_query(const AabbDeviceTree& t, const double* P, int64_t np, con
                        cudaStream_t stream);
 
 // Fills in the discs and slabs of a tree, its nodes' and its faces', whose records are on
-// the device (spans: nnodes, device; big: the nbig nodes of more than kDiscBig faces,
+// the device (big: the nbig nodes of more than kDiscBig faces,
 // device). *thin (device, set to 0 before) receives the number of faces thinner than
 // 1 : 1000: the reference's closest point on such a face may lie off it (the barycentric
 // quotients lose their digits), so no bound holds for it and only the reference's own
 // order says whether it is looked at.
 constexpr int kDiscBig = 256;
-cudaError_t aabb_discs(const AabbDeviceTree& t, const AabbSpan* spans, const int32_t* big,
-                       int64_t nbig, int32_t* thin, cudaStream_t stream);
+cudaError_t aabb_discs(const AabbDeviceTree& t, const int32_t* big, int64_t nbig, int32_t* thin,
+                       cudaStream_t stream);
 
 // s[i] <- sqrt(s[i]), negated where |w[i]| > 1/2 (inside a closed, consistently
 // oriented surface).

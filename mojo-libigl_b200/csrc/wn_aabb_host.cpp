@@ -214,7 +214,7 @@ float round_up(double x) {
 // has one parent.
 bool node_spans(const int64_t* nodes, int64_t nnodes, AabbSpan* span) {
   bool ordered = true;
-  for (int64_t i = 0; i < nnodes; ++i) span[i].slot = -1;
+  for (int64_t i = 0; i < nnodes; ++i) span[i] = AabbSpan{0, 0, -1, 0};
   for (int64_t i = nnodes - 1; i >= 0; --i) {  // children come after their parent
     const int64_t* nd = nodes + 4 * i;
     if (nd[3] > 0) {

@@ -1141,7 +1141,6 @@ int wn_aabb_create(const double* V, int64_t nv, const int64_t* F, int64_t nf,
         if (spans[i].last - spans[i].first > kDiscBig) big.push_back(static_cast<int32_t>(i));
     const int64_t nbig = static_cast<int64_t>(big.size());
     big.push_back(0);  // the count of thin faces
-    AabbSpan* spans_d = nullptr;
     int32_t* big_d = nullptr;
     int32_t thin = 0;
     // On the stream that the disc kernels run on: cudaMemcpy from pageable memory may
@@ -1157,27 +1156,26 @@ int wn_aabb_create(const double* V, int64_t nv, const int64_t* F, int64_t nf,
         (discs &&
          ((e = dev_malloc(&h->t.walk, sizeof(AabbWalkRec) * wrec.size())) != cudaSuccess ||
           (e = dev_malloc(&h->t.face_discs, sizeof(AabbDisc) * trec.size())) != cudaSuccess ||
-          (e = dev_malloc(&spans_d, sizeof(AabbSpan) * spans.size())) != cudaSuccess ||
+          (e = dev_malloc(&h->t.spans, sizeof(AabbSpan) * spans.size())) != cudaSuccess ||
           (e = dev_malloc(&big_d, sizeof(int32_t) * big.size())) != cudaSuccess ||
           (e = upload(h->t.walk, wrec.data(), sizeof(AabbWalkRec) * wrec.size())) !=
               cudaSuccess ||
-          (e = upload(spans_d, spans.data(), sizeof(AabbSpan) * spans.size())) != cudaSuccess ||
+          (e = upload(h->t.spans, spans.data(), sizeof(AabbSpan) * spans.size())) != cudaSuccess ||
           (e = upload(big_d, big.data(), sizeof(int32_t) * big.size())) != cudaSuccess ||
-          (e = aabb_discs(h->t, spans_d, big_d, nbig, big_d + nbig, c->stream)) != cudaSuccess ||
+          (e = aabb_discs(h->t, big_d, nbig, big_d + nbig, c->stream)) != cudaSuccess ||
           (e = cudaMemcpyAsync(&thin, big_d + nbig, sizeof(int32_t), cudaMemcpyDeviceToHost,
                                c->stream)) != cudaSuccess)) ||
         (e = cudaStreamSynchronize(c->stream)) != cudaSuccess) {
       cudaStreamSynchronize(c->stream);  // the host arrays' last readers
-      cudaFree(spans_d);
       cudaFree(big_d);
       cudaFree(h->t.nodes);
       cudaFree(h->t.tris);
       cudaFree(h->t.walk);
+      cudaFree(h->t.spans);
       cudaFree(h->t.face_discs);
       delete h;
       return cuda_fail(e, "device tree upload");
     }
-    cudaFree(spans_d);
     cudaFree(big_d);
     h->t.thin = thin;
     h->t.any_order = regular && thin == 0;
@@ -1196,6 +1194,7 @@ int wn_aabb_destroy(void* tree) {
   cudaFree(h->t.nodes);
   cudaFree(h->t.tris);
   cudaFree(h->t.walk);
+  cudaFree(h->t.spans);
   cudaFree(h->t.face_discs);
   cudaSetDevice(prev);
   delete h;

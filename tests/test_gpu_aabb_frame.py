@@ -91,3 +91,14 @@ def test_thin_faces(level, every):
     V = np.concatenate([V, V[at] + 1e-6])
     _check(V, F, P)
     _check(V + [4.5e5, 5.2e6, 300], F, P + [4.5e5, 5.2e6, 300])
+
+
+@pytest.mark.parametrize("spokes", [9, 40, 2000])
+def test_many_faces_at_one_vertex(spokes):
+    """A fan whose hub is the closest point of most points: every face ties."""
+    a = np.linspace(0, 2 * np.pi, spokes + 1)[:-1]
+    V = np.concatenate([[[0, 0, 1.0]], np.stack([np.cos(a), np.sin(a), 0 * a], 1)])
+    k = np.arange(spokes)
+    F = np.stack([0 * k, 1 + k, 1 + (k + 1) % spokes], 1)
+    P = np.random.default_rng(1).normal(size=(3000, 3)) * 0.3 + [0, 0, 1.5]
+    _check(V, F, np.concatenate([P, V[:50]]))
