@@ -56,6 +56,10 @@ constexpr int kGroup = 16;
 // walk's stack. The library's own trees have at most 30 (2^31 faces); a caller-made one may
 // have 63, and takes the reference's walk, whose stack is in local memory.
 constexpr size_t kStackBytes = 48 << 10;
+// Fewer faces than this are in the reference's order soon enough (1,000 points and 131,072,
+// us, its walk and the any-order one: 12 faces 33 and 36, 141 and 157; 40 around one vertex
+// 46 and 64, 159 and 213; 80 faces 77 and 62, 213 and 193).
+constexpr int64_t kOrderFaces = 64;
 // The reference's walk takes the discs' bounds on meshes of at least kDiscFaces of which one
 // in kDiscShare is thin at most, else the slabs alone (131,072 points, ms, slabs and discs:
 // one thin face in 327,681 3.7 and 2.4, in 20,481 0.96 and 1.00; a tenth of 327,680 10.0 and
@@ -561,7 +565,7 @@ cudaError_t aabb_query(const AabbDeviceTree& t, const double* P, int64_t np, con
   const int64_t blocks = (np + kAabbThreads - 1) / kAabbThreads;
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   const size_t stack_bytes = sizeof(uint2) * kAabbThreads * t.depth;
-  if (t.any_order && t.nnodes > 0 && stack_bytes <= kStackBytes)
+  if (t.any_order && t.nleaf_faces >= kOrderFaces && stack_bytes <= kStackBytes)
     aabb_any_order_kernel<<<static_cast<unsigned>(blocks), kAabbThreads, stack_bytes, stream>>>(a);
   else if (t.nleaf_faces >= kDiscFaces && t.thin <= t.nleaf_faces / kDiscShare)
     aabb_query_kernel<true><<<static_cast<unsigned>(blocks), kAabbThreads, 0, stream>>>(a);

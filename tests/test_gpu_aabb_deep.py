@@ -1,5 +1,5 @@
-"""Caller-made trees deeper than the library's own median split makes (leaves cut off one
-face at a time), up to the deepest that wn_aabb_create accepts: every bit of distance, face
+"""Caller-made trees deeper than the library's own median split makes (leaves cut off a few
+faces at a time), up to the deepest that wn_aabb_create accepts: every bit of distance, face
 and point as the host's walk has it."""
 
 import ctypes
@@ -14,26 +14,30 @@ from igl import _lib, synthetic  # noqa: E402
 pytestmark = pytest.mark.gpu
 
 
-def _chain(V, F):
-    """(boxes, nodes) of the tree whose level k splits off face k: len(F) levels."""
+def _chain(V, F, depth):
+    """(boxes, nodes) of the tree whose level k splits off the next faces: `depth` levels."""
     tri = V[F]
-    n = len(F)
-    boxes, nodes = np.empty((2 * n - 1, 6)), np.empty((2 * n - 1, 4), np.int64)
-    for k in range(n):
-        rest = tri[k:].reshape(-1, 3)
+    each = len(F) // depth
+    boxes, nodes = np.empty((2 * depth - 1, 6)), np.empty((2 * depth - 1, 4), np.int64)
+    for k in range(depth):
+        at = each * k
+        rest = tri[at:].reshape(-1, 3)
         boxes[2 * k] = np.r_[rest.min(0), rest.max(0)]
-        nodes[2 * k] = (2 * k + 1, 2 * k + 2, 0, 0) if k < n - 1 else (-1, -1, k, 1)
-        if k < n - 1:
-            boxes[2 * k + 1] = np.r_[tri[k].min(0), tri[k].max(0)]
-            nodes[2 * k + 1] = (-1, -1, k, 1)
+        if k == depth - 1:
+            nodes[2 * k] = (-1, -1, at, len(F) - at)
+            break
+        part = tri[at:at + each].reshape(-1, 3)
+        nodes[2 * k] = (2 * k + 1, 2 * k + 2, 0, 0)
+        boxes[2 * k + 1] = np.r_[part.min(0), part.max(0)]
+        nodes[2 * k + 1] = (-1, -1, at, each)
     return boxes, nodes
 
 
 @pytest.mark.parametrize("depth", [2, 47, 48, 49, 62, 63])
 def test_depths(depth):
     V, F = synthetic.bumpy_icosphere(2, seed=1)
-    F = np.ascontiguousarray(F[np.argsort(V[F].mean(1)[:, 0])][:depth])
-    boxes, nodes = _chain(V, F)
+    F = np.ascontiguousarray(F[np.argsort(V[F].mean(1)[:, 0])])
+    boxes, nodes = _chain(V, F, depth)
     order = np.arange(len(F))
     P = np.concatenate([V, synthetic.mixed_queries(V, F, 2000, seed=3, near_sigma=1e-2)])
     h, addr = _lib.lib(), _lib.addr

@@ -102,3 +102,11 @@ def test_many_faces_at_one_vertex(spokes):
     F = np.stack([0 * k, 1 + k, 1 + (k + 1) % spokes], 1)
     P = np.random.default_rng(1).normal(size=(3000, 3)) * 0.3 + [0, 0, 1.5]
     _check(V, F, np.concatenate([P, V[:50]]))
+
+
+@pytest.mark.parametrize("faces", [1, 2, 63, 64, 65, 80])
+def test_small_meshes(faces):
+    """On both sides of the size from which the walk has an order of its own."""
+    V, F = synthetic.bumpy_icosphere(1, seed=1)
+    P = np.concatenate([V, synthetic.mixed_queries(V, F, 3000, 5, near_sigma=1e-2)])
+    _check(V, np.ascontiguousarray(F[:faces]), P)
