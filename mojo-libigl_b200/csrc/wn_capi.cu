@@ -144,6 +144,11 @@ struct DeviceCtx {
   cudaEvent_t fork = nullptr, join = nullptr;
 };
 
+// cudaMemcpy from pageable memory and cudaMemset may return before the device has the data,
+// and only the legacy stream is ordered behind them: not the library's own stream, nor a
+// caller's non-blocking one. Waits for them, before a handle or context is used.
+cudaError_t uploads_done() { return cudaStreamSynchronize(cudaStreamLegacy); }
+
 std::mutex g_mutex;
 DeviceCtx g_ctx[kMaxDevices];
 
@@ -164,7 +169,8 @@ DeviceCtx* context(int* code) {
       (!c.err && (e = dev_malloc(&c.err, sizeof(int))) != cudaSuccess) ||
       (e = cudaMemset(c.err, 0, sizeof(int))) != cudaSuccess ||
       (!c.stats && (e = dev_malloc(&c.stats, 2 * sizeof(unsigned long long))) != cudaSuccess) ||
-      (e = cudaMemset(c.stats, 0, 2 * sizeof(unsigned long long))) != cudaSuccess) {
+      (e = cudaMemset(c.stats, 0, 2 * sizeof(unsigned long long))) != cudaSuccess ||
+      (e = uploads_done()) != cudaSuccess) {
     *code = cuda_fail(e, "device context setup");
     return nullptr;
   }
@@ -747,6 +753,7 @@ int wn_mixed_stats(int64_t* refined_pairs, int64_t* careful_visits, int reset) {
   cudaError_t e = cudaDeviceSynchronize();
   if (e == cudaSuccess) e = cudaMemcpy(h, c->stats, sizeof(h), cudaMemcpyDeviceToHost);
   if (e == cudaSuccess && reset) e = cudaMemset(c->stats, 0, sizeof(h));
+  if (e == cudaSuccess) e = uploads_done();
   if (e != cudaSuccess) return cuda_fail(e, "reading mixed-path counters");
   if (refined_pairs) *refined_pairs = static_cast<int64_t>(h[0]);
   if (careful_visits) *careful_visits = static_cast<int64_t>(h[1]);
@@ -973,6 +980,7 @@ int wn_batch_create(int64_t nmesh, const int64_t* nv, const int64_t* nf, const i
   BatchState* b = new BatchState();
   cudaError_t e = batch_create(b, nmesh, nv, nf, nq, faces, plan, c->sms);
   if (e == cudaSuccess) e = batch_edges_create(b, faces);
+  if (e == cudaSuccess) e = uploads_done();
   if (e != cudaSuccess) {
     batch_edges_destroy(b);
     batch_destroy(b);
@@ -1322,7 +1330,8 @@ int fwn_upload(FwnHandle* h) {
         (e = cudaMemcpy(d.moments, h->host.moments, sizeof(FwnMoments) * d.nnodes,
                         cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemcpy(d.tris, h->host.tris, sizeof(AabbTriRec) * h->host.nf,
-                        cudaMemcpyHostToDevice)) != cudaSuccess) {
+                        cudaMemcpyHostToDevice)) != cudaSuccess ||
+        (e = uploads_done()) != cudaSuccess) {
       cudaFree(d.nodes);
       cudaFree(d.moments);
       cudaFree(d.tris);

@@ -29,6 +29,14 @@ def test_tree_uploads_are_ordered_before_its_kernels():
     assert "cudaStreamSynchronize(" in body  # the host arrays end with the call
 
 
+@pytest.mark.parametrize("name", ["context", "wn_mixed_stats", "fwn_upload", "wn_batch_create"])
+def test_other_uploads_are_waited_for(name):
+    with open(os.path.join(CSRC, "wn_capi.cu")) as f:
+        body = _function(f.read(), name)
+    copies = list(re.finditer(r"\bcudaMemcpy\(|\bcudaMemset\(|batch_edges_create\(", body))
+    assert copies and "uploads_done()" in body[copies[-1].end():]
+
+
 @pytest.mark.gpu
 def test_trees_made_one_after_another():
     """Trees with and without thin faces in turn, each checked against the host's walk."""
