@@ -1441,8 +1441,10 @@ __global__ void __launch_bounds__(32 * kWarps, 4) exact_eval_kernel(const EvalAr
        off <= static_cast<double>(bound) + 0.02;
   if (ok)
     a.w[qi] = (near_angle + argument) / kTwoPi + k;
-  else
+  else if (isfinite(qx) && isfinite(qy) && isfinite(qz))
     a.list[atomicAdd(&a.info->nlist, 1)] = qi;
+  else
+    a.w[qi] = NAN;  // as every pair term is
 }
 
 // All pairs for the listed queries, one CTA per query: per-thread running products
