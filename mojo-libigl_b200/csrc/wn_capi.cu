@@ -240,7 +240,7 @@ int forward_fp64_host(const double* tri, const double* q, double* w, int64_t nf,
                                c->stream)) != cudaSuccess)
         return cuda_fail(e, "copy of the inputs");
       ExactBoundary boundary;
-      if ((e = exact_build(xp, tri_d, ld, q_d, c->scratch.ptr, kExactMostFp64, &boundary,
+      if ((e = exact_build(xp, tri_d, ld, q_d, c->scratch.ptr, false, &boundary,
                            c->stream)) != cudaSuccess)
         return cuda_fail(e, "mesh preparation");
       if (boundary.items >= 0) {
@@ -545,8 +545,7 @@ int wn_forward_exact_device(const double* tri, int64_t ld, const double* q, doub
     return WN_OK;  // the caller's all-pairs path needs less memory
   }
   ExactBoundary boundary;
-  e = exact_build(p, tri, ld, q, scratch, mixed ? kExactMostMixed : kExactMostFp64, &boundary,
-                  st);
+  e = exact_build(p, tri, ld, q, scratch, mixed != 0, &boundary, st);
   if (e == cudaSuccess && boundary.items >= 0) e = exact_eval(p, boundary, q, w, scratch, sms, st);
   cudaFreeAsync(scratch, st);
   if (e != cudaSuccess) return cuda_fail(e, "exact winding-number launch");

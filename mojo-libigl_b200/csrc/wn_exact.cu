@@ -1509,6 +1509,21 @@ bool exact_pays(int64_t nf, int64_t nq) {
          static_cast<double>(nf) * static_cast<double>(nq) >= 1.5e8;
 }
 
+// A warp goes over the whole boundary for its queries, which takes about 0.23 us an item
+// however few the warps are: with few queries that, and not the work, is what the boundary
+// costs. 301,466 F with 26,214 holes x 4,096 Q: 7.3 ms against 6.7 (FP64 streaming) and 4.7
+// (mixed), x 8,192 8.5 against 13.4 and 7.7, x 16,384 9.6 against 25 and 11.5; 1,205,862 F
+// with 104,858 holes x 4,096 27 against 25 and 12, x 16,384 38 against 99 and 36; 75,366 F
+// with 6,554 x 4,096 1.9 against 1.6 and 2.6. So it matters to mixed calls, whose own
+// preparation counts too (about 1.5 ms and 5 ns a face).
+bool boundary_pays(int64_t items, int64_t nf, int64_t nq, bool mixed) {
+  const double n = static_cast<double>(items), f = static_cast<double>(nf),
+               q = static_cast<double>(nq);
+  if (!mixed) return n <= kExactMostFp64 * f;
+  return n <= kExactMostMixed * f &&
+         n * (0.23e-6 + 4.8e-12 * q) <= 1.5e-3 + 5e-9 * f + 1.5e-12 * f * q;
+}
+
 ExactPlan plan_exact(int64_t nf, int64_t nq) {
   ExactPlan p;
   p.nf = nf;
@@ -1582,7 +1597,7 @@ T* at(void* scratch, size_t offset) {
 }  // namespace
 
 cudaError_t exact_build(const ExactPlan& p, const double* tri, int64_t ld, const double* q,
-                        void* scratch, double most, ExactBoundary* boundary, cudaStream_t stream) {
+                        void* scratch, bool mixed, ExactBoundary* boundary, cudaStream_t stream) {
   Info* info = at<Info>(scratch, p.info);
   Face64* faces = at<Face64>(scratch, p.faces64);
   uint32_t* partner = at<uint32_t>(scratch, p.partner);
@@ -1636,8 +1651,8 @@ cudaError_t exact_build(const ExactPlan& p, const double* tri, int64_t ld, const
           cudaSuccess ||
       (e = cudaStreamSynchronize(stream)) != cudaSuccess)
     return e;
-  const bool fit = !host.bad && host.nroot <= p.max_roots &&
-                   static_cast<double>(host.nitem) <= most * static_cast<double>(p.nf);
+  const bool fit =
+      !host.bad && host.nroot <= p.max_roots && boundary_pays(host.nitem, p.nf, p.nq, mixed);
   boundary->items = fit ? host.nitem : -1;
   boundary->loops = (host.nroot - host.nitem) / 2;  // a loop of n edges: n - 2 triangles
   if (!fit) return cudaSuccess;

