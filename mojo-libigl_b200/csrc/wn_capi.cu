@@ -220,25 +220,26 @@ int forward_fp64_host(const double* tri, const double* q, double* w, int64_t nf,
   DeviceCtx* c = context(&code);
   if (!c) return code;
   const int64_t ld = even_ld(nf);
+  cudaError_t e;
+  if ((e = c->tri.ensure(sizeof(double) * 9 * ld)) != cudaSuccess ||
+      (e = c->q.ensure(sizeof(double) * 3 * nq)) != cudaSuccess ||
+      (e = c->w.ensure(sizeof(double) * nq)) != cudaSuccess)
+    return cuda_fail(e, "device allocation");
+  double* tri_d = static_cast<double*>(c->tri.ptr);
+  double* q_d = static_cast<double*>(c->q.ptr);
+  double* w_d = static_cast<double*>(c->w.ptr);
+  if (nf > 0 && (e = cudaMemcpy2DAsync(tri_d, sizeof(double) * ld, tri, sizeof(double) * nf,
+                                       sizeof(double) * nf, 9, cudaMemcpyHostToDevice,
+                                       c->stream)) != cudaSuccess)
+    return cuda_fail(e, "copy of the triangle soup");
+  if ((e = cudaMemcpyAsync(q_d, q, sizeof(double) * 3 * nq, cudaMemcpyHostToDevice, c->stream)) !=
+      cudaSuccess)
+    return cuda_fail(e, "copy of the queries");
   if (automatic && exact_pays(nf, nq)) {
     // Its scratch is larger than the all-pairs path's: where it cannot be had, that
     // path serves the call.
     const ExactPlan xp = plan_exact(nf, nq);
-    cudaError_t e;
-    if ((e = c->tri.ensure(sizeof(double) * 9 * ld)) != cudaSuccess ||
-        (e = c->q.ensure(sizeof(double) * 3 * nq)) != cudaSuccess ||
-        (e = c->w.ensure(sizeof(double) * nq)) != cudaSuccess)
-      return cuda_fail(e, "device allocation");
     if (c->scratch.ensure(xp.bytes) == cudaSuccess) {
-      double* w_d = static_cast<double*>(c->w.ptr);
-      const double* q_d = static_cast<const double*>(c->q.ptr);
-      const double* tri_d = static_cast<const double*>(c->tri.ptr);
-      if ((e = cudaMemcpy2DAsync(c->tri.ptr, sizeof(double) * ld, tri, sizeof(double) * nf,
-                                 sizeof(double) * nf, 9, cudaMemcpyHostToDevice, c->stream)) !=
-              cudaSuccess ||
-          (e = cudaMemcpyAsync(c->q.ptr, q, sizeof(double) * 3 * nq, cudaMemcpyHostToDevice,
-                               c->stream)) != cudaSuccess)
-        return cuda_fail(e, "copy of the inputs");
       ExactBoundary boundary;
       if ((e = exact_build(xp, tri_d, ld, q_d, c->scratch.ptr, false, &boundary,
                            c->stream)) != cudaSuccess)
@@ -260,28 +261,13 @@ int forward_fp64_host(const double* tri, const double* q, double* w, int64_t nf,
   size_t scratch = sizeof(double) * (plan.scratch_doubles + 1);
   if (mode == kFp64Tiled)
     scratch = std::max(mixed_sort_scratch_bytes(nf), sizeof(double) * (tplan.scratch_doubles + 1));
-  cudaError_t e;
-  if ((e = c->tri.ensure(sizeof(double) * 9 * ld)) != cudaSuccess ||
-      (e = c->q.ensure(sizeof(double) * 3 * nq)) != cudaSuccess ||
-      (e = c->w.ensure(sizeof(double) * nq)) != cudaSuccess ||
-      (e = c->scratch.ensure(scratch)) != cudaSuccess)
-    return cuda_fail(e, "device allocation");
+  if ((e = c->scratch.ensure(scratch)) != cudaSuccess) return cuda_fail(e, "device allocation");
   if (mode == kFp64Tiled &&
       ((e = c->mesh_tiles.ensure(mixed_tiles_bytes(nf))) != cudaSuccess ||
        (e = c->mesh_tri64.ensure(mixed_tri64_bytes(nf))) != cudaSuccess ||
        (e = c->mesh_face_of.ensure(mixed_face_of_bytes(nf))) != cudaSuccess ||
        (e = c->mesh_reuse.ensure(mixed_reuse_bytes(nf))) != cudaSuccess))
     return cuda_fail(e, "device allocation");
-  double* tri_d = static_cast<double*>(c->tri.ptr);
-  double* q_d = static_cast<double*>(c->q.ptr);
-  double* w_d = static_cast<double*>(c->w.ptr);
-  if (nf > 0 && (e = cudaMemcpy2DAsync(tri_d, sizeof(double) * ld, tri, sizeof(double) * nf,
-                                       sizeof(double) * nf, 9, cudaMemcpyHostToDevice,
-                                       c->stream)) != cudaSuccess)
-    return cuda_fail(e, "copy of the triangle soup");
-  if ((e = cudaMemcpyAsync(q_d, q, sizeof(double) * 3 * nq, cudaMemcpyHostToDevice, c->stream)) !=
-      cudaSuccess)
-    return cuda_fail(e, "copy of the queries");
   if (mode == kFp64Tiled) {
     MixedMesh m;
     m.tiles = static_cast<unsigned char*>(c->mesh_tiles.ptr);

@@ -61,3 +61,11 @@ def test_trees_made_one_after_another():
             for a, b in zip(tree.query(p), expected[i % 2]):
                 assert a.cpu().numpy().tobytes() == np.asarray(b).tobytes()
             tree.close()
+
+
+def test_host_forward_uploads_its_inputs_once():
+    """Also where the path without all pairs declines and an all-pairs kernel runs."""
+    with open(os.path.join(CSRC, "wn_capi.cu")) as f:
+        body = _function(f.read(), "forward_fp64_host")
+    assert len(re.findall(r"cudaMemcpy2DAsync\(", body)) == 1
+    assert len(re.findall(r"cudaMemcpyHostToDevice", body)) == 2  # the soup and the queries
