@@ -204,6 +204,34 @@ int collect_device_error(DeviceCtx* c, cudaStream_t stream) {
 
 int64_t even_ld(int64_t nf) { return ((nf > 0 ? nf : 1) + 1) & ~int64_t(1); }
 
+// W without all pairs; *taken = false, and w untouched, where that does not pay or its
+// scratch cannot be had (an all-pairs kernel needs less). Waits for the stream once.
+cudaError_t exact_forward(const double* tri, int64_t ld, const double* q, double* w, int64_t nf,
+                          int64_t nq, bool mixed, int sms, bool* taken, cudaStream_t stream) {
+  *taken = false;
+  const ExactPlan p = plan_exact(nf, nq);
+  void* scratch = nullptr;
+  if (dev_malloc_async(&scratch, p.bytes, stream) != cudaSuccess) {
+    cudaGetLastError();
+    return cudaSuccess;
+  }
+  ExactBoundary boundary;
+  cudaError_t e = exact_boundary(p, tri, ld, scratch, mixed, &boundary, stream);
+  if (e == cudaSuccess && boundary.items >= 0) {
+    void* edges = nullptr;
+    const size_t bytes = exact_boundary_bytes(boundary);
+    if (bytes && dev_malloc_async(&edges, bytes, stream) != cudaSuccess) {
+      cudaGetLastError();
+    } else {
+      e = exact_eval(p, boundary, q, w, scratch, edges, sms, stream);
+      *taken = e == cudaSuccess;
+    }
+    if (edges) cudaFreeAsync(edges, stream);
+  }
+  cudaFreeAsync(scratch, stream);
+  return e;
+}
+
 int forward_fp64_host(const double* tri, const double* q, double* w, int64_t nf, int64_t nq,
                       int mode) {
   if (nf < 0 || nq < 0) return fail(WN_EINVAL, "negative size (nf=%lld, nq=%lld)",
@@ -236,24 +264,15 @@ int forward_fp64_host(const double* tri, const double* q, double* w, int64_t nf,
       cudaSuccess)
     return cuda_fail(e, "copy of the queries");
   if (automatic && exact_pays(nf, nq)) {
-    // Its scratch is larger than the all-pairs path's: where it cannot be had, that
-    // path serves the call.
-    const ExactPlan xp = plan_exact(nf, nq);
-    if (c->scratch.ensure(xp.bytes) == cudaSuccess) {
-      ExactBoundary boundary;
-      if ((e = exact_build(xp, tri_d, ld, q_d, c->scratch.ptr, false, &boundary,
-                           c->stream)) != cudaSuccess)
-        return cuda_fail(e, "mesh preparation");
-      if (boundary.items >= 0) {
-        if ((e = exact_eval(xp, boundary, q_d, w_d, c->scratch.ptr, c->sms, c->stream)) != cudaSuccess)
-          return cuda_fail(e, "exact winding-number launch");
-        if ((e = cudaMemcpyAsync(w, w_d, sizeof(double) * nq, cudaMemcpyDeviceToHost,
-                                 c->stream)) != cudaSuccess)
-          return cuda_fail(e, "copy of the result");
-        return collect_device_error(c, c->stream);
-      }
-    } else {
-      cudaGetLastError();
+    bool taken = false;
+    if ((e = exact_forward(tri_d, ld, q_d, w_d, nf, nq, false, c->sms, &taken, c->stream)) !=
+        cudaSuccess)
+      return cuda_fail(e, "exact winding-number launch");
+    if (taken) {
+      if ((e = cudaMemcpyAsync(w, w_d, sizeof(double) * nq, cudaMemcpyDeviceToHost, c->stream)) !=
+          cudaSuccess)
+        return cuda_fail(e, "copy of the result");
+      return collect_device_error(c, c->stream);
     }
   }
   const Fp64Plan plan = plan_fp64(nf, nq, c->sms);
@@ -524,18 +543,10 @@ int wn_forward_exact_device(const double* tri, int64_t ld, const double* q, doub
     if (!c) return code;
     sms = c->sms;
   }
-  const ExactPlan p = plan_exact(nf, nq);
-  void* scratch = nullptr;
-  if (dev_malloc_async(&scratch, p.bytes, st) != cudaSuccess) {
-    cudaGetLastError();
-    return WN_OK;  // the caller's all-pairs path needs less memory
-  }
-  ExactBoundary boundary;
-  e = exact_build(p, tri, ld, q, scratch, mixed != 0, &boundary, st);
-  if (e == cudaSuccess && boundary.items >= 0) e = exact_eval(p, boundary, q, w, scratch, sms, st);
-  cudaFreeAsync(scratch, st);
-  if (e != cudaSuccess) return cuda_fail(e, "exact winding-number launch");
-  *taken = boundary.items >= 0 ? 1 : 0;
+  bool done = false;
+  if ((e = exact_forward(tri, ld, q, w, nf, nq, mixed != 0, sms, &done, st)) != cudaSuccess)
+    return cuda_fail(e, "exact winding-number launch");
+  *taken = done ? 1 : 0;
   return WN_OK;
 }
 

@@ -1538,7 +1538,6 @@ ExactPlan plan_exact(int64_t nf, int64_t nq) {
     n = (n + kExactArity - 1) / kExactArity;
   }
   p.nnode = off;
-  p.max_roots = nf;
   uint32_t slots = 1024;
   while (slots < 3 * nf && slots < (1u << 30)) slots <<= 1;
   p.hash_slots = slots;
@@ -1561,10 +1560,6 @@ ExactPlan plan_exact(int64_t nf, int64_t nq) {
   p.eval = take(sizeof(NodeEval) * node);
   p.counts = take(sizeof(Counts) * leaf);
   p.first = take(sizeof(Counts) * leaf);
-  p.groups = take(sizeof(Group) * static_cast<size_t>(p.max_roots + 1));
-  p.roots = take(sizeof(Root) * static_cast<size_t>(p.max_roots + 1));
-  p.root_leaf = take(sizeof(int32_t) * static_cast<size_t>(p.max_roots + 1));
-  p.triangles = take(sizeof(Triangle) * static_cast<size_t>(p.max_roots + 1));
   p.perm = take(sizeof(uint32_t) * q);
   p.list = take(sizeof(uint32_t) * q);
   const size_t m = std::max(f, q);
@@ -1594,17 +1589,43 @@ template <class T>
 T* at(void* scratch, size_t offset) {
   return reinterpret_cast<T*>(static_cast<unsigned char*>(scratch) + offset);
 }
+
+// The boundary's block. Every group is at least one item, and so is every triangle.
+struct Edges {
+  Group* groups;
+  Triangle* triangles;
+  Root* roots;
+  int32_t* leaf;
+  size_t bytes;
+
+  Edges(const ExactBoundary& b, void* block) {
+    const size_t items = static_cast<size_t>(b.items), edges = static_cast<size_t>(b.edges);
+    size_t end = 0;
+    auto take = [&](size_t size) {
+      const size_t here = end;
+      end += (size + 255) & ~size_t(255);
+      return here;
+    };
+    groups = at<Group>(block, take(sizeof(Group) * items));
+    triangles = at<Triangle>(block, take(sizeof(Triangle) * items));
+    roots = at<Root>(block, take(sizeof(Root) * edges));
+    leaf = at<int32_t>(block, take(sizeof(int32_t) * edges));
+    bytes = end;
+  }
+};
 }  // namespace
 
-cudaError_t exact_build(const ExactPlan& p, const double* tri, int64_t ld, const double* q,
-                        void* scratch, bool mixed, ExactBoundary* boundary, cudaStream_t stream) {
+size_t exact_boundary_bytes(const ExactBoundary& boundary) {
+  return boundary.items > 0 ? Edges(boundary, nullptr).bytes : 0;
+}
+
+cudaError_t exact_boundary(const ExactPlan& p, const double* tri, int64_t ld, void* scratch,
+                           bool mixed, ExactBoundary* boundary, cudaStream_t stream) {
   Info* info = at<Info>(scratch, p.info);
   Face64* faces = at<Face64>(scratch, p.faces64);
   uint32_t* partner = at<uint32_t>(scratch, p.partner);
   uint8_t* lead = at<uint8_t>(scratch, p.lead);
-  Moments* moments = at<Moments>(scratch, p.moments);
-  NodeTest* test = at<NodeTest>(scratch, p.test);
-  Counts *counts = at<Counts>(scratch, p.counts), *first = at<Counts>(scratch, p.first);
+  Counts* counts = at<Counts>(scratch, p.counts);
   uint32_t *keys_in = at<uint32_t>(scratch, p.keys_in), *keys_out = at<uint32_t>(scratch, p.keys_out);
   uint32_t *vals_in = at<uint32_t>(scratch, p.vals_in), *vals_out = at<uint32_t>(scratch, p.vals_out);
   uint32_t *heads = at<uint32_t>(scratch, p.heads), *next = at<uint32_t>(scratch, p.next);
@@ -1612,12 +1633,6 @@ cudaError_t exact_build(const ExactPlan& p, const double* tri, int64_t ld, const
   const uint32_t mask = p.hash_slots - 1;
   const int th = 256;
   size_t tb = p.cub_bytes;
-  Levels levels;
-  levels.nlevel = p.nlevel;
-  for (int k = 0; k < kExactMaxLevels; ++k) {
-    levels.off[k] = p.level_off[k];
-    levels.n[k] = p.level_n[k];
-  }
   cudaError_t e;
   exact_init_kernel<<<1, 32, 0, stream>>>(info);
   if ((e = cudaMemsetAsync(heads, 0xff, sizeof(uint32_t) * p.hash_slots, stream)) != cudaSuccess ||
@@ -1651,12 +1666,36 @@ cudaError_t exact_build(const ExactPlan& p, const double* tri, int64_t ld, const
           cudaSuccess ||
       (e = cudaStreamSynchronize(stream)) != cudaSuccess)
     return e;
+  g_launches.fetch_add(9, std::memory_order_relaxed);
   const bool fit =
-      !host.bad && host.nroot <= p.max_roots && boundary_pays(host.nitem, p.nf, p.nq, mixed);
+      !host.bad && host.nroot <= p.nf && boundary_pays(host.nitem, p.nf, p.nq, mixed);
+  boundary->edges = host.nroot;
   boundary->items = fit ? host.nitem : -1;
   boundary->loops = (host.nroot - host.nitem) / 2;  // a loop of n edges: n - 2 triangles
-  if (!fit) return cudaSuccess;
-  tb = p.cub_bytes;
+  return cudaSuccess;
+}
+
+namespace {
+cudaError_t build_tree(const ExactPlan& p, const ExactBoundary& boundary, const Edges& edges,
+                       const double* q, void* scratch, cudaStream_t stream) {
+  Info* info = at<Info>(scratch, p.info);
+  Face64* faces = at<Face64>(scratch, p.faces64);
+  uint8_t* lead = at<uint8_t>(scratch, p.lead);
+  Moments* moments = at<Moments>(scratch, p.moments);
+  NodeTest* test = at<NodeTest>(scratch, p.test);
+  Counts *counts = at<Counts>(scratch, p.counts), *first = at<Counts>(scratch, p.first);
+  uint32_t *keys_in = at<uint32_t>(scratch, p.keys_in), *keys_out = at<uint32_t>(scratch, p.keys_out);
+  uint32_t *vals_in = at<uint32_t>(scratch, p.vals_in), *succ = at<uint32_t>(scratch, p.succ);
+  void* temp = at<unsigned char>(scratch, p.cub);
+  const int th = 256;
+  Levels levels;
+  levels.nlevel = p.nlevel;
+  for (int k = 0; k < kExactMaxLevels; ++k) {
+    levels.off[k] = p.level_off[k];
+    levels.n[k] = p.level_n[k];
+  }
+  cudaError_t e;
+  size_t tb = p.cub_bytes;
   if ((e = cub::DeviceScan::ExclusiveScan(temp, tb, counts, first, AddCounts(), Counts{0, 0, 0},
                                           static_cast<int>(p.nleaf), stream)) != cudaSuccess)
     return e;
@@ -1677,9 +1716,8 @@ cudaError_t exact_build(const ExactPlan& p, const double* tri, int64_t ld, const
   exact_finish_kernel<<<blocks(p.nnode, 64), 64, 0, stream>>>(p.nnode, moments, test,
                                                               at<NodeEval>(scratch, p.eval));
   exact_groups_kernel<<<blocks(3 * p.nf, th), th, 0, stream>>>(
-      faces, 3 * p.nf, p.nleaf, succ, lead, counts, first, p.max_roots, test,
-      at<Group>(scratch, p.groups), at<Root>(scratch, p.roots), at<int32_t>(scratch, p.root_leaf),
-      at<Triangle>(scratch, p.triangles), info);
+      faces, 3 * p.nf, p.nleaf, succ, lead, counts, first, boundary.edges, test, edges.groups,
+      edges.roots, edges.leaf, edges.triangles, info);
   exact_query_box_kernel<<<std::min(blocks(p.nq, th), 592u), th, 0, stream>>>(q, p.nq, info);
   exact_query_keys_kernel<<<blocks(p.nq, th), th, 0, stream>>>(q, p.nq, info, keys_in, vals_in);
   tb = p.cub_bytes;
@@ -1687,11 +1725,10 @@ cudaError_t exact_build(const ExactPlan& p, const double* tri, int64_t ld, const
                                            at<uint32_t>(scratch, p.perm), static_cast<int>(p.nq),
                                            0, 30, stream)) != cudaSuccess)
     return e;
-  g_launches.fetch_add(15, std::memory_order_relaxed);
+  g_launches.fetch_add(6, std::memory_order_relaxed);
   return cudaGetLastError();
 }
 
-namespace {
 template <int SUB>
 void launch_eval(const EvalArgs& a, cudaStream_t stream) {
   const int per_block = kWarps * (32 / SUB);
@@ -1720,17 +1757,20 @@ static int lanes_per_query(const ExactPlan& p, const ExactBoundary& boundary) {
 }
 
 cudaError_t exact_eval(const ExactPlan& p, const ExactBoundary& boundary, const double* q, double* w,
-                       void* scratch, int sms, cudaStream_t stream) {
+                       void* scratch, void* block, int sms, cudaStream_t stream) {
+  const Edges edges(boundary, block);
+  const cudaError_t e = build_tree(p, boundary, edges, q, scratch, stream);
+  if (e != cudaSuccess) return e;
   EvalArgs a;
   a.faces = at<Face64>(scratch, p.faces64);
   a.faces32 = at<Face32>(scratch, p.faces32);
   a.nb = at<int32_t>(scratch, p.nb);
   a.test = at<NodeTest>(scratch, p.test);
   a.eval = at<NodeEval>(scratch, p.eval);
-  a.groups = at<Group>(scratch, p.groups);
-  a.roots = at<Root>(scratch, p.roots);
-  a.root_leaf = at<int32_t>(scratch, p.root_leaf);
-  a.triangles = at<Triangle>(scratch, p.triangles);
+  a.groups = edges.groups;
+  a.roots = edges.roots;
+  a.root_leaf = edges.leaf;
+  a.triangles = edges.triangles;
   a.q = q;
   a.perm = at<uint32_t>(scratch, p.perm);
   a.w = w;

@@ -19,10 +19,8 @@ struct ExactPlan {
   int64_t nleaf = 0, nnode = 0;
   int nlevel = 0;
   int64_t level_off[kExactMaxLevels] = {}, level_n[kExactMaxLevels] = {};
-  int64_t max_roots = 0;   // root edges kept; more than this and the method is not taken
   uint32_t hash_slots = 0;  // a power of two
-  size_t info, faces64, faces32, partner, nb, lead, moments, test, eval, counts, first, groups,
-      roots, root_leaf, triangles;
+  size_t info, faces64, faces32, partner, nb, lead, moments, test, eval, counts, first;
   size_t keys_in, keys_out, vals_in, vals_out, heads, next, pick, succ, perm, list, cub;
   size_t cub_bytes = 0, bytes = 0;
 };
@@ -42,21 +40,25 @@ constexpr double kExactMostFp64 = 0.55, kExactMostMixed = 0.13;
 // Whether a boundary of `items` costs less than all pairs of an FP64 or a mixed call.
 bool boundary_pays(int64_t items, int64_t nf, int64_t nq, bool mixed);
 
-// What the boundary costs a query: triangles and single edges, and the loops that the
-// triangles fan.
+// The mesh's boundary: its edges, the triangles and single edges that stand for them (what
+// it costs a query), and the loops that the triangles fan.
 struct ExactBoundary {
-  int64_t items = -1, loops = 0;
+  int64_t edges = 0, items = -1, loops = 0;
 };
 
-// Pairs the mesh's edges, waits for the stream and reports the boundary; items = -1 if
-// an all-pairs call (FP64, or mixed) costs less than they or the mesh is not fit for the method (nothing
-// further is done then). Else builds the tree and the query order in `scratch`
-// (plan.bytes).
-cudaError_t exact_build(const ExactPlan& p, const double* tri, int64_t ld, const double* q,
-                        void* scratch, bool mixed, ExactBoundary* boundary, cudaStream_t stream);
+// Pairs the mesh's edges in `scratch` (plan.bytes), waits for the stream and reports the
+// boundary; items = -1 if an all-pairs call (FP64, or mixed) costs less than they or the
+// mesh is not fit for the method.
+cudaError_t exact_boundary(const ExactPlan& p, const double* tri, int64_t ld, void* scratch,
+                           bool mixed, ExactBoundary* boundary, cudaStream_t stream);
 
-// W of the queries (in the order given) after exact_build on the same stream.
+// Memory for the boundary itself, known now only: none on a closed mesh, where room for what
+// the method takes at most would be 228 bytes a face.
+size_t exact_boundary_bytes(const ExactBoundary& boundary);
+
+// Builds the tree and the query order in `scratch` and the boundary in `edges`, after
+// exact_boundary, and evaluates W of the queries (in the order given).
 cudaError_t exact_eval(const ExactPlan& p, const ExactBoundary& boundary, const double* q,
-                       double* w, void* scratch, int sms, cudaStream_t stream);
+                       double* w, void* scratch, void* edges, int sms, cudaStream_t stream);
 
 }  // namespace wn
