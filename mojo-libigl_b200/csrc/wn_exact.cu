@@ -323,6 +323,7 @@ __global__ void exact_query_keys_kernel(const double* __restrict__ q, int64_t nq
 
 // ---- edge partners -----------------------------------------------------------
 
+// A. Appleby's 32-bit finaliser (MurmurHash3), a coordinate's halves mixed in between.
 __device__ __forceinline__ uint32_t point_hash(const double* v) {
   uint32_t h = 0x9e3779b9u;
 #pragma unroll
@@ -362,7 +363,7 @@ __global__ void exact_gather_kernel(const double* __restrict__ tri, int64_t ld, 
   const uint32_t h[3] = {point_hash(v), point_hash(v + 3), point_hash(v + 6)};
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    const uint32_t slot = ((h[c] + h[(c + 1) % 3]) * 0x9e3779b1u >> 7) & mask;
+    const uint32_t slot = hash_slot(h[c] + h[(c + 1) % 3], mask);
     const uint32_t e = static_cast<uint32_t>(3 * i + c);
     next[e] = atomicExch(heads + slot, e);
   }
@@ -396,7 +397,7 @@ __global__ void exact_partner_kernel(const Face64* __restrict__ faces, int64_t n
     nb[e] = -1;
     return;
   }
-  const uint32_t head = heads[((point_hash(u) + point_hash(v)) * 0x9e3779b1u >> 7) & mask];
+  const uint32_t head = heads[hash_slot(point_hash(u) + point_hash(v), mask)];
   int rank = 0, nopp = 0, steps = 0;
   uint32_t opp = ~0u;
   for (uint32_t o = head; o != ~0u && steps <= kChain; o = next[o], ++steps) {
@@ -441,7 +442,7 @@ struct AddCounts {
 };
 
 __device__ __forceinline__ uint32_t point_slot(const double* v, uint32_t mask) {
-  return (point_hash(v) * 0x9e3779b1u >> 7) & mask;
+  return hash_slot(point_hash(v), mask);
 }
 
 // Root edges into the chains of their first points.

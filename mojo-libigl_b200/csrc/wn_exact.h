@@ -25,6 +25,17 @@ struct ExactPlan {
   size_t cub_bytes = 0, bytes = 0;
 };
 
+// Slot of a 32-bit hash in a table of mask + 1 <= 2^32 slots: the high half of its product
+// with 2^64 / golden ratio (D. Knuth, TAOCP vol. 3, 6.4), every bit of which depends on the
+// hash. A 32-bit product left 25 bits, so tables of more slots (above 11 million faces) had
+// chains as long as one of 2^25 has.
+#if defined(__CUDACC__)
+__host__ __device__
+#endif
+inline uint32_t hash_slot(uint32_t h, uint32_t mask) {
+  return static_cast<uint32_t>(h * 0x9e3779b97f4a7c15ull >> 32) & mask;
+}
+
 // Whether a call of this size should take the method (the mesh's edges still decide).
 bool exact_pays(int64_t nf, int64_t nq);
 
