@@ -141,11 +141,12 @@ int wn_forward_fp64_device(const double* tri, int64_t ld, const double* q, doubl
  * far faces through their boundary edges (FP64) and an integer whose approximation carries
  * an error bound. Within rounding of wn_forward_fp64_device (<= 1e-12). *taken = 1 when w
  * holds the result; *taken = 0 (status WN_OK, w untouched) when the call is too small, the
- * stream is being captured, the faces do not share enough edges for it to pay, a coordinate
- * is not finite or beyond 1e75, or its scratch (about 320 bytes per face, up to 340 per
+ * stream is being captured, the faces do not share enough edges for it to pay, the mesh is
+ * dense (surface all around) or crowded into a small part of its extent, a coordinate is not
+ * finite or beyond 1e75, or its scratch (about 320 bytes per face, up to 340 per
  * triangle or edge of the boundary, 24 per query) could not be allocated: then use one of the
  * all-pairs entry points; mixed = 1 says that this would be a mixed-precision one, which is
- * harder to beat. Waits for the stream once. Device pointers; tri: 9 rows with row stride ld
+ * harder to beat (on dense meshes the FP64 pairs are done here then). Waits for the stream once. Device pointers; tri: 9 rows with row stride ld
  * doubles. */
 int wn_exact_pays(int64_t nf, int64_t nq); /* 1: the sizes are worth the call */
 int wn_forward_exact_device(const double* tri, int64_t ld, const double* q, double* w, int64_t nf,

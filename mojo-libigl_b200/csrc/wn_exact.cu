@@ -40,8 +40,9 @@
 // Edges cancel by position: two directed sides with bitwise equal endpoints in
 // opposite directions are partners, whatever their indices, so triangle soups
 // whose faces meet work like meshes, and any input is correct: an unpaired side
-// is simply a root edge. Where too many are left the method does not pay
-// (kExactMost*), and an all-pairs kernel does the call.
+// is simply a root edge. Where too many are left (kExactMost*, boundary_pays), or the
+// mesh is dense or crowded (kMostDense, kMostCrowded*), the method does not pay and an
+// all-pairs kernel does the call.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -70,6 +71,22 @@ constexpr int kMinExp = (1023 - 7) << 20;  // |z_e| >= ~2^-7, else try another d
 constexpr int kChain = 64;           // longest hash chain that is searched for partners
 constexpr int kMaxLoop = 8;          // boundary loops of at most this many edges become fans
 constexpr double kFarQuery = 1e9;    // queries beyond this many extents: all pairs
+// Meshes that the method is the slower one for, whatever their edges:
+// Dense ones: the area in a face's coarse cell, in faces of the cell, in the mean over the
+// faces. Every query then has surface all around it: expansions are far only under strict
+// opening rules, and the second and later walks of exact_eval_kernel cost more than the
+// pairs. 65,536 Q, ms, this and the FP64 streaming kernel: 128 concentric spheres (9.9) 52
+// and 52 (16,384 Q), 256 (25) 144 and 105; 10,000 spheres of radius 0.1 in a cube of side 2
+// (8.9) 52 and 64, 0.15 (18.8) 89 and 64, 0.2 (33) 170 and 64; the tetrahedra of a grid of
+// 12^3 (11.8) 19 and 13, 16^3 (10.9) 25 and 32, 24^3 (12.3) 104 and 106, 32^3 (14.5) 101 and
+// 62 (16,384 Q); 20,000 tetrahedra of side 0.1 (15.8) 44 and 26.
+constexpr double kMostDense = 11.5;
+// Crowded ones: faces that share a cell of the order with this share of all faces, in the
+// mean (a triangle 1,000 times the rest's size away, or a part of 1 : 1,000). Within a cell
+// the order is the input's, and every leaf is near: an outlier at 10^6 61 ms, 26 (FP64
+// streaming) and 13 (mixed); at 10^3 (0.12) 40, 26 and 12; a ball of 1 : 1,000 beside a ground
+// of its own, half of the queries near either (0.11) 12, 28 and 12.
+constexpr double kMostCrowdedFp64 = 0.5, kMostCrowdedMixed = 0.02;
 
 struct Info {
   unsigned long long lo[3], hi[3];    // vertex box, ordered keys
@@ -78,7 +95,14 @@ struct Info {
   int32_t nroot, nitem, ngroup;       // root edges, the triangles and single edges that
                                       // stand for them, the groups they form
   int32_t nlist;                      // queries left to exact_fallback_kernel
+  unsigned long long crowd;           // sum over the order's cells of their faces, squared
+  unsigned long long density;         // sum over the faces of their coarse cells' area, in faces
+                                      // of a cell (2^-16)
 };
+
+// Coarse cells, 32 to an axis: the upper half of the order's key.
+constexpr int kCoarseShift = 15, kCoarse = 1 << 15;
+constexpr double kCoarseUnit = 1 << 16;
 
 // 80-byte face: corners A, B, C (FP64), in sorted order.
 struct Face64 {
@@ -165,7 +189,10 @@ __global__ void exact_init_kernel(Info* info) {
     info->lo[t] = info->qlo[t] = ~0ull;
     info->hi[t] = info->qhi[t] = 0ull;
   }
-  if (t == 0) info->bad = info->nroot = info->nitem = info->ngroup = info->nlist = 0;
+  if (t == 0) {
+    info->bad = info->nroot = info->nitem = info->ngroup = info->nlist = 0;
+    info->crowd = info->density = 0;
+  }
 }
 
 // Block-wide min/max of three coordinates into ordered keys: one atomic per block
@@ -290,18 +317,32 @@ __device__ __forceinline__ uint32_t cell_key(const double p[3], const double lo[
 
 __global__ void exact_face_keys_kernel(const double* __restrict__ tri, int64_t ld, int64_t nf,
                                        const Info* __restrict__ info, uint32_t* keys,
-                                       uint32_t* vals) {
+                                       uint32_t* vals, unsigned long long* coarse) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= nf) return;
-  double p[3], lo[3], hi[3];
+  double p[3], lo[3], hi[3], u[3], v[3];
+  double ext = 0.0;
 #pragma unroll
   for (int x = 0; x < 3; ++x) {
-    p[x] = (tri[x * ld + i] + tri[(3 + x) * ld + i] + tri[(6 + x) * ld + i]) * (1.0 / 3.0);
+    const double a = tri[x * ld + i], b = tri[(3 + x) * ld + i], c = tri[(6 + x) * ld + i];
+    p[x] = (a + b + c) * (1.0 / 3.0);
+    u[x] = b - a;
+    v[x] = c - a;
     lo[x] = okey_inv(info->lo[x]);
     hi[x] = okey_inv(info->hi[x]);
+    ext = fmax(ext, hi[x] - lo[x]);
   }
-  keys[i] = cell_key(p, lo, hi);
+  const uint32_t key = cell_key(p, lo, hi);
+  keys[i] = key;
   vals[i] = static_cast<uint32_t>(i);
+  const double s = ext > 0.0 ? 32.0 / ext : 0.0;  // sides in cells
+  const double nx = (u[1] * s) * (v[2] * s) - (u[2] * s) * (v[1] * s),
+               ny = (u[2] * s) * (v[0] * s) - (u[0] * s) * (v[2] * s),
+               nz = (u[0] * s) * (v[1] * s) - (u[1] * s) * (v[0] * s);
+  const double area = 0.5 * sqrt(nx * nx + ny * ny + nz * nz);
+  // In whole units: the sum is the same in any order.
+  atomicAdd(coarse + (key >> kCoarseShift),
+            static_cast<unsigned long long>(fmin(area, 4096.0) * kCoarseUnit + 0.5));
 }
 
 __global__ void exact_query_keys_kernel(const double* __restrict__ q, int64_t nq,
@@ -345,14 +386,38 @@ __device__ __forceinline__ const double* corner_of(const Face64* faces, uint32_t
   return faces[edge / 3u].v + 3 * c;
 }
 
+constexpr int kGatherThreads = 128;
 // Sorted faces as 80-byte records; every side enters the chain of its hash slot
 // (side e = 3 * sorted face + corner, from that corner to the next).
 __global__ void exact_gather_kernel(const double* __restrict__ tri, int64_t ld, int64_t nf,
-                                    const uint32_t* __restrict__ order, Face64* faces,
-                                    uint32_t* heads, uint32_t mask, uint32_t* next) {
+                                    const uint32_t* __restrict__ order,
+                                    const uint32_t* __restrict__ keys,
+                                    const unsigned long long* __restrict__ coarse, Face64* faces,
+                                    uint32_t* heads, uint32_t mask, uint32_t* next, Info* info) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  unsigned long long around = i < nf ? coarse[keys[i] >> kCoarseShift] : 0;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) around += __shfl_xor_sync(~0u, around, o);
+  __shared__ unsigned long long part[kGatherThreads / 32];
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = around;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < kGatherThreads / 32; ++k) around += part[k];
+    atomicAdd(&info->density, around);
+  }
   if (i >= nf) return;
   const uint32_t f = order[i];
+  // The first face of a cell that holds more than 64.
+  const uint32_t key = keys[i];
+  if (i + 64 < nf && keys[i + 64] == key && (i == 0 || keys[i - 1] != key)) {
+    int64_t lo = i + 64, hi = nf;  // key at lo; not at hi
+    while (hi - lo > 1) {
+      const int64_t mid = lo + (hi - lo) / 2;
+      if (keys[mid] == key) lo = mid; else hi = mid;
+    }
+    const unsigned long long n = static_cast<unsigned long long>(hi - i);
+    atomicAdd(&info->crowd, n * n);
+  }
   double v[10];
 #pragma unroll
   for (int r = 0; r < 9; ++r) v[r] = tri[r * ld + f];
@@ -1559,7 +1624,8 @@ ExactPlan plan_exact(int64_t nf, int64_t nq) {
   p.moments = take(sizeof(Moments) * node);
   p.test = take(sizeof(NodeTest) * node);
   p.eval = take(sizeof(NodeEval) * node);
-  p.counts = take(sizeof(Counts) * leaf);
+  p.counts = take(sizeof(Counts) * leaf);  // set to 0 together with the next
+  p.coarse = take(sizeof(unsigned long long) * kCoarse);
   p.first = take(sizeof(Counts) * leaf);
   p.perm = take(sizeof(uint32_t) * q);
   p.list = take(sizeof(uint32_t) * q);
@@ -1627,6 +1693,7 @@ cudaError_t exact_boundary(const ExactPlan& p, const double* tri, int64_t ld, vo
   uint32_t* partner = at<uint32_t>(scratch, p.partner);
   uint8_t* lead = at<uint8_t>(scratch, p.lead);
   Counts* counts = at<Counts>(scratch, p.counts);
+  unsigned long long* coarse = at<unsigned long long>(scratch, p.coarse);
   uint32_t *keys_in = at<uint32_t>(scratch, p.keys_in), *keys_out = at<uint32_t>(scratch, p.keys_out);
   uint32_t *vals_in = at<uint32_t>(scratch, p.vals_in), *vals_out = at<uint32_t>(scratch, p.vals_out);
   uint32_t *heads = at<uint32_t>(scratch, p.heads), *next = at<uint32_t>(scratch, p.next);
@@ -1637,16 +1704,17 @@ cudaError_t exact_boundary(const ExactPlan& p, const double* tri, int64_t ld, vo
   cudaError_t e;
   exact_init_kernel<<<1, 32, 0, stream>>>(info);
   if ((e = cudaMemsetAsync(heads, 0xff, sizeof(uint32_t) * p.hash_slots, stream)) != cudaSuccess ||
-      (e = cudaMemsetAsync(counts, 0, sizeof(Counts) * p.nleaf, stream)) != cudaSuccess)
+      (e = cudaMemsetAsync(counts, 0, p.coarse - p.counts + sizeof(unsigned long long) * kCoarse,
+                           stream)) != cudaSuccess)
     return e;
   exact_face_box_kernel<<<std::min(blocks(p.nf, th), 592u), th, 0, stream>>>(tri, ld, p.nf, info);
   exact_face_keys_kernel<<<blocks(p.nf, th), th, 0, stream>>>(tri, ld, p.nf, info, keys_in,
-                                                              vals_in);
+                                                              vals_in, coarse);
   if ((e = cub::DeviceRadixSort::SortPairs(temp, tb, keys_in, keys_out, vals_in, vals_out,
                                            static_cast<int>(p.nf), 0, 30, stream)) != cudaSuccess)
     return e;
-  exact_gather_kernel<<<blocks(p.nf, 128), 128, 0, stream>>>(tri, ld, p.nf, vals_out, faces, heads,
-                                                             mask, next);
+  exact_gather_kernel<<<blocks(p.nf, kGatherThreads), kGatherThreads, 0, stream>>>(
+      tri, ld, p.nf, vals_out, keys_out, coarse, faces, heads, mask, next, info);
   exact_partner_kernel<<<blocks(3 * p.nf, th), th, 0, stream>>>(
       faces, 3 * p.nf, heads, mask, next, partner, at<int32_t>(scratch, p.nb));
   uint32_t *pick = at<uint32_t>(scratch, p.pick), *succ = at<uint32_t>(scratch, p.succ);
@@ -1668,8 +1736,13 @@ cudaError_t exact_boundary(const ExactPlan& p, const double* tri, int64_t ld, vo
       (e = cudaStreamSynchronize(stream)) != cudaSuccess)
     return e;
   g_launches.fetch_add(9, std::memory_order_relaxed);
-  const bool fit =
-      !host.bad && host.nroot <= p.nf && boundary_pays(host.nitem, p.nf, p.nq, mixed);
+  const double nf = static_cast<double>(p.nf);
+  const bool dense = static_cast<double>(host.density) > kMostDense * kCoarseUnit * nf;
+  const bool crowded = static_cast<double>(host.crowd) >
+                       (mixed ? kMostCrowdedMixed : kMostCrowdedFp64) * nf * nf;
+  const bool fit = !host.bad && !dense && !crowded && host.nroot <= p.nf &&
+                   boundary_pays(host.nitem, p.nf, p.nq, mixed);
+  boundary->dense = dense && !host.bad;
   boundary->edges = host.nroot;
   boundary->items = fit ? host.nitem : -1;
   boundary->loops = (host.nroot - host.nitem) / 2;  // a loop of n edges: n - 2 triangles

@@ -21,7 +21,7 @@ struct ExactPlan {
   int64_t level_off[kExactMaxLevels] = {}, level_n[kExactMaxLevels] = {};
   uint32_t hash_slots = 0;  // a power of two
   size_t info, faces64, faces32, partner, nb, lead, moments, test, eval, counts, first;
-  size_t keys_in, keys_out, vals_in, vals_out, heads, next, pick, succ, perm, list, cub;
+  size_t keys_in, keys_out, vals_in, vals_out, coarse, heads, next, pick, succ, perm, list, cub;
   size_t cub_bytes = 0, bytes = 0;
 };
 
@@ -55,6 +55,7 @@ bool boundary_pays(int64_t items, int64_t nf, int64_t nq, bool mixed);
 // it costs a query), and the loops that the triangles fan.
 struct ExactBoundary {
   int64_t edges = 0, items = -1, loops = 0;
+  bool dense = false;  // surface all around: FP64 pairs cost less than mixed ones, too
 };
 
 // Pairs the mesh's edges in `scratch` (plan.bytes), waits for the stream and reports the

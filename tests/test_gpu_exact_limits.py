@@ -98,3 +98,38 @@ print(nf, free - torch.cuda.mem_get_info()[0])
     assert out.returncode == 0, out.stderr
     nf, used = (int(x) for x in out.stdout.split())
     assert used <= 400 * nf
+
+
+def _spheres(n, radius):
+    v, f = synthetic.icosahedron()
+    c = np.random.default_rng(3).uniform(-1, 1, (n, 1, 3))
+    return ((c + radius * v).reshape(-1, 3),
+            (np.arange(n)[:, None, None] * len(v) + f).reshape(-1, 3))
+
+
+def _with_outlier(V, F, away):
+    return (np.concatenate([V, V[:3] + away]),
+            np.concatenate([F, [[len(V), len(V) + 1, len(V) + 2]]]))
+
+
+@pytest.mark.parametrize("mesh, fp64, mixed", [
+    ("dense", None, True), ("sparse", True, True), ("outlier", False, False),
+    ("near outlier", True, True)])
+def test_meshes_that_all_pairs_suit_better(mesh, fp64, mixed):
+    """Surface all around every query (52,800 faces of overlapping spheres; a mixed call is
+    done by FP64 pairs then), and one triangle so far away that the others share a cell."""
+    if mesh in ("dense", "sparse"):
+        V, F = _spheres(3000, 0.3 if mesh == "dense" else 0.03)
+        O = synthetic.box_points(V, 30000, seed=1)
+    else:
+        V, F = synthetic.bumpy_icosphere(5, seed=1)
+        O = synthetic.mixed_queries(V, F, 30000, seed=2)
+        V, F = _with_outlier(V, F, 1e7 if mesh == "outlier" else 30.0)
+    Vt, Ft, Ot = _tensors(V, F, O)
+    tri, ld, nf = wa.triangle_soa(Vt, Ft)
+    ref = wa.forward_fp64(tri, ld, nf, Ot)
+    for taken, is_mixed in ((fp64, False), (mixed, True)):
+        w = wa.forward_exact(tri, ld, nf, Ot, mixed=is_mixed)
+        assert (w is not None) == bool(taken)
+        if w is not None:
+            assert float((w - ref).abs().max()) <= 1e-12
