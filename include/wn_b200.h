@@ -146,7 +146,7 @@ int wn_forward_fp64_device(const double* tri, int64_t ld, const double* q, doubl
  * finite or beyond 1e75, or its scratch (about 320 bytes per face, up to 340 per
  * triangle or edge of the boundary, 24 per query) could not be allocated: then use one of the
  * all-pairs entry points; mixed = 1 says that this would be a mixed-precision one, which is
- * harder to beat (on dense meshes the FP64 pairs are done here then). Waits for the stream once. Device pointers; tri: 9 rows with row stride ld
+ * harder to beat (where FP64 pairs cost less, they are done here then). Waits for the stream once. Device pointers; tri: 9 rows with row stride ld
  * doubles. */
 int wn_exact_pays(int64_t nf, int64_t nq); /* 1: the sizes are worth the call */
 int wn_forward_exact_device(const double* tri, int64_t ld, const double* q, double* w, int64_t nf,

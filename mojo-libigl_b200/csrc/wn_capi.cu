@@ -205,7 +205,8 @@ int collect_device_error(DeviceCtx* c, cudaStream_t stream) {
 int64_t even_ld(int64_t nf) { return ((nf > 0 ? nf : 1) + 1) & ~int64_t(1); }
 
 // W without all pairs; *taken = false, and w untouched, where that does not pay or its
-// scratch cannot be had (an all-pairs kernel needs less). Waits for the stream once.
+// scratch cannot be had (an all-pairs kernel needs less). A mixed call is done by the FP64
+// all-pairs kernel where that is the cheaper one. Waits for the stream once.
 cudaError_t exact_forward(const double* tri, int64_t ld, const double* q, double* w, int64_t nf,
                           int64_t nq, bool mixed, int sms, int* err, bool* taken,
                           cudaStream_t stream) {
@@ -228,12 +229,13 @@ cudaError_t exact_forward(const double* tri, int64_t ld, const double* q, double
       *taken = e == cudaSuccess;
     }
     if (edges) cudaFreeAsync(edges, stream);
-  } else if (e == cudaSuccess && mixed && boundary.dense && !(ld & 1) &&
-             !(reinterpret_cast<uintptr_t>(tri) & 15)) {
-    // Most pairs of such a mesh are near ones, which the mixed kernel refines in FP64 after it
-    // has done them in FP32 (65,536 Q, ms, FP64 streaming and mixed: 10,000 spheres of radius
-    // 0.2 in a cube of side 2 64 and 83, 20,000 tetrahedra of side 0.1 26 and 48, of 0.3 30
-    // and 61; at the worst 256 concentric spheres 105 and 97).
+  } else if (e == cudaSuccess && mixed && !(ld & 1) && !(reinterpret_cast<uintptr_t>(tri) & 15) &&
+             (boundary.dense || fp64_pairs_seconds(nf, nq) <= mixed_pairs_seconds(nf, nq))) {
+    // All pairs in FP64 are the cheaper ones: few pairs, beside which the mixed kernel's
+    // preparation is large, or a dense mesh, where most pairs are near ones, which the mixed
+    // kernel refines in FP64 after it has done them in FP32 (65,536 Q, ms, FP64 and mixed:
+    // 10,000 spheres of radius 0.2 in a cube of side 2 64 and 83, 20,000 tetrahedra of side 0.1
+    // 26 and 48, of 0.3 30 and 61; at the worst 256 concentric spheres 105 and 97).
     const Fp64Plan plan = plan_fp64(nf, nq, sms);
     void* partial = nullptr;
     if (dev_malloc_async(&partial, sizeof(double) * (plan.scratch_doubles + 1), stream) !=

@@ -92,6 +92,7 @@ struct Info {
   unsigned long long lo[3], hi[3];    // vertex box, ordered keys
   unsigned long long qlo[3], qhi[3];  // box of the queries clamped to twice the mesh's
   int32_t bad;                        // a vertex is not finite
+  int32_t nopen;                      // sides without a partner
   int32_t nroot, nitem, ngroup;       // root edges, the triangles and single edges that
                                       // stand for them, the groups they form
   int32_t nlist;                      // queries left to exact_fallback_kernel
@@ -190,7 +191,7 @@ __global__ void exact_init_kernel(Info* info) {
     info->hi[t] = info->qhi[t] = 0ull;
   }
   if (t == 0) {
-    info->bad = info->nroot = info->nitem = info->ngroup = info->nlist = 0;
+    info->bad = info->nopen = info->nroot = info->nitem = info->ngroup = info->nlist = 0;
     info->crowd = info->density = 0;
   }
 }
@@ -441,13 +442,12 @@ __global__ void exact_gather_kernel(const double* __restrict__ tri, int64_t ld, 
 // than kChain stay unpaired, all of them alike: still a valid boundary.
 constexpr uint32_t kNoPartner = ~0u, kNoLength = ~1u;
 
-__global__ void exact_partner_kernel(const Face64* __restrict__ faces, int64_t nedge,
-                                     const uint32_t* __restrict__ heads, uint32_t mask,
-                                     const uint32_t* __restrict__ next,
-                                     uint32_t* __restrict__ partner, int32_t* __restrict__ nb) {
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= nedge) return;
-  const uint32_t e = static_cast<uint32_t>(i);
+// True if side e stays unpaired.
+__device__ __forceinline__ bool pair_side(const Face64* __restrict__ faces, uint32_t e,
+                                          const uint32_t* __restrict__ heads, uint32_t mask,
+                                          const uint32_t* __restrict__ next,
+                                          uint32_t* __restrict__ partner,
+                                          int32_t* __restrict__ nb) {
   double u[3], v[3];
   {
     const double *pu = corner_of(faces, e, 0), *pv = corner_of(faces, e, 1);
@@ -460,7 +460,7 @@ __global__ void exact_partner_kernel(const Face64* __restrict__ faces, int64_t n
   if (same_point(u, v)) {
     partner[e] = kNoLength;
     nb[e] = -1;
-    return;
+    return false;
   }
   const uint32_t head = heads[hash_slot(point_hash(u) + point_hash(v), mask)];
   int rank = 0, nopp = 0, steps = 0;
@@ -494,6 +494,19 @@ __global__ void exact_partner_kernel(const Face64* __restrict__ faces, int64_t n
   const uint32_t leaf = e / kLeafEdges, other = opp / kLeafEdges;
   partner[e] = rank < nopp ? opp : kNoPartner;
   nb[e] = rank < nopp && other != leaf ? static_cast<int32_t>(other) : -1;
+  return rank >= nopp;
+}
+
+__global__ void exact_partner_kernel(const Face64* __restrict__ faces, int64_t nedge,
+                                     const uint32_t* __restrict__ heads, uint32_t mask,
+                                     const uint32_t* __restrict__ next,
+                                     uint32_t* __restrict__ partner, int32_t* __restrict__ nb,
+                                     Info* info) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const bool open = i < nedge && pair_side(faces, static_cast<uint32_t>(i), heads, mask, next,
+                                           partner, nb);
+  const int n = __syncthreads_count(open);
+  if (threadIdx.x == 0 && n) atomicAdd(&info->nopen, n);
 }
 
 // What a leaf's sides lead, and (exclusive sums) what comes before it.
@@ -510,12 +523,19 @@ __device__ __forceinline__ uint32_t point_slot(const double* v, uint32_t mask) {
   return hash_slot(point_hash(v), mask);
 }
 
+// More sides without a partner than faces: the method is not taken (exact_boundary), and the
+// kernels that look for loops leave at once.
+__device__ __forceinline__ bool too_open(const Info* info, int64_t nedge) {
+  return 3ll * info->nopen > nedge;
+}
+
 // Root edges into the chains of their first points.
 __global__ void exact_root_hash_kernel(const Face64* __restrict__ faces, int64_t nedge,
                                        const uint32_t* __restrict__ partner, uint32_t* heads,
-                                       uint32_t mask, uint32_t* next) {
+                                       uint32_t mask, uint32_t* next,
+                                       const Info* __restrict__ info) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= nedge || partner[i] != kNoPartner) return;
+  if (too_open(info, nedge) || i >= nedge || partner[i] != kNoPartner) return;
   const uint32_t e = static_cast<uint32_t>(i);
   next[e] = atomicExch(heads + point_slot(corner_of(faces, e, 0), mask), e);
 }
@@ -538,9 +558,10 @@ __device__ __forceinline__ bool each_root(const Face64* faces, const uint32_t* h
 __global__ void exact_pick_kernel(const Face64* __restrict__ faces, int64_t nedge,
                                   const uint32_t* __restrict__ partner,
                                   const uint32_t* __restrict__ heads, uint32_t mask,
-                                  const uint32_t* __restrict__ next, uint32_t* __restrict__ pick) {
+                                  const uint32_t* __restrict__ next, uint32_t* __restrict__ pick,
+                                  const Info* __restrict__ info) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= nedge || partner[i] != kNoPartner) return;
+  if (too_open(info, nedge) || i >= nedge || partner[i] != kNoPartner) return;
   const uint32_t e = static_cast<uint32_t>(i);
   const double *u = corner_of(faces, e, 0), *v = corner_of(faces, e, 1);
   uint32_t best = ~0u;
@@ -578,9 +599,10 @@ __global__ void exact_successor_kernel(const Face64* __restrict__ faces, int64_t
                                        const uint32_t* __restrict__ heads, uint32_t mask,
                                        const uint32_t* __restrict__ next,
                                        const uint32_t* __restrict__ pick,
-                                       uint32_t* __restrict__ succ) {
+                                       uint32_t* __restrict__ succ,
+                                       const Info* __restrict__ info) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= nedge || partner[i] != kNoPartner) return;
+  if (too_open(info, nedge) || i >= nedge || partner[i] != kNoPartner) return;
   const uint32_t e = static_cast<uint32_t>(i);
   uint32_t s = ~0u;
   if (picked(pick, e)) {
@@ -606,6 +628,7 @@ __global__ void exact_loops_kernel(const uint32_t* __restrict__ partner,
                                    const uint32_t* __restrict__ succ, int64_t nedge,
                                    uint8_t* __restrict__ lead,
                                    Counts* __restrict__ counts, Info* info) {
+  if (too_open(info, nedge)) return;
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const uint32_t e = static_cast<uint32_t>(i);
   int count = 0;
@@ -1580,14 +1603,13 @@ bool exact_pays(int64_t nf, int64_t nq) {
 // costs. 301,466 F with 26,214 holes x 4,096 Q: 7.3 ms against 6.7 (FP64 streaming) and 4.7
 // (mixed), x 8,192 8.5 against 13.4 and 7.7, x 16,384 9.6 against 25 and 11.5; 1,205,862 F
 // with 104,858 holes x 4,096 27 against 25 and 12, x 16,384 38 against 99 and 36; 75,366 F
-// with 6,554 x 4,096 1.9 against 1.6 and 2.6. So it matters to mixed calls, whose own
-// preparation counts too (about 1.5 ms and 5 ns a face).
+// with 6,554 x 4,096 1.9 against 1.6 and 2.6. So it matters to mixed calls.
 bool boundary_pays(int64_t items, int64_t nf, int64_t nq, bool mixed) {
   const double n = static_cast<double>(items), f = static_cast<double>(nf),
                q = static_cast<double>(nq);
   if (!mixed) return n <= kExactMostFp64 * f;
   return n <= kExactMostMixed * f &&
-         n * (0.23e-6 + 4.8e-12 * q) <= 1.5e-3 + 5e-9 * f + 1.5e-12 * f * q;
+         n * (0.23e-6 + 4.8e-12 * q) <= mixed_pairs_seconds(nf, nq);
 }
 
 ExactPlan plan_exact(int64_t nf, int64_t nq) {
@@ -1716,16 +1738,16 @@ cudaError_t exact_boundary(const ExactPlan& p, const double* tri, int64_t ld, vo
   exact_gather_kernel<<<blocks(p.nf, kGatherThreads), kGatherThreads, 0, stream>>>(
       tri, ld, p.nf, vals_out, keys_out, coarse, faces, heads, mask, next, info);
   exact_partner_kernel<<<blocks(3 * p.nf, th), th, 0, stream>>>(
-      faces, 3 * p.nf, heads, mask, next, partner, at<int32_t>(scratch, p.nb));
+      faces, 3 * p.nf, heads, mask, next, partner, at<int32_t>(scratch, p.nb), info);
   uint32_t *pick = at<uint32_t>(scratch, p.pick), *succ = at<uint32_t>(scratch, p.succ);
   if ((e = cudaMemsetAsync(heads, 0xff, sizeof(uint32_t) * p.hash_slots, stream)) != cudaSuccess)
     return e;
   exact_root_hash_kernel<<<blocks(3 * p.nf, th), th, 0, stream>>>(faces, 3 * p.nf, partner, heads,
-                                                                  mask, next);
+                                                                  mask, next, info);
   exact_pick_kernel<<<blocks(3 * p.nf, th), th, 0, stream>>>(faces, 3 * p.nf, partner, heads, mask,
-                                                             next, pick);
+                                                             next, pick, info);
   exact_successor_kernel<<<blocks(3 * p.nf, th), th, 0, stream>>>(faces, 3 * p.nf, partner, heads,
-                                                                  mask, next, pick, succ);
+                                                                  mask, next, pick, succ, info);
   exact_loops_kernel<<<blocks(3 * p.nf, th), th, 0, stream>>>(partner, succ, 3 * p.nf, lead,
                                                               counts, info);
   // Whether it pays is known here: a mesh whose edges do not cancel goes no further.
@@ -1740,7 +1762,7 @@ cudaError_t exact_boundary(const ExactPlan& p, const double* tri, int64_t ld, vo
   const bool dense = static_cast<double>(host.density) > kMostDense * kCoarseUnit * nf;
   const bool crowded = static_cast<double>(host.crowd) >
                        (mixed ? kMostCrowdedMixed : kMostCrowdedFp64) * nf * nf;
-  const bool fit = !host.bad && !dense && !crowded && host.nroot <= p.nf &&
+  const bool fit = !host.bad && !dense && !crowded && host.nopen <= p.nf &&
                    boundary_pays(host.nitem, p.nf, p.nq, mixed);
   boundary->dense = dense && !host.bad;
   boundary->edges = host.nroot;

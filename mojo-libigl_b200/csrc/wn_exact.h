@@ -48,6 +48,18 @@ ExactPlan plan_exact(int64_t nf, int64_t nq);
 // against 21.0 and 11.6). Few queries take fewer still (boundary_pays).
 constexpr double kExactMostFp64 = 0.55, kExactMostMixed = 0.13;
 
+// Seconds that all pairs take in FP64 and in mixed precision, with the mesh's preparation,
+// which sorts more than 16,384 faces in several passes (20,480 F without shared edges x 8,192
+// Q, ms, FP64 and mixed: 0.9 and 1.6, x 16,384 1.7 and 1.9, x 65,536 6.6 and 3.6; 14,336 F x
+// 16,384 Q 1.2 and 0.93).
+inline double fp64_pairs_seconds(int64_t nf, int64_t nq) {
+  return 4.9e-12 * static_cast<double>(nf) * static_cast<double>(nq);
+}
+inline double mixed_pairs_seconds(int64_t nf, int64_t nq) {
+  const double f = static_cast<double>(nf);
+  return (nf > 16384 ? 1.5e-3 : 0.5e-3) + 5e-9 * f + 1.5e-12 * f * static_cast<double>(nq);
+}
+
 // Whether a boundary of `items` costs less than all pairs of an FP64 or a mixed call.
 bool boundary_pays(int64_t items, int64_t nf, int64_t nq, bool mixed);
 

@@ -133,3 +133,19 @@ def test_meshes_that_all_pairs_suit_better(mesh, fp64, mixed):
         assert (w is not None) == bool(taken)
         if w is not None:
             assert float((w - ref).abs().max()) <= 1e-12
+
+
+@pytest.mark.parametrize("queries, taken", [(8192, True), (65536, False)])
+def test_soups_without_shared_edges(queries, taken):
+    """A mixed call that is declined takes the cheaper all-pairs kernel: FP64 for few pairs,
+    beside which the mixed kernel's preparation is large, else mixed (None here)."""
+    V, F = synthetic.unshare_vertices(*synthetic.bumpy_icosphere(5, seed=1))
+    T = V.reshape(-1, 3, 3)
+    V = (T.mean(1, keepdims=True) + 0.98 * (T - T.mean(1, keepdims=True))).reshape(-1, 3)
+    Vt, Ft, Ot = _tensors(V, F, synthetic.mixed_queries(V, F, queries, seed=3))
+    tri, ld, nf = wa.triangle_soa(Vt, Ft)
+    assert wa.forward_exact(tri, ld, nf, Ot) is None
+    w = wa.forward_exact(tri, ld, nf, Ot, mixed=True)
+    assert (w is not None) == taken
+    if taken:
+        assert torch.equal(w, wa.forward_fp64(tri, ld, nf, Ot))
