@@ -879,15 +879,26 @@ cudaError_t adjoint_fp64(const AdjointPlan& p, const double* tri, int64_t ld, in
   return cudaGetLastError();
 }
 
+// The kernel of an edge adjoint and its edges a CTA. Four edges a thread share one reduction,
+// but up to two blocks of them would be padding (2^20 Q, ms, the library's terms with two, and
+// the cheaper ones with two and four edges a thread: 3 edges 2.58, 1.47, 2.69; 200 2.15, 1.48,
+// 2.69; 257 5.05 and 2.70 with four).
+using EdgeKernel = void (*)(EdgeAdjointArgs);
+struct EdgeVariant {
+  EdgeKernel kernel;
+  int64_t edges;
+};
+EdgeVariant edge_variant(int64_t ne, bool soup) {
+  if (soup) return {adjoint_edges_kernel<kAdjThreads, kAdjFpt, kAdjQc, true>, kAdjThreads * kAdjFpt};
+  if (ne <= kAdjThreads * kAdjFpt)
+    return {adjoint_edges_kernel<kAdjThreads, kAdjFpt, kAdjQc, false>, kAdjThreads * kAdjFpt};
+  return {adjoint_edges_kernel<kAdjThreads, kAdjEpt, kAdjQc, false>, kAdjThreads * kAdjEpt};
+}
+
 AdjointPlan plan_adjoint_edges(int64_t ne, int64_t nq, int sms, bool soup) {
-  const int ept = soup ? kAdjFpt : kAdjEpt;
-  const int slots = resident_ctas(
-      soup ? reinterpret_cast<const void*>(
-                 adjoint_edges_kernel<kAdjThreads, kAdjFpt, kAdjQc, true>)
-           : reinterpret_cast<const void*>(
-                 adjoint_edges_kernel<kAdjThreads, kAdjEpt, kAdjQc, false>),
-      kAdjThreads, 0, sms);
-  return plan_waves(cdiv(ne, kAdjThreads * ept), nq, slots, kAdjQc);
+  const EdgeVariant v = edge_variant(ne, soup);
+  const int slots = resident_ctas(reinterpret_cast<const void*>(v.kernel), kAdjThreads, 0, sms);
+  return plan_waves(cdiv(ne, v.edges), nq, slots, kAdjQc);
 }
 
 size_t adjoint_edges_scratch_bytes(const AdjointPlan& p, int64_t le, int64_t nq) {
@@ -911,8 +922,7 @@ cudaError_t adjoint_edges(const AdjointPlan& p, const double* edges, int64_t le,
   if (e != cudaSuccess) return e;
   EdgeAdjointArgs a{edges, le, ne, q, gw, nq, p.blocks_per_range, p.queries_per_group,
                     dO_part, dE_part};
-  auto kernel = soup ? adjoint_edges_kernel<kAdjThreads, kAdjFpt, kAdjQc, true>
-                     : adjoint_edges_kernel<kAdjThreads, kAdjEpt, kAdjQc, false>;
+  const EdgeKernel kernel = edge_variant(ne, soup).kernel;
   kernel<<<dim3(static_cast<unsigned>(p.nranges), static_cast<unsigned>(p.ngroups)), kAdjThreads,
            0, stream>>>(a);
   finish_dq_kernel<<<static_cast<unsigned>(cdiv(nq * 3, 256)), 256, 0, stream>>>(dO_part, p.nranges,
