@@ -1603,6 +1603,9 @@ constexpr int kEaQc = kFaQc;
 // 16 8.0; 4,572 boundary edges x 262,144: 6.4, 5.8, 5.0, 4.7). Their partial sums grow
 // with the root of this.
 constexpr int kEdgeWaves = 16;
+// ... so calls whose scratch would pass this take fewer, down to the two that they had before
+// (10^7 edges x 10^7 queries 58 GB with 16, 20 with two).
+constexpr size_t kMostPartials = size_t(8) << 30;
 constexpr int kEaQcNoDq = 32;  // without dL/do shares a 32-query chunk is cheap in shared memory
 
 // Scratch layout of adjoint_edges_mixed (each piece 256-byte aligned).
@@ -1646,8 +1649,12 @@ AdjointPlan plan_adjoint_edges_mixed(int64_t ne, int64_t nq, int sms, bool no_dq
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   const int slots = resident_ctas(reinterpret_cast<const void*>(kernel), kFaThreads, smem, sms);
   const int64_t ntiles = std::max<int64_t>(1, cdiv(ne, kTileFaces));
-  return plan_balanced(cdiv(ntiles, kFaTiles), nq, slots, no_dq ? kEaQcNoDq : kEaQc,
-                       6 * ntiles * kTileFaces, kEdgeWaves);
+  for (int waves = kEdgeWaves;; waves /= 2) {
+    const AdjointPlan p =
+        plan_balanced(cdiv(ntiles, kFaTiles), nq, slots, no_dq ? kEaQcNoDq : kEaQc,
+                      6 * ntiles * kTileFaces, waves);
+    if (waves <= 2 || adjoint_edges_mixed_scratch_bytes(p, ne, nq) <= kMostPartials) return p;
+  }
 }
 
 size_t adjoint_edges_mixed_scratch_bytes(const AdjointPlan& p, int64_t ne, int64_t nq) {
