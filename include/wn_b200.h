@@ -237,6 +237,9 @@ int wn_batch_set_adjoint_fp64(void* batch, int fp64);
  * persistent grid, partial sums, qpt, target_pairs, boundary edges, adjoint
  * work items (of the selected precision), tile_faces, adjoint in FP64 (0/1). */
 int wn_batch_info(void* batch, int64_t* out, int64_t n);
+/* Pairs of a work item that wn_batch_create makes of `target_pairs` for a batch of
+ * total_pairs: fewer where the items would be too few for the last ones to end together. */
+int wn_batch_item_pairs(double total_pairs, int64_t target_pairs, int64_t* item_pairs);
 int wn_batch_destroy(void* batch);
 
 /* ---- adjoint (no reference counterpart) ---------------------------------

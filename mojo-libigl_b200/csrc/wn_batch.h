@@ -51,6 +51,9 @@ struct BatchState {
   BatchEdges* edges = nullptr;
 };
 
+// Pairs of a work item: at most `target_pairs`, fewer where a batch needs more items.
+int64_t batch_item_pairs(double total_pairs, int64_t target_pairs, int sms);
+
 // Host-side layout + device allocation. F: total_nf x 3, vertex indices local to
 // each mesh. Returns a CUDA error (allocation) or cudaSuccess.
 cudaError_t batch_create(BatchState* b, int64_t nmesh, const int64_t* nv, const int64_t* nf,

@@ -1058,6 +1058,17 @@ int wn_batch_info(void* batch, int64_t* out, int64_t n) {
   return WN_OK;
 }
 
+int wn_batch_item_pairs(double total_pairs, int64_t target_pairs, int64_t* item_pairs) {
+  if (!item_pairs || !(total_pairs >= 0.0) || target_pairs < 1)
+    return fail(WN_EINVAL, "bad total_pairs or target_pairs, or a null pointer");
+  std::lock_guard<std::mutex> lock(g_mutex);
+  int code = WN_OK;
+  DeviceCtx* c = context(&code);
+  if (!c) return code;
+  *item_pairs = batch_item_pairs(total_pairs, target_pairs, c->sms);
+  return WN_OK;
+}
+
 int wn_batch_destroy(void* batch) {
   if (!batch) return WN_OK;
   BatchState* b = static_cast<BatchState*>(batch);

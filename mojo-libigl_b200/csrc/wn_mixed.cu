@@ -1275,6 +1275,14 @@ cudaError_t dmalloc(T** p, size_t count) {
 
 }  // namespace
 
+// Items of at most `target_pairs`, and enough of them that the last ones end together:
+// kBatchItemsPerCta for each of the (at least four per SM) resident CTAs. An item of 2^17
+// pairs takes 0.1 ms, far above its start-up.
+int64_t batch_item_pairs(double total_pairs, int64_t target_pairs, int sms) {
+  const double even = total_pairs / (4.0 * std::max(sms, 1) * kBatchItemsPerCta);
+  return std::min<int64_t>(target_pairs, std::max<int64_t>(1 << 17, static_cast<int64_t>(even)));
+}
+
 cudaError_t batch_create(BatchState* b, int64_t nmesh, const int64_t* nv, const int64_t* nf,
                          const int64_t* nq, const int64_t* F, const BatchPlan& plan, int sms) {
   b->plan = plan;
@@ -1306,16 +1314,10 @@ cudaError_t batch_create(BatchState* b, int64_t nmesh, const int64_t* nv, const 
 
   // Work items and partial-sum layout.
   const int64_t per_block = int64_t(128) * plan.qpt;
-  // Items of at most plan.target_pairs, and enough of them that the last ones end
-  // together: kBatchItemsPerCta for each of the (at least four per SM) resident CTAs. An
-  // item of 2^17 pairs takes 0.1 ms, far above its start-up.
   double total_pairs = 0.0;
   for (int64_t m = 0; m < nmesh; ++m)
     total_pairs += static_cast<double>(nf[m]) * static_cast<double>(nq[m]);
-  const int64_t target_pairs = std::min<int64_t>(
-      plan.target_pairs,
-      std::max<int64_t>(1 << 17, static_cast<int64_t>(total_pairs / (4.0 * std::max(sms, 1) *
-                                                                     kBatchItemsPerCta))));
+  const int64_t target_pairs = batch_item_pairs(total_pairs, plan.target_pairs, sms);
   std::vector<BatchItem> items;
   std::vector<BatchMeshInfo> info(nmesh);
   int64_t p_off = 0;

@@ -18,6 +18,7 @@ accuracy beyond the tested bound.
 
 from __future__ import annotations
 
+import ctypes
 import itertools
 import json
 import math
@@ -26,16 +27,27 @@ import os
 import numpy as np
 import torch
 
+from . import _lib
+from .autograd import _check
 from .batched import Batch
 
 DEFAULT_SPACE = {
     "tile_faces": (64, 32),
     "qpt": (2, 1, 4),
-    "target_pairs": (1 << 23, 1 << 21),
+    "target_pairs": (1 << 23, 1 << 18),
     "ctas_per_sm": (0, 2),
     "kappa": (4.0, 3.0),
 }
-# The first value of each dimension is the starting point of the descent.
+# The first value of each dimension is the starting point of the descent. target_pairs is an
+# upper limit, which batches below about 4e10 pairs do not come near at 2^21 and more.
+
+
+def _item_pairs(total_pairs: float, target_pairs: int) -> int:
+    """What the library makes of target_pairs for a batch of this size."""
+    handle = _lib.lib()
+    out = ctypes.c_int64(0)
+    _check(handle.wn_batch_item_pairs(total_pairs, target_pairs, ctypes.byref(out)))
+    return out.value
 
 
 def cache_path() -> str:
@@ -96,7 +108,12 @@ def tune(meshes, queries, space=None, backward: bool = True, sample_queries: int
     timed = {}
 
     def measure(cfg: dict) -> float:
-        k = tuple(sorted(cfg.items()))
+        # Configurations that make the same work items are one: timed once, under the first.
+        launch = dict(cfg)
+        if "target_pairs" in cfg:
+            pairs = sum(len(F) * len(O) for (_, F), O in zip(meshes, sample))
+            launch["target_pairs"] = _item_pairs(float(pairs), cfg["target_pairs"])
+        k = tuple(sorted(launch.items()))
         if k not in timed:
             batch = Batch(meshes, sample, **cfg)
             try:
