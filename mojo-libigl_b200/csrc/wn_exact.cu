@@ -1832,24 +1832,37 @@ void launch_eval(const EvalArgs& a, cudaStream_t stream) {
 }
 }  // namespace
 
-// Lanes per query. More of them shrink the warp's box and fill the GPU where queries
-// are few, but every warp walks the tree and reads the mesh's boundary for itself.
-// Measured at 1 / 2 / 4 / 8 lanes, ms:
-//   closed   327,680 F x 16,384 Q 4.4 / 2.5 / 1.5 / 1.1   x 131,072 3.1 / 2.0 / 1.8 / 1.8
-//            x 2^20 5.1 / 4.6 / 5.6 / 7.8; 20,480 F x 2^20 2.3 / 2.5 / 3.4 / 5.3
-//   edges    28,322 F (terrain) x 16,384 1.5 / 0.86 / 0.68 / 0.70   x 65,536 1.4 / 1.0 /
-//            1.1 / 1.4   x 2^20 6.7 / 7.3 / 9.6 / 14.9;
-//            243,602 F x 131,072 5.7 / 4.8, x 262,144 8.2 / 7.2
-//   holes    19,456 F x 16,384 1.05 / 0.77 / 0.78 / 0.99   x 65,536 1.2 / 1.1 / 1.6 / 2.6
-//            x 2^20 6.5 / 7.8 / 18.3 / 34.4
+// Lanes per query. More of them shrink the warp's box and fill the GPU where queries are few
+// beside the mesh, but every warp walks the tree and reads the mesh's boundary for itself. Each
+// line is the number of queries from which fewer lanes are the quicker ones, between the sizes
+// where both were measured (ms at 1 / 2 / 4 / 8 lanes):
+//   closed   5,120 F x 32,768 Q 0.50 / 0.42 / 0.42 / 0.45   x 80,000 0.52 / 0.50 / 0.55 / 0.64
+//            x 180,000 0.66 / 0.67 / 0.78; 20,480 F x 24,000 0.68 / 0.55 / 0.50 / 0.51
+//            x 50,000 0.68 / 0.57 / 0.56 / 0.64   x 400,000 1.26 / 1.27 / 1.62; 81,920 F x 32,768
+//            1.41 / 1.00 / 0.75 / 0.72   x 80,000 1.36 / 0.94 / 0.88 / 0.99   x 600,000 2.24 /
+//            2.16 / 2.83; 327,680 F x 80,000 2.8 / 1.9 / 1.7 / 1.6   x 180,000 3.1 / 2.2 / 2.0
+//            x 400,000 3.6 / 2.9 / 3.1   x 2^20 5.1 / 4.6 / 5.6 / 7.8
+//   edges    (terrain) 28,322 F x 16,384 2.0 / 1.04 / 0.79 / 0.78   x 50,000 1.6 / 1.19 / 1.12 /
+//            1.25   x 262,144 2.8 / 2.6 / 3.0   x 600,000 4.8 / 4.7 / 5.9   x 2^20 7.3 / 7.6 / 9.6;
+//            243,602 F x 24,000 8.9 / 4.4 / 2.8 / 2.6   x 131,072 8.7 / 5.7 / 5.7   x 600,000 16.3 /
+//            15.0 / 17.3; 498,002 F x 50,000 13 / 8.2 / 6.2 / 5.4   x 262,144 17.7 / 14.0 / 13.7
+//   holes    18,842 F, 0.087 items a face, x 12,000 1.29 / 0.93 / 0.92 / 1.23   x 24,000 1.28 /
+//            0.96 / 1.32   x 100,000 1.74 / 1.68 / 3.2   x 131,072 1.90 / 1.99   x 2^20 6.5 / 7.8;
+//            79,462 F, 0.03 a face, x 100,000 2.8 / 2.4 / 4.6   x 180,000 3.4 / 3.5
 static int lanes_per_query(const ExactPlan& p, const ExactBoundary& boundary) {
-  const bool closed = boundary.items < 64, holes = 4 * boundary.loops > boundary.items;
-  const int64_t enough = closed ? 262144 : (holes ? 32768 : 131072);
-  int sub = 1;
-  while (sub < 8 && p.nq * sub < enough) sub *= 2;
-  if (closed && sub < 8 && 2 * p.nq < p.nf) sub *= 2;
-  if (sub == 1 && p.nq < (closed ? 8 * p.nf : std::max<int64_t>(100000, holes ? 0 : p.nf + p.nf / 8))) sub = 2;
-  return sub;
+  struct Lines {
+    double eight, four, two;  // below these
+  };
+  const double f = static_cast<double>(p.nf), q = static_cast<double>(p.nq);
+  Lines l;
+  if (boundary.items < 64)
+    l = {std::max(24e3, 0.41 * f), std::max(32768.0, std::min(1.4 * f, 300e3)),
+         std::max(180e3, 8.0 * f)};
+  else if (4 * boundary.loops <= boundary.items)
+    l = {std::max(20e3, 0.15 * f), 40e3 + 0.45 * f, std::max(500e3, 6.0 * f)};
+  else
+    l = {8192.0, 16384.0, 20 * boundary.items > p.nf ? 120e3 : 180e3};
+  return q < l.eight ? 8 : (q < l.four ? 4 : (q < l.two ? 2 : 1));
 }
 
 cudaError_t exact_eval(const ExactPlan& p, const ExactBoundary& boundary, const double* q, double* w,
