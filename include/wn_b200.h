@@ -124,6 +124,9 @@ int wn_fault_armed(void);
 /* Measured FMA-pipe peak of the current device in TFLOP/s (FMA = 2 flops),
  * bits = 64 or 32: the roofline denominator of these FP64/FP32-bound kernels. */
 int wn_probe_fma_tflops(int bits, double* tflops);
+/* 1/sqrt(x) and 1/x as the kernels' cheaper pair terms compute them, n device values (for the
+ * test of their error). */
+int wn_probe_roots_device(const double* x, int64_t n, double* rsqrt, double* rcp, void* stream);
 
 /* ---- plain FP64 forward (no reference counterpart beyond mli_winding_gpu) */
 

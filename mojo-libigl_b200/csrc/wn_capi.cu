@@ -449,6 +449,13 @@ int wn_inject_fault(int kind, int64_t after) {
 
 int wn_fault_armed(void) { return g_fault_kind.load() != WN_FAULT_NONE ? 1 : 0; }
 
+int wn_probe_roots_device(const double* x, int64_t n, double* rsqrt, double* rcp, void* stream) {
+  if (n < 0 || n > (int64_t(1) << 32) || (n > 0 && (!x || !rsqrt || !rcp)))
+    return fail(WN_EINVAL, "bad n=%lld or a null pointer", (long long)n);
+  const cudaError_t e = probe_roots(x, n, rsqrt, rcp, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? WN_OK : cuda_fail(e, "square-root probe");
+}
+
 int wn_probe_fma_tflops(int bits, double* tflops) {
   WN_NVTX_RANGE();
   if ((bits != 32 && bits != 64) || !tflops) return fail(WN_EINVAL, "bits must be 32 or 64");

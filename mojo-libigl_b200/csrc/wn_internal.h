@@ -49,6 +49,8 @@ cudaError_t launch_wait_selftest(uint32_t polls, int* err, cudaStream_t stream);
 
 // FMA-pipe peak probe (wn_probe.cu): TFLOP/s for bits = 64 or 32.
 cudaError_t probe_fma_tflops(int bits, int sms, cudaStream_t stream, double* tflops);
+cudaError_t probe_roots(const double* x, int64_t n, double* rsqrt, double* rcp,
+                        cudaStream_t stream);
 
 // ---- plain FP64 forward (wn_fp64.cu) ---------------------------------------
 enum Fp64Mode : int {

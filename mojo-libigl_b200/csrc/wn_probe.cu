@@ -70,7 +70,25 @@ __global__ void wait_selftest_kernel(uint32_t polls, int* err) {
   atomicOr(err, kErrWaitTimeout);
 }
 
+__global__ void __launch_bounds__(256) roots_kernel(const double* __restrict__ x, int64_t n,
+                                                    double* __restrict__ rsqrt,
+                                                    double* __restrict__ rcp) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
+  if (i >= n) return;
+  rsqrt[i] = rsqrt64(x[i]);
+  rcp[i] = rcp64(x[i]);
+}
+
 }  // namespace
+
+// rsqrt64 and rcp64 (wn_common.cuh) of n values, for the test of their error.
+cudaError_t probe_roots(const double* x, int64_t n, double* rsqrt, double* rcp,
+                        cudaStream_t stream) {
+  if (n <= 0) return cudaSuccess;
+  roots_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(x, n, rsqrt, rcp);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_wait_selftest(uint32_t polls, int* err, cudaStream_t stream) {
   wait_selftest_kernel<<<1, 32, 0, stream>>>(polls, err);

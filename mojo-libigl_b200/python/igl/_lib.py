@@ -58,6 +58,7 @@ _WN_SIGNATURES = {
     "wn_inject_fault": ([C_INT, I], C_INT),
     "wn_fault_armed": ([], C_INT),
     "wn_probe_fma_tflops": ([C_INT, ctypes.POINTER(ctypes.c_double)], C_INT),
+    "wn_probe_roots_device": ([P, I, P, P, P], C_INT),
     "wn_forward_fp64_host": ([P, P, P, I, I, C_INT], C_INT),
     "wn_forward_fp64_device": ([P, I, P, P, I, I, C_INT, P], C_INT),
     "wn_exact_pays": ([I, I], C_INT),
