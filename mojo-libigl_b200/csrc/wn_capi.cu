@@ -225,7 +225,7 @@ cudaError_t exact_forward(const double* tri, int64_t ld, const double* q, double
     if (bytes && dev_malloc_async(&edges, bytes, stream) != cudaSuccess) {
       cudaGetLastError();
     } else {
-      e = exact_eval(p, boundary, q, w, scratch, edges, sms, stream);
+      e = exact_eval(p, boundary, q, w, scratch, edges, mixed, sms, stream);
       *taken = e == cudaSuccess;
     }
     if (edges) cudaFreeAsync(edges, stream);
@@ -244,6 +244,7 @@ cudaError_t exact_forward(const double* tri, int64_t ld, const double* q, double
     } else {
       e = launch_fp64(plan, kFp64ArgProd, tri, ld, nf, q, nq, w, static_cast<double*>(partial),
                       err, stream);
+      if (e == cudaSuccess) e = exact_infinite(q, nq, w, stream);
       *taken = e == cudaSuccess;
       cudaFreeAsync(partial, stream);
     }

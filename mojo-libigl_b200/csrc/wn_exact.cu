@@ -1031,6 +1031,7 @@ struct EvalArgs {
   uint32_t* list;
   Info* info;
   int64_t nf, nq, top;  // top: the root node
+  bool mixed;           // stands in for the mixed kernel
 };
 
 struct WarpBox {
@@ -1206,6 +1207,16 @@ struct WarpMem {
   uint32_t farl[64], midl[64];
   uint8_t emit[32];
 };
+
+__device__ __forceinline__ bool at_infinity(double x, double y, double z) {
+  return !isnan(x) && !isnan(y) && !isnan(z) && (isinf(x) || isinf(y) || isinf(z));
+}
+
+__global__ void exact_infinite_kernel(const double* __restrict__ q, int64_t nq,
+                                      double* __restrict__ w) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i < nq && at_infinity(q[3 * i], q[3 * i + 1], q[3 * i + 2])) w[i] = 0.0;
+}
 
 // One warp per 32 / SUB consecutive queries of the Hilbert order, SUB lanes to a
 // query. The walk is the warp's: its lanes test 32 nodes at a time against the box
@@ -1532,8 +1543,8 @@ __global__ void __launch_bounds__(32 * kWarps, 4) exact_eval_kernel(const EvalAr
     a.w[qi] = (near_angle + argument) / kTwoPi + k;
   else if (isfinite(qx) && isfinite(qy) && isfinite(qz))
     a.list[atomicAdd(&a.info->nlist, 1)] = qi;
-  else
-    a.w[qi] = NAN;  // as every pair term is
+  else  // as every pair term is, and the mixed kernel's sum
+    a.w[qi] = a.mixed && at_infinity(qx, qy, qz) ? 0.0 : NAN;
 }
 
 // All pairs for the listed queries, one CTA per query: per-thread running products
@@ -1866,7 +1877,7 @@ static int lanes_per_query(const ExactPlan& p, const ExactBoundary& boundary) {
 }
 
 cudaError_t exact_eval(const ExactPlan& p, const ExactBoundary& boundary, const double* q, double* w,
-                       void* scratch, void* block, int sms, cudaStream_t stream) {
+                       void* scratch, void* block, bool mixed, int sms, cudaStream_t stream) {
   const Edges edges(boundary, block);
   const cudaError_t e = build_tree(p, boundary, edges, q, scratch, stream);
   if (e != cudaSuccess) return e;
@@ -1888,6 +1899,7 @@ cudaError_t exact_eval(const ExactPlan& p, const ExactBoundary& boundary, const 
   a.nf = p.nf;
   a.nq = p.nq;
   a.top = p.nnode - 1;
+  a.mixed = mixed;
   switch (lanes_per_query(p, boundary)) {
     case 1: launch_eval<1>(a, stream); break;
     case 2: launch_eval<2>(a, stream); break;
@@ -1897,6 +1909,12 @@ cudaError_t exact_eval(const ExactPlan& p, const ExactBoundary& boundary, const 
   exact_fallback_kernel<<<static_cast<unsigned>(std::max(sms, 1) * 4), 256, 0, stream>>>(
       a.faces, p.nf, q, a.list, a.info, w);
   g_launches.fetch_add(2, std::memory_order_relaxed);
+  return cudaGetLastError();
+}
+
+cudaError_t exact_infinite(const double* q, int64_t nq, double* w, cudaStream_t stream) {
+  exact_infinite_kernel<<<blocks(nq, 256), 256, 0, stream>>>(q, nq, w);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
   return cudaGetLastError();
 }
 

@@ -81,8 +81,14 @@ cudaError_t exact_boundary(const ExactPlan& p, const double* tri, int64_t ld, vo
 size_t exact_boundary_bytes(const ExactBoundary& boundary);
 
 // Builds the tree and the query order in `scratch` and the boundary in `edges`, after
-// exact_boundary, and evaluates W of the queries (in the order given).
+// exact_boundary, and evaluates W of the queries (in the order given). Infinite queries get
+// what the all-pairs kernel that this stands in for gives them: NaN in FP64, 0 in mixed
+// precision.
 cudaError_t exact_eval(const ExactPlan& p, const ExactBoundary& boundary, const double* q,
-                       double* w, void* scratch, void* edges, int sms, cudaStream_t stream);
+                       double* w, void* scratch, void* edges, bool mixed, int sms,
+                       cudaStream_t stream);
+
+// Sets w to 0 for infinite queries: FP64 pairs in a mixed call.
+cudaError_t exact_infinite(const double* q, int64_t nq, double* w, cudaStream_t stream);
 
 }  // namespace wn

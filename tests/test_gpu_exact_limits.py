@@ -149,3 +149,25 @@ def test_soups_without_shared_edges(queries, taken):
     assert (w is not None) == taken
     if taken:
         assert torch.equal(w, wa.forward_fp64(tri, ld, nf, Ot))
+
+
+@pytest.mark.parametrize("mesh", ["closed", "open", "separate", "dense"])
+@pytest.mark.parametrize("queries", [2000, 12000, 70000])
+def test_infinite_queries_in_float32(mesh, queries):
+    """0 by the mixed kernel, and so by whatever does a mixed call in its place; NaN for NaN."""
+    V, F = synthetic.bumpy_icosphere(5, seed=2)
+    if mesh == "open":
+        F = synthetic.delete_faces(F, 0.05, seed=2)
+    elif mesh == "separate":
+        V, F = synthetic.unshare_vertices(V, F)
+        V = V + np.repeat(np.random.default_rng(0).normal(size=(len(F), 3)) * 1e-3, 3, 0)
+    elif mesh == "dense":
+        V, F = _spheres(1024, 0.4)
+    O = synthetic.box_points(V, queries, seed=3)
+    bad = [[np.inf, 0, 0], [0, -np.inf, 0], [np.inf, np.inf, -np.inf], [1e200, 0, 0]]
+    O[:4] = bad
+    O[4], O[5] = [np.nan, 0, 0], [np.inf, np.nan, 0]
+    Vt, Ft, Ot = _tensors(V, F, O)
+    w = wa.winding_number_torch(Vt.float(), Ft, Ot.float())
+    assert w[:4].tolist() == [0.0] * 4
+    assert torch.isnan(w[4:6]).all() and torch.isfinite(w[6:]).all()
