@@ -388,6 +388,30 @@ __device__ __forceinline__ T block_reduce(T v, T* part, F f) {
   return v;
 }
 
+// A node's walk record, its discs without bounds yet.
+__global__ void aabb_walk_kernel(const AabbNodeRec* __restrict__ nodes,
+                                 const AabbSpan* __restrict__ spans, int64_t n, const AabbFrame f,
+                                 AabbWalkRec* __restrict__ walk) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const AabbNodeRec& r = nodes[i];
+  const AabbDisc none{{0.f, 0.f, 0.f}, INFINITY, {0.f, 0.f, 0.f}, INFINITY};
+  AabbWalkRec w;
+  const bool leaf = r.count > 0;
+  w.left = leaf ? spans[i].slot : r.left;
+  w.right = r.right;
+  w.start = leaf ? r.start : spans[r.right].first;
+  w.count = r.count;
+  w.ldisc = w.rdisc = none;
+  for (int k = 0; k < 3; ++k) {  // unused in a leaf
+    w.lbox[k] = __double2float_rd((r.lbox[k] - f.c[k]) * f.s);
+    w.rbox[k] = __double2float_rd((r.rbox[k] - f.c[k]) * f.s);
+    w.lbox[3 + k] = __double2float_ru((r.lbox[3 + k] - f.c[k]) * f.s);
+    w.rbox[3 + k] = __double2float_ru((r.rbox[3 + k] - f.c[k]) * f.s);
+  }
+  walk[i] = w;
+}
+
 __device__ __forceinline__ double3 local_corner(const AabbTriRec& t, int j, const AabbFrame& f) {
   const double* x = j == 0 ? t.a : (j == 1 ? t.b : t.c);
   return make_double3((x[0] - f.c[0]) * f.s, (x[1] - f.c[1]) * f.s, (x[2] - f.c[2]) * f.s);
@@ -578,6 +602,8 @@ cudaError_t aabb_query(const AabbDeviceTree& t, const double* P, int64_t np, con
 cudaError_t aabb_discs(const AabbDeviceTree& t, const int32_t* big, int64_t nbig,
                        int32_t* thin, cudaStream_t stream) {
   if (t.nnodes <= 0) return cudaSuccess;
+  aabb_walk_kernel<<<static_cast<unsigned>((t.nnodes + 255) / 256), 256, 0, stream>>>(
+      t.nodes, t.spans, t.nnodes, t.frame, t.walk);
   aabb_disc_kernel<<<static_cast<unsigned>(t.nnodes), 32, 0, stream>>>(t.tris, t.spans, nullptr,
                                                                        t.frame, t.walk, t.nodes);
   if (nbig > 0)
@@ -585,7 +611,7 @@ cudaError_t aabb_discs(const AabbDeviceTree& t, const int32_t* big, int64_t nbig
                                                                       t.walk, t.nodes);
   aabb_face_disc_kernel<<<static_cast<unsigned>((t.nleaf_faces + 255) / 256), 256, 0, stream>>>(
       t.tris, t.nleaf_faces, t.frame, t.face_discs, thin);
-  g_launches.fetch_add(nbig > 0 ? 3 : 2, std::memory_order_relaxed);
+  g_launches.fetch_add(nbig > 0 ? 4 : 3, std::memory_order_relaxed);
   return cudaGetLastError();
 }
 

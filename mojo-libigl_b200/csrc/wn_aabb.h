@@ -110,7 +110,7 @@ cudaError_t aabb_query(const AabbDeviceTree& t, const double* P, int64_t np, con
                        double* sqrd, int64_t* index, double* closest, int* err,
                        cudaStream_t stream);
 
-// Fills in the discs and slabs of a tree, its nodes' and its faces', whose records are on
+// Makes the walk records of a tree and its faces' discs, and fills in its slabs; the others are on
 // the device (big: the nbig nodes of more than kDiscBig faces,
 // device). *thin (device, set to 0 before) receives the number of faces thinner than
 // 1 : 1000: the reference's closest point on such a face may lie off it (the barycentric
@@ -135,17 +135,16 @@ int64_t aabb_build(const double* V, int64_t nv, const int64_t* F, int64_t nf, in
                    double* boxes, int64_t* nodes, int64_t* order, int threads, const char** why);
 
 // Validates caller-supplied tree arrays and converts them to the device
-// records (host memory, caller-sized: nnodes node and walk records and spans, nf face
-// records); the discs are left without bounds, for aabb_discs to fill in on the device.
-// *scale receives the largest |coordinate| of the mesh and *frame its frame; *regular whether every box holds
-// its children's boxes or its faces and every face lies in one leaf, as in the trees
-// that aabb_build makes. Returns the depth (root = 1), or a negative value with the
-// reason in *why.
+// records (host memory, caller-sized: nnodes node records and spans, nf face records); the
+// slabs are left without bounds, for aabb_discs to fill in on the device.
+// *scale receives the largest |coordinate| of the mesh and *frame its frame; *regular
+// whether every box holds its children's boxes or its faces and every face lies in one leaf,
+// as in the trees that aabb_build makes. Returns the depth (root = 1), or a negative value
+// with the reason in *why.
 int64_t aabb_pack(const double* V, int64_t nv, const int64_t* F, int64_t nf, const double* boxes,
                   const int64_t* nodes, const int64_t* order, int64_t nnodes,
-                  AabbNodeRec* node_out, AabbWalkRec* walk_out, AabbSpan* span_out,
-                  AabbTriRec* tri_out, double* scale, AabbFrame* frame, bool* regular,
-                  const char** why);
+                  AabbNodeRec* node_out, AabbSpan* span_out, AabbTriRec* tri_out, double* scale,
+                  AabbFrame* frame, bool* regular, const char** why);
 
 // The walk's bounds are computed in FP32 in the tree's frame: kWalkMargin * (ext + |px'| +
 // |py'| + |pz'|) covers the rounding of p', of the differences and of their products (under

@@ -196,18 +196,6 @@ int64_t aabb_build(const double* V, int64_t nv, const int64_t* F, int64_t nf, in
 
 namespace {
 
-float round_down(double x) {
-  float f = static_cast<float>(x);
-  if (static_cast<double>(f) > x) f = std::nextafter(f, -INFINITY);
-  return f;
-}
-
-float round_up(double x) {
-  float f = static_cast<float>(x);
-  if (static_cast<double>(f) < x) f = std::nextafter(f, INFINITY);
-  return f;
-}
-
 // Every node's run of face records (empty where its children's are not one run, possible
 // only in a caller-made tree) and its place beside its parent; true if every internal
 // node's run is its left child's followed by its right child's and every node but the root
@@ -263,7 +251,7 @@ bool holds(const double* box, const double* points, int64_t n) {
 
 int64_t aabb_pack(const double* V, int64_t nv, const int64_t* F, int64_t nf, const double* boxes,
                   const int64_t* nodes, const int64_t* order, int64_t nnodes,
-                  AabbNodeRec* node_out, AabbWalkRec* walk_out, AabbSpan* span_out,
+                  AabbNodeRec* node_out, AabbSpan* span_out,
                   AabbTriRec* tri_out, double* scale, AabbFrame* frame, bool* regular,
                   const char** why) {
   *regular = false;
@@ -349,35 +337,16 @@ int64_t aabb_pack(const double* V, int64_t nv, const int64_t* F, int64_t nf, con
     *why = "tree deeper than the traversal stack";
     return -1;
   }
-  bool sound = node_spans(nodes, nnodes, span_out);
-  sound = sound && frame->s > 0.0;
-  const AabbDisc none{{0.f, 0.f, 0.f}, INFINITY, {0.f, 0.f, 0.f}, INFINITY};
-  auto local = [&](double x, int k) { return (x - frame->c[k]) * frame->s; };
-  for (int64_t i = 0; i < nnodes; ++i) {
+  bool sound = node_spans(nodes, nnodes, span_out) && frame->s > 0.0;
+  for (int64_t i = 0; sound && i < nnodes; ++i) {
     const AabbNodeRec& r = node_out[i];
-    AabbWalkRec& w = walk_out[i];
     const double* box = boxes + 6 * i;
-    w.ldisc = w.rdisc = none;
-    w.start = r.start;
-    w.count = r.count;
     if (r.count > 0) {
-      w.left = span_out[i].slot;
-      w.right = -1;
-      for (int k = 0; k < 6; ++k) w.lbox[k] = w.rbox[k] = 0.f;
       for (int64_t k = r.start; sound && k < static_cast<int64_t>(r.start) + r.count; ++k)
         sound = holds(box, tri_out[k].a, 3);  // the three corners lie behind each other
       continue;
     }
-    w.left = r.left;
-    w.right = r.right;
-    w.start = span_out[r.right].first;
-    sound = sound && holds(box, r.lbox, 2) && holds(box, r.rbox, 2);
-    for (int k = 0; k < 3; ++k) {
-      w.lbox[k] = round_down(local(r.lbox[k], k));
-      w.rbox[k] = round_down(local(r.rbox[k], k));
-      w.lbox[3 + k] = round_up(local(r.lbox[3 + k], k));
-      w.rbox[3 + k] = round_up(local(r.rbox[3 + k], k));
-    }
+    sound = holds(box, r.lbox, 2) && holds(box, r.rbox, 2);
   }
   *regular = sound;
   return depth;

@@ -14,7 +14,9 @@
 #include <cstdio>
 #include <algorithm>
 #include <cstdlib>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -1154,17 +1156,18 @@ int wn_aabb_create(const double* V, int64_t nv, const int64_t* F, int64_t nf,
   if (nv < 0 || nf < 0 || nnodes < 0) return fail(WN_EINVAL, "negative size");
   if (nnodes > 0 && (!V || !F || !boxes || !nodes || !order))
     return fail(WN_EINVAL, "null pointer");
-  std::vector<AabbNodeRec> nrec(static_cast<size_t>(nnodes));
-  std::vector<AabbTriRec> trec(static_cast<size_t>(nnodes > 0 ? nf : 0));
-  std::vector<AabbWalkRec> wrec(static_cast<size_t>(nnodes));
-  std::vector<AabbSpan> spans(static_cast<size_t>(nnodes));
+  // Not set to zero first: aabb_pack writes every record.
+  const size_t ntri = static_cast<size_t>(nnodes > 0 ? nf : 0);
+  std::unique_ptr<AabbNodeRec[]> nrec(new (std::nothrow) AabbNodeRec[static_cast<size_t>(nnodes)]);
+  std::unique_ptr<AabbTriRec[]> trec(new (std::nothrow) AabbTriRec[ntri]);
+  std::unique_ptr<AabbSpan[]> spans(new (std::nothrow) AabbSpan[static_cast<size_t>(nnodes)]);
+  if (!nrec || !trec || !spans) return fail(WN_ENOMEM, "host memory for the tree's records");
   const char* why = "";
   double scale = 0.0;
   AabbFrame frame;
   bool regular = false;
-  const int64_t depth = aabb_pack(V, nv, F, nf, boxes, nodes, order, nnodes, nrec.data(),
-                                  wrec.data(), spans.data(), trec.data(), &scale, &frame,
-                                  &regular, &why);
+  const int64_t depth = aabb_pack(V, nv, F, nf, boxes, nodes, order, nnodes, nrec.get(),
+                                  spans.get(), trec.get(), &scale, &frame, &regular, &why);
   if (depth < 0) return fail(WN_EINVAL, "invalid tree: %s", why);
   std::lock_guard<std::mutex> lock(g_mutex);
   int code = WN_OK;
@@ -1173,7 +1176,7 @@ int wn_aabb_create(const double* V, int64_t nv, const int64_t* F, int64_t nf,
   AabbHandle* h = new AabbHandle();
   cudaGetDevice(&h->device);
   h->t.nnodes = nnodes;
-  h->t.nleaf_faces = static_cast<int64_t>(trec.size());
+  h->t.nleaf_faces = static_cast<int64_t>(ntri);
   h->t.depth = static_cast<int>(depth);
   h->t.scale = scale;
   h->t.frame = frame;
@@ -1194,18 +1197,17 @@ int wn_aabb_create(const double* V, int64_t nv, const int64_t* F, int64_t nf,
       return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream);
     };
     cudaError_t e;
-    if ((e = dev_malloc(&h->t.nodes, sizeof(AabbNodeRec) * nrec.size())) != cudaSuccess ||
-        (e = dev_malloc(&h->t.tris, sizeof(AabbTriRec) * trec.size())) != cudaSuccess ||
-        (e = upload(h->t.nodes, nrec.data(), sizeof(AabbNodeRec) * nrec.size())) != cudaSuccess ||
-        (e = upload(h->t.tris, trec.data(), sizeof(AabbTriRec) * trec.size())) != cudaSuccess ||
+    const size_t n = static_cast<size_t>(nnodes);
+    if ((e = dev_malloc(&h->t.nodes, sizeof(AabbNodeRec) * n)) != cudaSuccess ||
+        (e = dev_malloc(&h->t.tris, sizeof(AabbTriRec) * ntri)) != cudaSuccess ||
+        (e = upload(h->t.nodes, nrec.get(), sizeof(AabbNodeRec) * n)) != cudaSuccess ||
+        (e = upload(h->t.tris, trec.get(), sizeof(AabbTriRec) * ntri)) != cudaSuccess ||
         (discs &&
-         ((e = dev_malloc(&h->t.walk, sizeof(AabbWalkRec) * wrec.size())) != cudaSuccess ||
-          (e = dev_malloc(&h->t.face_discs, sizeof(AabbDisc) * trec.size())) != cudaSuccess ||
-          (e = dev_malloc(&h->t.spans, sizeof(AabbSpan) * spans.size())) != cudaSuccess ||
+         ((e = dev_malloc(&h->t.walk, sizeof(AabbWalkRec) * n)) != cudaSuccess ||
+          (e = dev_malloc(&h->t.face_discs, sizeof(AabbDisc) * ntri)) != cudaSuccess ||
+          (e = dev_malloc(&h->t.spans, sizeof(AabbSpan) * n)) != cudaSuccess ||
           (e = dev_malloc(&big_d, sizeof(int32_t) * big.size())) != cudaSuccess ||
-          (e = upload(h->t.walk, wrec.data(), sizeof(AabbWalkRec) * wrec.size())) !=
-              cudaSuccess ||
-          (e = upload(h->t.spans, spans.data(), sizeof(AabbSpan) * spans.size())) != cudaSuccess ||
+          (e = upload(h->t.spans, spans.get(), sizeof(AabbSpan) * n)) != cudaSuccess ||
           (e = upload(big_d, big.data(), sizeof(int32_t) * big.size())) != cudaSuccess ||
           (e = aabb_discs(h->t, big_d, nbig, big_d + nbig, c->stream)) != cudaSuccess ||
           (e = cudaMemcpyAsync(&thin, big_d + nbig, sizeof(int32_t), cudaMemcpyDeviceToHost,
