@@ -43,10 +43,12 @@ enum { WN_FAULT_NONE = 0, WN_FAULT_ALLOC = 1 };
 
 /* FP64 accumulation modes of the plain kernel. */
 enum {
-  WN_FP64_ARGPROD = 0, /* bit-exact pair terms, argument-of-product sum */
+  WN_FP64_ARGPROD = 0, /* argument-of-product sum; pair terms bit-exact wherever a branch of the
+                          angle is near, elsewhere within a few roundings */
   WN_FP64_DIRECT = 1,  /* bit-exact pair terms, one atan2 per pair */
-  WN_FP64_TILED = 2    /* WN_FP64_ARGPROD over a prepared mesh (Morton tiles, faces in
-                          strips) that reuses repeated corners; host entry only */
+  WN_FP64_TILED = 2    /* argument-of-product sum, bit-exact pair terms over a prepared mesh
+                          (Morton tiles, faces in strips) that reuses repeated corners; host
+                          entry only */
 };
 
 /* ---- reference-compatible entry points --------------------------------- */

@@ -1169,7 +1169,8 @@ struct MixedEdgeArgs {
 template <int QC, bool DQ = true>
 struct EdgeAdjSmem {
   float dO32[DQ ? QC * 3 : 1][kFaRow];  // per-thread FP32 dL/do shares, row 3*query + axis
-  double acc64[12][kFaThreads];  // per-edge FP64 sums (thread-private columns)
+  double acc64[12][kFaThreads];  // per-edge FP64 sums; a warp's lanes add to one another's
+                                 // columns, between its barriers (a query's near edges)
   double red64[kFaTiles][QC][3];
   double dsum[QC * 3];
   double4 q64[QC];

@@ -54,9 +54,11 @@ cudaError_t probe_roots(const double* x, int64_t n, double* rsqrt, double* rcp,
 
 // ---- plain FP64 forward (wn_fp64.cu) ---------------------------------------
 enum Fp64Mode : int {
-  kFp64ArgProd = 0,  // bit-exact pair terms, argument-of-product accumulation
+  kFp64ArgProd = 0,  // argument-of-product accumulation; pair terms bit-exact wherever a branch
+                     // of the angle is near, elsewhere within a few roundings
   kFp64Direct = 1,   // bit-exact pair terms, one atan2 per pair
-  kFp64Tiled = 2,    // kFp64ArgProd over a prepared mesh, repeated corners reused
+  kFp64Tiled = 2,    // bit-exact pair terms over a prepared mesh, repeated corners reused,
+                     // argument-of-product accumulation
   kFp64Auto = 3,     // internal: near faces + boundary (wn_exact.cu) where that pays, else
                      // kFp64ArgProd
 };

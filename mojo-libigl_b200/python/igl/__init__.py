@@ -55,7 +55,8 @@ __all__ = [
     "per_vertex_normals",
 ]
 
-# "fp64": the plain FP64 kernel, pair terms bit-identical to the reference.
+# "fp64": FP64 throughout, pair terms bit-identical to the reference's wherever their last
+# bits can matter.
 # "mixed": FP32 pair terms with compensated accumulation and FP64 refinement
 # of near-surface pairs (max abs error vs FP64 reported by the tests/bench).
 PRECISIONS = ("fp64", "mixed")

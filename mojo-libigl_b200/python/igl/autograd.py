@@ -80,9 +80,9 @@ def forward_fp64(tri: torch.Tensor, ld: int, nf: int, O: torch.Tensor) -> torch.
 
 
 def use_prepared_fp64(nf: int, nq: int) -> bool:
-    """Whether a mesh's preparation (~2 ms) is small beside one FP64 forward. The
-    streaming kernel is the faster one at every size all the same; a prepared mesh
-    serves callers that keep it."""
+    """Whether a mesh's preparation (~2 ms) is small beside one FP64 forward. Nothing in
+    the package asks: the streaming kernel is the faster one at every size all the
+    same, and the exact path where it applies."""
     return 4096 <= nf <= 0x7FFFFFFF and float(nf) * nq >= 1e9
 
 
