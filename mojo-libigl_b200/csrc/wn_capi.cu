@@ -232,7 +232,7 @@ cudaError_t exact_forward(const double* tri, int64_t ld, const double* q, double
     }
     if (edges) cudaFreeAsync(edges, stream);
   } else if (e == cudaSuccess && mixed && !(ld & 1) && !(reinterpret_cast<uintptr_t>(tri) & 15) &&
-             (boundary.dense || fp64_pairs_seconds(nf, nq) <= mixed_pairs_seconds(nf, nq))) {
+             (boundary.dense || fp64_pairs_pay(nf, nq))) {
     // All pairs in FP64 are the cheaper ones: few pairs, beside which the mixed kernel's
     // preparation is large, or a dense mesh, where most pairs are near ones, which the mixed
     // kernel refines in FP64 after it has done them in FP32 (65,536 Q, ms, FP64 and mixed:

@@ -1614,13 +1614,15 @@ bool exact_pays(int64_t nf, int64_t nq) {
 // costs. 301,466 F with 26,214 holes x 4,096 Q: 7.3 ms against 6.7 (FP64 streaming) and 4.7
 // (mixed), x 8,192 8.5 against 13.4 and 7.7, x 16,384 9.6 against 25 and 11.5; 1,205,862 F
 // with 104,858 holes x 4,096 27 against 25 and 12, x 16,384 38 against 99 and 36; 75,366 F
-// with 6,554 x 4,096 1.9 against 1.6 and 2.6. So it matters to mixed calls.
+// with 6,554 x 4,096 1.9 against 1.6 and 2.6. So it matters to mixed calls, whose own
+// preparation counts too (about 1.5 ms and 5 ns a face; 0.8 and 1 on a faster host, where the
+// last of these takes 1.4 ms).
 bool boundary_pays(int64_t items, int64_t nf, int64_t nq, bool mixed) {
   const double n = static_cast<double>(items), f = static_cast<double>(nf),
                q = static_cast<double>(nq);
   if (!mixed) return n <= kExactMostFp64 * f;
   return n <= kExactMostMixed * f &&
-         n * (0.23e-6 + 4.8e-12 * q) <= mixed_pairs_seconds(nf, nq);
+         n * (0.23e-6 + 4.8e-12 * q) <= 1.5e-3 + 5e-9 * f + 1.5e-12 * f * q;
 }
 
 ExactPlan plan_exact(int64_t nf, int64_t nq) {

@@ -48,16 +48,14 @@ ExactPlan plan_exact(int64_t nf, int64_t nq);
 // against 21.0 and 11.6). Few queries take fewer still (boundary_pays).
 constexpr double kExactMostFp64 = 0.55, kExactMostMixed = 0.13;
 
-// Seconds that all pairs take in FP64 and in mixed precision, with the mesh's preparation,
-// which sorts more than 16,384 faces in several passes (20,480 F without shared edges x 8,192
-// Q, ms, FP64 and mixed: 0.9 and 1.6, x 16,384 1.7 and 1.9, x 65,536 6.6 and 3.6; 14,336 F x
-// 16,384 Q 1.2 and 0.93).
-inline double fp64_pairs_seconds(int64_t nf, int64_t nq) {
-  return 4.9e-12 * static_cast<double>(nf) * static_cast<double>(nq);
-}
-inline double mixed_pairs_seconds(int64_t nf, int64_t nq) {
-  const double f = static_cast<double>(nf);
-  return (nf > 16384 ? 1.5e-3 : 0.5e-3) + 5e-9 * f + 1.5e-12 * f * static_cast<double>(nq);
+// Whether all pairs cost less in FP64 than in mixed precision with the mesh's preparation,
+// whose allocations and waits take the host 0.75 ms at least (two hosts, ms, FP64 and mixed:
+// 20,480 F without shared edges x 8,192 Q 0.9 and 0.9 to 1.5, x 16,384 1.7 and 1.3 to 1.9,
+// x 65,536 6.6 and 3.0 to 3.6; 57,344 F x 4,096 Q 1.2 and 1.0 to 2.2; up to 16,384 F it is half
+// as much: 14,336 F x 16,384 Q 1.2 and 0.9).
+inline bool fp64_pairs_pay(int64_t nf, int64_t nq) {
+  const double pairs = static_cast<double>(nf) * static_cast<double>(nq);
+  return 4.9e-12 * pairs <= (nf > 16384 ? 0.75e-3 : 0.4e-3) + 1.55e-12 * pairs;
 }
 
 // Whether a boundary of `items` costs less than all pairs of an FP64 or a mixed call.
