@@ -98,7 +98,7 @@ struct Info {
   int32_t nlist;                      // queries left to exact_fallback_kernel
   unsigned long long crowd;           // sum over the order's cells of their faces, squared
   unsigned long long density;         // sum over the faces of their coarse cells' area, in faces
-                                      // of a cell (2^-16)
+                                      // of a cell (2^-8: below 2^63 for 10^7 of the largest)
 };
 
 // Coarse cells, 32 to an axis: the upper half of the order's key.
@@ -404,7 +404,7 @@ __global__ void exact_gather_kernel(const double* __restrict__ tri, int64_t ld, 
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int k = 1; k < kGatherThreads / 32; ++k) around += part[k];
-    atomicAdd(&info->density, around);
+    atomicAdd(&info->density, around >> 8);
   }
   if (i >= nf) return;
   const uint32_t f = order[i];
@@ -1772,7 +1772,7 @@ cudaError_t exact_boundary(const ExactPlan& p, const double* tri, int64_t ld, vo
     return e;
   g_launches.fetch_add(9, std::memory_order_relaxed);
   const double nf = static_cast<double>(p.nf);
-  const bool dense = static_cast<double>(host.density) > kMostDense * kCoarseUnit * nf;
+  const bool dense = static_cast<double>(host.density) > kMostDense * (kCoarseUnit / 256.0) * nf;
   const bool crowded = static_cast<double>(host.crowd) >
                        (mixed ? kMostCrowdedMixed : kMostCrowdedFp64) * nf * nf;
   const bool fit = !host.bad && !dense && !crowded && host.nopen <= p.nf &&
