@@ -42,8 +42,9 @@ def test_queries_that_are_not_finite(bad, axes):
     got, ref = wa.forward_exact(tri, ld, nf, Qt), wa.forward_fp64(tri, ld, nf, Qt)
     assert bool(torch.isnan(ref[::2]).all()) and bool(torch.isnan(got[::2]).all())
     assert float((got - ref)[1::2].abs().max()) <= 1e-12
+    # 0.9 to 1.0 times the finite queries' cost; 11.6 to 12.2 when summed over all pairs.
     assert (_ms(lambda: wa.forward_exact(tri, ld, nf, Qt))
-            < 10 * _ms(lambda: wa.forward_exact(tri, ld, nf, Ot)))
+            < 4 * _ms(lambda: wa.forward_exact(tri, ld, nf, Ot)))
 
 
 def _holes(level):
